@@ -38,30 +38,38 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
   return *reinterpret_cast<const uint32_t*>(&v);
 }
 
+// Every GEMM of the network is cut into column blocks of MLP_NC columns beside the 128-row tiles,
+// one CTA each.  What bounds these GEMMs (512 x 256 x 256) is the epilogue's chain of TMEM reads,
+// expf and stores, 16 columns at a time, not the 0.07 us of tensor work: with one block of 256
+// columns a hidden layer took 33 us on 4 of the 152 SMs, with 32-column blocks on 32 SMs 9 us.
+// The K loop of a column is the same in either form, and so are the results, bit for bit.
+constexpr int MLP_NC = 32;
+
 // ---------------------------------------------------------------- GEMM epilogues
 // forward: z = acc + b; hidden layers store silu(z) (row-major and transposed, BF16) and
-// silu'(z); the last layer stores z
-template <int NCOL> struct FwdEpi {
+// silu'(z); the last layer stores the real outputs of z, packed [Bt][out_dim]
+struct FwdEpi {
   const float* bias;
-  int last, Bt;
-  bf16* H;   // [Bt][NCOL]
-  bf16* HT;  // [NCOL][Bt]
-  float* S;  // [Bt][NCOL]
-  float* Y;  // [Bt][NCOL]
-  __device__ void row(uint32_t taddr, int row, int m0, int) {
+  int last, Bt, ld, out_dim;
+  bf16* H;   // [Bt][ld]
+  bf16* HT;  // [ld][Bt]
+  float* S;  // [Bt][ld]
+  float* Y;  // [Bt][out_dim]
+  __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int r = m0 + row;
-#pragma unroll 1
-    for (int c0 = 0; c0 < NCOL; c0 += 16) {
+#pragma unroll
+    for (int q0 = 0; q0 < MLP_NC; q0 += 16) {
+      const int c0 = sp * MLP_NC + q0;
       float a[16];
-      umma::tmem_ld16(taddr + c0, a);
+      umma::tmem_ld16(taddr + q0, a);
       umma::tmem_ld_wait();
       float z[16];
 #pragma unroll
       for (int j = 0; j < 16; ++j) z[j] = a[j] + bias[c0 + j];
       if (last) {
-        float4* y = reinterpret_cast<float4*>(Y + (size_t)r * NCOL + c0);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) y[q] = make_float4(z[4 * q], z[4 * q + 1], z[4 * q + 2], z[4 * q + 3]);
+        for (int j = 0; j < 16; ++j)
+          if (c0 + j < out_dim) Y[(size_t)r * out_dim + c0 + j] = z[j];
         continue;
       }
       float h[16], d[16];
@@ -71,32 +79,32 @@ template <int NCOL> struct FwdEpi {
         h[j] = z[j] * s;
         d[j] = s * (1.f + z[j] * (1.f - s));
       }
-      uint4* hp = reinterpret_cast<uint4*>(H + (size_t)r * NCOL + c0);
+      uint4* hp = reinterpret_cast<uint4*>(H + (size_t)r * ld + c0);
       hp[0] = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
       hp[1] = make_uint4(pack_bf16(h[8], h[9]), pack_bf16(h[10], h[11]), pack_bf16(h[12], h[13]),
                          pack_bf16(h[14], h[15]));
 #pragma unroll
       for (int j = 0; j < 16; ++j) HT[(size_t)(c0 + j) * Bt + r] = __float2bfloat16_rn(h[j]);
-      float4* sp = reinterpret_cast<float4*>(S + (size_t)r * NCOL + c0);
+      float4* dp = reinterpret_cast<float4*>(S + (size_t)r * ld + c0);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) sp[q] = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
+      for (int q = 0; q < 4; ++q) dp[q] = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
     }
   }
 };
 
 // weight gradient: rows are output units; rows beyond the padded width are not stored
-template <int NCOL> struct DwEpi {
-  float* G;  // [out_p][NCOL]
-  int out_p;
-  __device__ void row(uint32_t taddr, int row, int m0, int) {
+struct DwEpi {
+  float* G;  // [out_p][ld]
+  int out_p, ld;
+  __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int r = m0 + row;
-#pragma unroll 1
-    for (int c0 = 0; c0 < NCOL; c0 += 16) {
+#pragma unroll
+    for (int q0 = 0; q0 < MLP_NC; q0 += 16) {
       float a[16];
-      umma::tmem_ld16(taddr + c0, a);
+      umma::tmem_ld16(taddr + q0, a);
       umma::tmem_ld_wait();
       if (r >= out_p) continue;
-      float4* g = reinterpret_cast<float4*>(G + (size_t)r * NCOL + c0);
+      float4* g = reinterpret_cast<float4*>(G + (size_t)r * ld + sp * MLP_NC + q0);
 #pragma unroll
       for (int q = 0; q < 4; ++q) g[q] = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
     }
@@ -104,29 +112,30 @@ template <int NCOL> struct DwEpi {
 };
 
 // input gradient of a hidden layer: dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1}), BF16, both layouts
-template <int NCOL> struct DhEpi {
-  const float* S;  // [Bt][NCOL]
-  bf16* dZ;        // [Bt][NCOL]
-  bf16* dZT;       // [NCOL][Bt]
-  int Bt;
-  __device__ void row(uint32_t taddr, int row, int m0, int) {
+struct DhEpi {
+  const float* S;  // [Bt][ld]
+  bf16* dZ;        // [Bt][ld]
+  bf16* dZT;       // [ld][Bt]
+  int Bt, ld;
+  __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int r = m0 + row;
-#pragma unroll 1
-    for (int c0 = 0; c0 < NCOL; c0 += 16) {
+#pragma unroll
+    for (int q0 = 0; q0 < MLP_NC; q0 += 16) {
+      const int c0 = sp * MLP_NC + q0;
       float a[16];
-      umma::tmem_ld16(taddr + c0, a);
+      umma::tmem_ld16(taddr + q0, a);
       umma::tmem_ld_wait();
-      const float4* sp = reinterpret_cast<const float4*>(S + (size_t)r * NCOL + c0);
+      const float4* sp4 = reinterpret_cast<const float4*>(S + (size_t)r * ld + c0);
       float d[16];
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        const float4 s = sp[q];
+        const float4 s = sp4[q];
         d[4 * q] = a[4 * q] * s.x;
         d[4 * q + 1] = a[4 * q + 1] * s.y;
         d[4 * q + 2] = a[4 * q + 2] * s.z;
         d[4 * q + 3] = a[4 * q + 3] * s.w;
       }
-      uint4* dp = reinterpret_cast<uint4*>(dZ + (size_t)r * NCOL + c0);
+      uint4* dp = reinterpret_cast<uint4*>(dZ + (size_t)r * ld + c0);
       dp[0] = make_uint4(pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]), pack_bf16(d[4], d[5]), pack_bf16(d[6], d[7]));
       dp[1] = make_uint4(pack_bf16(d[8], d[9]), pack_bf16(d[10], d[11]), pack_bf16(d[12], d[13]),
                          pack_bf16(d[14], d[15]));
@@ -138,37 +147,40 @@ template <int NCOL> struct DhEpi {
 
 // ---------------------------------------------------------------- small kernels
 // minibatch rows of the dataset (training) or of a caller's chunk (idx == null): BF16 input
-// rows and their transpose, FP32 targets; rows >= nvalid are zero
+// rows and their transpose, FP32 targets; rows >= nvalid are zero.  The padding columns past
+// in_dim were zeroed with the buffers and are never written
 __global__ void k_mlp_gather(const float* __restrict__ X, const float* __restrict__ T, const int* __restrict__ idx,
-                             const int* counter, int in_dim, int out_dim, int out_p, int Bt, int nvalid, bf16* H0,
-                             bf16* HT0, float* Tb) {
+                             const int* counter, int in_dim, int out_dim, int Bt, int nvalid, bf16* H0, bf16* HT0,
+                             float* Tb) {
   const int step = counter ? *counter : 0;
-  const int total = Bt * PADW;
+  const int total = Bt * max(in_dim, out_dim);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
     const int c = t / Bt, r = t % Bt;  // c-major: the transposed store is coalesced
-    float v = 0.f;
     long long src = -1;
     if (r < nvalid) src = idx ? (long long)idx[(long long)step * Bt + r] : (long long)r;
-    if (src >= 0 && c < in_dim) v = X[src * in_dim + c];
-    const bf16 b = __float2bfloat16_rn(v);
-    HT0[(size_t)c * Bt + r] = b;
-    H0[(size_t)r * PADW + c] = b;
-    if (c < out_p) Tb[(size_t)r * out_p + c] = (src >= 0 && c < out_dim && T) ? T[src * out_dim + c] : 0.f;
+    if (c < in_dim) {
+      const bf16 b = __float2bfloat16_rn(src >= 0 ? X[src * in_dim + c] : 0.f);
+      HT0[(size_t)c * Bt + r] = b;
+      H0[(size_t)r * PADW + c] = b;
+    }
+    if (T && c < out_dim) Tb[(size_t)r * out_dim + c] = src >= 0 ? T[src * out_dim + c] : 0.f;
   }
 }
 
 // mean squared error over the valid rows and the first out_dim outputs; its gradient
-// 2 (y - t) / (n out_dim) in both layouts (BF16)
+// 2 (y - t) / (n out_dim) in both layouts (BF16).  Only the out_dim real columns are visited:
+// the padding columns of dZ and dZT were zeroed with the buffers and stay zero (over all 64
+// columns of 512 rows one block took 40 us, over the surrogate's two it takes 4.5 us)
 __global__ void k_mlp_loss(const float* __restrict__ Y, const float* __restrict__ Tb, int nvalid, int out_dim,
-                           int out_p, int Bt, bf16* dZ, bf16* dZT, float* loss, const int* counter) {
+                           int out_p, int Bt, bf16* dZ, bf16* dZT, float* loss, int* counter) {
   __shared__ float red[32];
   const float scale = 2.f / ((float)nvalid * (float)out_dim);
   float acc = 0.f;
-  for (int t = threadIdx.x; t < Bt * out_p; t += blockDim.x) {
+  for (int t = threadIdx.x; t < Bt * out_dim; t += blockDim.x) {
     const int j = t / Bt, r = t % Bt;
     float g = 0.f;
-    if (r < nvalid && j < out_dim) {
-      const float e = Y[(size_t)r * out_p + j] - Tb[(size_t)r * out_p + j];
+    if (r < nvalid) {
+      const float e = Y[(size_t)r * out_dim + j] - Tb[(size_t)r * out_dim + j];
       acc = fmaf(e, e, acc);
       g = scale * e;
     }
@@ -182,59 +194,125 @@ __global__ void k_mlp_loss(const float* __restrict__ Y, const float* __restrict_
   if (threadIdx.x == 0) {
     float s = 0.f;
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w];
-    loss[counter ? *counter : 0] = s / ((float)nvalid * (float)out_dim);
+    const int step = counter ? *counter : 0;
+    loss[step] = s / ((float)nvalid * (float)out_dim);
+    if (counter) *counter = step + 1;  // the update that follows is step *counter - 1
   }
 }
 
-// bias gradient: column sums of dZ in row order (deterministic)
-__global__ void k_mlp_bias_grad(const bf16* __restrict__ dZ, int Bt, int out_p, float* gb) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= out_p) return;
-  float s = 0.f;
-  for (int r = 0; r < Bt; ++r) s += __bfloat162float(dZ[(size_t)r * out_p + c]);
-  gb[c] = s;
-}
-
-// Adam on the flat FP32 parameters (Kingma & Ba), learning rate interpolated linearly from
-// lr0 to lr1 over the run; the step number comes from the device counter
-__global__ void k_mlp_adam(float* P, const float* __restrict__ G, float* M, float* V, long long n, const int* counter,
-                           float lr0, float lr1, long long total_steps, float b1, float b2, float eps) {
-  const int step = *counter;
-  const float frac = total_steps > 1 ? (float)step / (float)(total_steps - 1) : 0.f;
-  const float lr = lr0 + (lr1 - lr0) * frac;
-  const float c1 = 1.f - powf(b1, (float)(step + 1)), c2 = 1.f - powf(b2, (float)(step + 1));
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float g = G[i];
-    const float m = b1 * M[i] + (1.f - b1) * g;
-    const float v = b2 * V[i] + (1.f - b2) * g * g;
-    M[i] = m;
-    V[i] = v;
-    P[i] -= lr * (m / c1) / (sqrtf(v / c2) + eps);
-  }
-}
-
-struct PackLayer {
-  long long w_off;
-  int in_p, out_p;
+struct UpdLayer {
+  long long w_off, b_off;
+  int in_p, out_p, tiles, tiles_i;  // 32 x 32 weight tiles of the layer, and per row of tiles
   bf16* W;
   bf16* WT;
+  const bf16* dZ;  // [Bt][out]
 };
-struct PackArgs {
-  PackLayer l[NL];
+struct UpdArgs {
+  UpdLayer l[NL];
 };
-// BF16 copies of the weights, [out][in] and [in][out]; optionally advances the step counter
-__global__ void k_mlp_pack(const float* __restrict__ P, PackArgs a, int* counter) {
-  const PackLayer& L = a.l[blockIdx.y];
-  const int total = L.in_p * L.out_p;
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int o = t / L.in_p, i = t % L.in_p;
-    const bf16 b = __float2bfloat16_rn(P[L.w_off + t]);
-    L.W[t] = b;
-    L.WT[(size_t)i * L.out_p + o] = b;
-  }
-  if (counter && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicAdd(counter, 1);
+struct AdamArgs {
+  float *M, *V;
+  const int* counter;
+  float lr0, lr1;
+  long long total_steps;
+  float b1, b2, eps;
+};
+__device__ __forceinline__ float adam_step(float* P, const AdamArgs& a, long long i, float g, float lr, float c1,
+                                           float c2) {
+  const float m = a.b1 * a.M[i] + (1.f - a.b1) * g;
+  const float v = a.b2 * a.V[i] + (1.f - a.b2) * g * g;
+  a.M[i] = m;
+  a.V[i] = v;
+  const float p = P[i] - lr * (m / c1) / (sqrtf(v / c2) + a.eps);
+  P[i] = p;
+  return p;
 }
-
+constexpr int UPD_THREADS = 256;
+constexpr int UPD_BIAS = 32;    // output units per bias block
+constexpr int UPD_ROWS = 128;   // rows of dZ staged per round of a bias block (the batch is a multiple)
+// What follows a backward pass, in one launch: blocks of 32 x 32 weights and blocks of UPD_BIAS
+// output units.  UPD_ADAM: the Adam step (Kingma & Ba; learning rate interpolated linearly from
+// lr0 to lr1 over the run, the step number from the device counter).  UPD_PACK: the BF16 copies of
+// the weights, [out][in] and, through a shared-memory tile, [in][out].  UPD_BIAS_GRAD: the bias
+// gradients, summed in the order of the rows by one thread per unit, over a tile of rows that the
+// whole block has brought into shared memory (the additions of a tile take 0.3 us; a thread that
+// loads its own rows waits for memory between them).  These are 1.3 MB of reads and writes, bound by launch latency and the depth of each
+// chain: as an Adam launch, a pack launch and a sum by one thread per unit and layer they took
+// 9 + 6.5 + 4 x 30 us per training step, together 9.7 us.
+enum { UPD_ADAM = 1, UPD_PACK = 2, UPD_BIAS_GRAD = 4 };
+__global__ void __launch_bounds__(UPD_THREADS)
+    k_mlp_update(float* P, float* G, const __grid_constant__ UpdArgs u, AdamArgs a, int Bt, int what) {
+  __shared__ bf16 tile[32][33];
+  __shared__ bf16 stage[UPD_ROWS][32];
+  int blk = blockIdx.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float lr = 0.f, c1 = 1.f, c2 = 1.f;
+  if (what & UPD_ADAM) {
+    const int step = *a.counter - 1;  // advanced by the loss kernel
+    const float frac = a.total_steps > 1 ? (float)step / (float)(a.total_steps - 1) : 0.f;
+    lr = a.lr0 + (a.lr1 - a.lr0) * frac;
+    c1 = 1.f - powf(a.b1, (float)(step + 1));
+    c2 = 1.f - powf(a.b2, (float)(step + 1));
+  }
+#pragma unroll 1
+  for (int l = 0; l < NL; ++l) {
+    const UpdLayer& L = u.l[l];
+    if (blk < L.tiles) {
+      const int o0 = blk / L.tiles_i * 32, i0 = blk % L.tiles_i * 32;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int o = warp + 8 * q;
+        const long long e = L.w_off + (long long)(o0 + o) * L.in_p + i0 + lane;
+        const float p = (what & UPD_ADAM) ? adam_step(P, a, e, G[e], lr, c1, c2) : P[e];
+        if (what & UPD_PACK) {
+          const bf16 b = __float2bfloat16_rn(p);
+          L.W[(size_t)(o0 + o) * L.in_p + i0 + lane] = b;
+          tile[o][lane] = b;
+        }
+      }
+      if (what & UPD_PACK) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const int i = warp + 8 * q;
+          L.WT[(size_t)(i0 + i) * L.out_p + o0 + lane] = tile[lane][i];
+        }
+      }
+      return;
+    }
+    blk -= L.tiles;
+    const int nb = L.out_p / UPD_BIAS;
+    if (blk < nb) {
+      if (!(what & UPD_BIAS_GRAD)) return;
+      const int o = blk * UPD_BIAS + lane;
+      float s = 0.f;
+      const bf16* src = L.dZ + (size_t)warp * L.out_p + o;
+      bf16 v[UPD_ROWS / 8];
+      auto load = [&](int r0) {
+#pragma unroll
+        for (int q = 0; q < UPD_ROWS / 8; ++q) v[q] = src[(size_t)(r0 + 8 * q) * L.out_p];
+      };
+      load(0);
+      for (int r0 = 0; r0 < Bt; r0 += UPD_ROWS) {
+        __syncthreads();  // the previous tile has been summed
+#pragma unroll
+        for (int q = 0; q < UPD_ROWS / 8; ++q) stage[warp + 8 * q][lane] = v[q];
+        __syncthreads();
+        if (r0 + UPD_ROWS < Bt) load(r0 + UPD_ROWS);  // lands while this tile is summed
+        if (warp == 0) {
+#pragma unroll 32
+          for (int q = 0; q < UPD_ROWS; ++q) s += __bfloat162float(stage[q][lane]);
+        }
+      }
+      if (warp == 0) {
+        G[L.b_off + o] = s;
+        if (what & UPD_ADAM) adam_step(P, a, L.b_off + o, s, lr, c1, c2);
+      }
+      return;
+    }
+    blk -= nb;
+  }
+}
 struct Layer {
   int in, out, in_p, out_p, out_m;  // out_m: rows of dZ^T (at least one 128-row M tile)
   long long w_off, b_off;
@@ -271,8 +349,9 @@ struct kura_mlp {
   float *Tb = nullptr, *loss = nullptr, *Xin = nullptr, *Tin = nullptr;
   int *counter = nullptr, *err = nullptr;
   CUtensorMap fA[NL], fX[NL], wA[NL], wX[NL], hA[NL], hX[NL];
-  cudaStream_t st = nullptr;
+  cudaStream_t st = nullptr, st2 = nullptr;  // st2: the weight gradients, beside the input gradients
   cudaEvent_t ev[2] = {nullptr, nullptr};
+  cudaEvent_t evz[NL] = {}, evw = nullptr;  // dZ of a layer is ready; the weight gradients are
   std::vector<void*> allocs;
 };
 
@@ -304,85 +383,69 @@ cudaError_t dalloc(kura_mlp* m, T** p, size_t count) {
 
 constexpr unsigned long long GEMM_LIMIT_NS = 20000000000ull;
 
-template <int NCOL, class Epi>
-cudaError_t gemm(kura_mlp* m, const CUtensorMap& a, const CUtensorMap& x, int mtiles, int ktiles, const Epi& e) {
-  kura::k_tensor_gemm<NCOL, Epi><<<std::min(mtiles, m->sms), kura::TG_THREADS, kura::TGCfg<NCOL>::SMEM, m->st>>>(
-      a, x, mtiles, mtiles, ktiles, 1, 0, e, m->err, GEMM_LIMIT_NS, nullptr);
+template <class Epi>
+cudaError_t gemm(kura_mlp* m, cudaStream_t st, const CUtensorMap& a, const CUtensorMap& x, int mtiles, int width,
+                 int ktiles, const Epi& e) {
+  constexpr int NC = kura::MLP_NC;
+  const int nsplit = width / NC;
+  kura::k_tensor_gemm<NC, Epi><<<std::min(mtiles * nsplit, m->sms), kura::TG_THREADS, kura::TGCfg<NC>::SMEM, st>>>(
+      a, x, mtiles, mtiles, ktiles, nsplit, NC, e, m->err, GEMM_LIMIT_NS, nullptr);
   return cudaGetLastError();
 }
-
-template <int NCOL>
-cudaError_t set_attrs_n() {
-  cudaError_t e = cudaFuncSetAttribute(kura::k_tensor_gemm<NCOL, kura::FwdEpi<NCOL>>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, kura::TGCfg<NCOL>::SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kura::k_tensor_gemm<NCOL, kura::DwEpi<NCOL>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kura::TGCfg<NCOL>::SMEM);
-  if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(kura::k_tensor_gemm<NCOL, kura::DhEpi<NCOL>>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             kura::TGCfg<NCOL>::SMEM);
-  return e;
+template <class Epi>
+cudaError_t set_attr() {
+  return cudaFuncSetAttribute(kura::k_tensor_gemm<kura::MLP_NC, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              kura::TGCfg<kura::MLP_NC>::SMEM);
 }
 
-// dispatch on a padded width (64, 128, 256)
-template <class F>
-cudaError_t by_width(int w, F&& f) {
-  switch (w) {
-    case 64: return f(std::integral_constant<int, 64>());
-    case 128: return f(std::integral_constant<int, 128>());
-    case 256: return f(std::integral_constant<int, 256>());
-    default: return cudaErrorInvalidValue;
-  }
-}
-
-cudaError_t forward(kura_mlp* m) {
+// the first `rows` rows of the batch (rounded up to row tiles)
+cudaError_t forward(kura_mlp* m, int rows) {
   for (int l = 0; l < NL; ++l) {
     const Layer& L = m->L[l];
     const bool last = (l == NL - 1);
-    cudaError_t e = by_width(L.out_p, [&](auto w) {
-      constexpr int W = decltype(w)::value;
-      kura::FwdEpi<W> ep{m->P + L.b_off, last ? 1 : 0, m->Bt, last ? nullptr : m->H[l + 1],
-                         last ? nullptr : m->HT[l + 1], last ? nullptr : m->S[l + 1], last ? m->Y : nullptr};
-      return gemm<W>(m, m->fA[l], m->fX[l], m->Bt / kura::TG_BM, L.in_p / kura::TG_BK, ep);
-    });
+    kura::FwdEpi ep{m->P + L.b_off, last ? 1 : 0, m->Bt, L.out_p, L.out, last ? nullptr : m->H[l + 1],
+                    last ? nullptr : m->HT[l + 1], last ? nullptr : m->S[l + 1], last ? m->Y : nullptr};
+    // of the last layer only the column blocks that hold real outputs
+    const int width = last ? kura::round_up(L.out, kura::MLP_NC) : L.out_p;
+    cudaError_t e = gemm(m, m->st, m->fA[l], m->fX[l], kura::round_up(rows, kura::TG_BM) / kura::TG_BM, width,
+                         L.in_p / kura::TG_BK, ep);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
+// The input gradients follow one another; each layer's weight gradient needs only that layer's dZ
+// and runs beside them on the second stream.
 cudaError_t backward(kura_mlp* m) {
-  for (int l = NL - 1; l >= 0; --l) {
+  cudaError_t e = cudaSuccess;
+  for (int l = NL - 1; l >= 0 && e == cudaSuccess; --l) {
     const Layer& L = m->L[l];
-    cudaError_t e = by_width(L.in_p, [&](auto w) {
-      constexpr int W = decltype(w)::value;
-      kura::DwEpi<W> ep{m->G + L.w_off, L.out_p};
-      return gemm<W>(m, m->wA[l], m->wX[l], L.out_m / kura::TG_BM, m->Bt / kura::TG_BK, ep);
-    });
-    if (e != cudaSuccess) return e;
-    kura::k_mlp_bias_grad<<<(L.out_p + 127) / 128, 128, 0, m->st>>>(m->dZ[l], m->Bt, L.out_p, m->G + L.b_off);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    if (l == 0) break;
-    e = by_width(L.in_p, [&](auto w) {
-      constexpr int W = decltype(w)::value;
-      kura::DhEpi<W> ep{m->S[l], m->dZ[l - 1], m->dZT[l - 1], m->Bt};
-      return gemm<W>(m, m->hA[l], m->hX[l], m->Bt / kura::TG_BM, L.out_p / kura::TG_BK, ep);
-    });
-    if (e != cudaSuccess) return e;
+    e = cudaEventRecord(m->evz[l], m->st);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(m->st2, m->evz[l], 0);
+    kura::DwEpi dw{m->G + L.w_off, L.out_p, L.in_p};
+    if (e == cudaSuccess)
+      e = gemm(m, m->st2, m->wA[l], m->wX[l], L.out_m / kura::TG_BM, L.in_p, m->Bt / kura::TG_BK, dw);
+    if (l == 0 || e != cudaSuccess) break;
+    kura::DhEpi dh{m->S[l], m->dZ[l - 1], m->dZT[l - 1], m->Bt, L.in_p};
+    e = gemm(m, m->st, m->hA[l], m->hX[l], m->Bt / kura::TG_BM, L.in_p, L.out_p / kura::TG_BK, dh);
   }
-  return cudaSuccess;
+  if (e == cudaSuccess) e = cudaEventRecord(m->evw, m->st2);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(m->st, m->evw, 0);
+  return e;
 }
 
-kura::PackArgs pack_args(kura_mlp* m) {
-  kura::PackArgs a;
-  for (int l = 0; l < NL; ++l) a.l[l] = {m->L[l].w_off, m->L[l].in_p, m->L[l].out_p, m->W[l], m->WT[l]};
-  return a;
-}
-
-cudaError_t pack(kura_mlp* m, int* counter) {
-  kura::k_mlp_pack<<<dim3(64, NL), 256, 0, m->st>>>(m->P, pack_args(m), counter);
+cudaError_t update(kura_mlp* m, const kura::AdamArgs& a, int what) {
+  kura::UpdArgs u;
+  int blocks = 0;
+  for (int l = 0; l < NL; ++l) {
+    const Layer& L = m->L[l];
+    u.l[l] = {L.w_off, L.b_off, L.in_p, L.out_p, (L.in_p / 32) * (L.out_p / 32), L.in_p / 32, m->W[l], m->WT[l], m->dZ[l]};
+    blocks += u.l[l].tiles + L.out_p / kura::UPD_BIAS;
+  }
+  kura::k_mlp_update<<<blocks, kura::UPD_THREADS, 0, m->st>>>(m->P, m->G, u, a, m->Bt, what);
   return cudaGetLastError();
 }
+cudaError_t pack(kura_mlp* m) { return update(m, kura::AdamArgs{}, kura::UPD_PACK); }
 
 int check_err(kura_mlp* m) {
   int e = 0;
@@ -462,8 +525,8 @@ extern "C" int kura_mlp_create(int32_t in_dim, int32_t hidden, int32_t out_dim, 
     if (e == cudaSuccess) e = dalloc(m, &m->dZ[l], (size_t)Bt * L.out_p);
     if (e == cudaSuccess) e = dalloc(m, &m->dZT[l], (size_t)Bt * L.out_m);
   }
-  if (e == cudaSuccess) e = dalloc(m, &m->Y, (size_t)Bt * m->L[NL - 1].out_p);
-  if (e == cudaSuccess) e = dalloc(m, &m->Tb, (size_t)Bt * m->L[NL - 1].out_p);
+  if (e == cudaSuccess) e = dalloc(m, &m->Y, (size_t)Bt * out_dim);
+  if (e == cudaSuccess) e = dalloc(m, &m->Tb, (size_t)Bt * out_dim);
   if (e == cudaSuccess) e = dalloc(m, &m->Xin, (size_t)Bt * in_dim);
   if (e == cudaSuccess) e = dalloc(m, &m->Tin, (size_t)Bt * out_dim);
   if (e == cudaSuccess) e = dalloc(m, &m->loss, 1);
@@ -472,21 +535,24 @@ extern "C" int kura_mlp_create(int32_t in_dim, int32_t hidden, int32_t out_dim, 
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&m->ev[0]);
   if (e == cudaSuccess) e = cudaEventCreate(&m->ev[1]);
-  if (e == cudaSuccess) e = set_attrs_n<64>();
-  if (e == cudaSuccess) e = set_attrs_n<128>();
-  if (e == cudaSuccess) e = set_attrs_n<256>();
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->st2, cudaStreamNonBlocking);
+  for (cudaEvent_t* v : {&m->evz[0], &m->evz[1], &m->evz[2], &m->evz[3], &m->evw})
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = set_attr<kura::FwdEpi>();
+  if (e == cudaSuccess) e = set_attr<kura::DwEpi>();
+  if (e == cudaSuccess) e = set_attr<kura::DhEpi>();
   if (e != cudaSuccess)
     return bail(mlp_fail(e == cudaErrorMemoryAllocation ? KURA_ERR_NOMEM : KURA_ERR_CUDA, cudaGetErrorString(e)));
   // tensor maps of every GEMM operand (the buffers never move)
   for (int l = 0; l < NL; ++l) {
     const Layer& L = m->L[l];
     int bad = kura::make_tmap_bf16(&m->fA[l], m->H[l], L.in_p, Bt, kura::TG_BM);
-    bad |= kura::make_tmap_bf16(&m->fX[l], m->W[l], L.in_p, L.out_p, std::min(256, L.out_p));
+    bad |= kura::make_tmap_bf16(&m->fX[l], m->W[l], L.in_p, L.out_p, kura::MLP_NC);
     bad |= kura::make_tmap_bf16(&m->wA[l], m->dZT[l], Bt, L.out_m, kura::TG_BM);
-    bad |= kura::make_tmap_bf16(&m->wX[l], m->HT[l], Bt, L.in_p, std::min(256, L.in_p));
+    bad |= kura::make_tmap_bf16(&m->wX[l], m->HT[l], Bt, L.in_p, kura::MLP_NC);
     if (l > 0) {
       bad |= kura::make_tmap_bf16(&m->hA[l], m->dZ[l], L.out_p, Bt, kura::TG_BM);
-      bad |= kura::make_tmap_bf16(&m->hX[l], m->WT[l], L.out_p, L.in_p, std::min(256, L.in_p));
+      bad |= kura::make_tmap_bf16(&m->hX[l], m->WT[l], L.out_p, L.in_p, kura::MLP_NC);
     }
     if (bad) return bail(mlp_fail(KURA_ERR_CUDA, "cuTensorMapEncodeTiled failed for an MLP operand"));
   }
@@ -499,7 +565,7 @@ extern "C" int kura_mlp_create(int32_t in_dim, int32_t hidden, int32_t out_dim, 
       for (int i = 0; i < L.in; ++i) p[L.w_off + (long long)o * L.in_p + i] = (float)((2 * kura::uniform01(s) - 1) * a);
   }
   e = cudaMemcpy(m->P, p.data(), sizeof(float) * off, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = pack(m, nullptr);
+  if (e == cudaSuccess) e = pack(m);
   if (e == cudaSuccess) e = cudaStreamSynchronize(m->st);
   if (e != cudaSuccess) return bail(mlp_fail(KURA_ERR_CUDA, cudaGetErrorString(e)));
   *out = m;
@@ -509,11 +575,16 @@ extern "C" int kura_mlp_create(int32_t in_dim, int32_t hidden, int32_t out_dim, 
 extern "C" void kura_mlp_destroy(kura_mlp* m) {
   if (!m) return;
   cudaSetDevice(m->device);
-  if (m->st) cudaStreamSynchronize(m->st);
+  for (cudaStream_t st : {m->st, m->st2})
+    if (st) cudaStreamSynchronize(st);
   for (void* p : m->allocs) cudaFree(p);
   for (cudaEvent_t v : m->ev)
     if (v) cudaEventDestroy(v);
-  if (m->st) cudaStreamDestroy(m->st);
+  for (cudaEvent_t v : m->evz)
+    if (v) cudaEventDestroy(v);
+  if (m->evw) cudaEventDestroy(m->evw);
+  for (cudaStream_t st : {m->st, m->st2})
+    if (st) cudaStreamDestroy(st);
   delete m;
 }
 
@@ -547,7 +618,7 @@ extern "C" int kura_mlp_set_params(kura_mlp* m, const float* params, int64_t cou
   }
   MLPCU(cudaStreamSynchronize(m->st));
   MLPCU(cudaMemcpy(m->P, pad.data(), sizeof(float) * m->nparam, cudaMemcpyHostToDevice));
-  MLPCU(pack(m, nullptr));
+  MLPCU(pack(m));
   MLPCU(cudaStreamSynchronize(m->st));
   return KURA_OK;
 }
@@ -555,16 +626,14 @@ extern "C" int kura_mlp_set_params(kura_mlp* m, const float* params, int64_t cou
 extern "C" int kura_mlp_forward(kura_mlp* m, const float* x, int64_t n, float* y) {
   if (!m || !x || !y || n < 0) return mlp_fail(KURA_ERR_INVALID, "bad argument");
   MLPCU(cudaSetDevice(m->device));
-  const Layer& Lo = m->L[NL - 1];
   for (int64_t r0 = 0; r0 < n; r0 += m->Bt) {
     const int rows = (int)std::min<int64_t>(m->Bt, n - r0);
     MLPCU(cudaMemcpyAsync(m->Xin, x + r0 * m->in_dim, sizeof(float) * rows * m->in_dim, cudaMemcpyHostToDevice, m->st));
-    kura::k_mlp_gather<<<64, 256, 0, m->st>>>(m->Xin, nullptr, nullptr, nullptr, m->in_dim, m->out_dim, Lo.out_p,
-                                              m->Bt, rows, m->H[0], m->HT[0], m->Tb);
+    kura::k_mlp_gather<<<64, 256, 0, m->st>>>(m->Xin, nullptr, nullptr, nullptr, m->in_dim, m->out_dim, m->Bt, rows,
+                                              m->H[0], m->HT[0], m->Tb);
     MLPCU(cudaGetLastError());
-    MLPCU(forward(m));
-    MLPCU(cudaMemcpy2DAsync(y + r0 * m->out_dim, sizeof(float) * m->out_dim, m->Y, sizeof(float) * Lo.out_p,
-                            sizeof(float) * m->out_dim, rows, cudaMemcpyDeviceToHost, m->st));
+    MLPCU(forward(m, rows));
+    MLPCU(cudaMemcpyAsync(y + r0 * m->out_dim, m->Y, sizeof(float) * m->out_dim * rows, cudaMemcpyDeviceToHost, m->st));
     MLPCU(cudaStreamSynchronize(m->st));
     int rc = check_err(m);
     if (rc != KURA_OK) return rc;
@@ -580,14 +649,15 @@ extern "C" int kura_mlp_gradients(kura_mlp* m, const float* x, const float* targ
   const Layer& Lo = m->L[NL - 1];
   MLPCU(cudaMemcpyAsync(m->Xin, x, sizeof(float) * n * m->in_dim, cudaMemcpyHostToDevice, m->st));
   MLPCU(cudaMemcpyAsync(m->Tin, target, sizeof(float) * n * m->out_dim, cudaMemcpyHostToDevice, m->st));
-  kura::k_mlp_gather<<<64, 256, 0, m->st>>>(m->Xin, m->Tin, nullptr, nullptr, m->in_dim, m->out_dim, Lo.out_p, m->Bt,
-                                            (int)n, m->H[0], m->HT[0], m->Tb);
+  kura::k_mlp_gather<<<64, 256, 0, m->st>>>(m->Xin, m->Tin, nullptr, nullptr, m->in_dim, m->out_dim, m->Bt, (int)n,
+                                            m->H[0], m->HT[0], m->Tb);
   MLPCU(cudaGetLastError());
-  MLPCU(forward(m));
+  MLPCU(forward(m, m->Bt));
   kura::k_mlp_loss<<<1, 1024, 0, m->st>>>(m->Y, m->Tb, (int)n, m->out_dim, Lo.out_p, m->Bt, m->dZ[NL - 1],
                                           m->dZT[NL - 1], m->loss, nullptr);
   MLPCU(cudaGetLastError());
   MLPCU(backward(m));
+  MLPCU(update(m, kura::AdamArgs{}, kura::UPD_BIAS_GRAD));
   std::vector<float> pad(m->nparam);
   float l = 0.f;
   MLPCU(cudaStreamSynchronize(m->st));
@@ -642,22 +712,19 @@ extern "C" int kura_mlp_train(kura_mlp* m, const float* x, const float* target, 
     // one training step, captured
     MLPCU(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = cudaSuccess;
-    kura::k_mlp_gather<<<64, 256, 0, m->st>>>(dX, dT, dI, m->counter, m->in_dim, m->out_dim, Lo.out_p, m->Bt, m->Bt,
-                                              m->H[0], m->HT[0], m->Tb);
+    kura::k_mlp_gather<<<64, 256, 0, m->st>>>(dX, dT, dI, m->counter, m->in_dim, m->out_dim, m->Bt, m->Bt, m->H[0],
+                                              m->HT[0], m->Tb);
     e = cudaGetLastError();
-    if (e == cudaSuccess) e = forward(m);
+    if (e == cudaSuccess) e = forward(m, m->Bt);
     if (e == cudaSuccess) {
       kura::k_mlp_loss<<<1, 1024, 0, m->st>>>(m->Y, m->Tb, m->Bt, m->out_dim, Lo.out_p, m->Bt, m->dZ[NL - 1],
                                               m->dZT[NL - 1], dL, m->counter);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = backward(m);
-    if (e == cudaSuccess) {
-      kura::k_mlp_adam<<<160, 256, 0, m->st>>>(m->P, m->G, m->Mo, m->Vo, m->nparam, m->counter, lr, lr_final, total,
-                                               0.9f, 0.999f, 1e-8f);
-      e = cudaGetLastError();
-    }
-    if (e == cudaSuccess) e = pack(m, m->counter);
+    if (e == cudaSuccess)
+      e = update(m, kura::AdamArgs{m->Mo, m->Vo, m->counter, lr, lr_final, total, 0.9f, 0.999f, 1e-8f},
+                 kura::UPD_ADAM | kura::UPD_PACK | kura::UPD_BIAS_GRAD);
     cudaError_t ce = cudaStreamEndCapture(m->st, &g);
     MLPCU(e);
     MLPCU(ce);

@@ -64,6 +64,31 @@ def test_gradients_match_oracle(native, n):
         assert k == g.size
 
 
+@pytest.mark.parametrize("in_dim,hidden,out_dim,batch,n", [(64, 128, 33, 128, 1), (1, 64, 64, 256, 129), (17, 256, 32, 384, 384)])
+def test_column_blocks_match_oracle(native, in_dim, hidden, out_dim, batch, n):
+    """Widths at the edges of the GEMMs' 32-column blocks, part-filled row tiles and batches; the tolerances are
+    those of the tests above (the same BF16 storage, FP32 sums in another order)."""
+    rng = np.random.default_rng(n)
+    x = rng.normal(size=(n, in_dim)).astype(np.float32)
+    t = rng.normal(size=(n, out_dim)).astype(np.float32)
+    dims = mo.dims_of(in_dim, hidden, out_dim)
+    with native.MLP(in_dim, out_dim, hidden=hidden, batch=batch, seed=4) as m:
+        p = m.params() + rng.normal(0, 0.02, m.param_count).astype(np.float32)
+        m.set_params(p)
+        ref, _ = mo.forward(p, x, dims, bf16=True)
+        for _ in range(2):  # a chunk of fewer rows leaves nothing behind for the next
+            assert np.max(np.abs(m.forward(x) - ref)) <= 2e-3 * np.max(np.abs(ref)) + 1e-6
+            m.forward(x[:1])
+        loss, g = m.gradients(x, t)
+        lref, gref = mo.loss_and_grads(p, x, t, dims, bf16=True)
+        assert abs(loss - lref) <= 1e-3 * lref
+        k = 0
+        for i, o in zip(dims[:-1], dims[1:]):
+            for size in (o * i, o):
+                assert rel(g[k:k + size], gref[k:k + size]) < 1e-2, (k, size)
+                k += size
+
+
 def test_one_training_step_is_oracle_adam(native):
     with native.MLP(IN, OUT, hidden=256, batch=256, seed=9) as m:
         p0 = m.params().astype(np.float64)
