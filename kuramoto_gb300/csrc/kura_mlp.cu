@@ -49,6 +49,7 @@ constexpr int MLP_NC = 32;
 // forward: z = acc + b; hidden layers store silu(z) (row-major and transposed, BF16) and
 // silu'(z); the last layer stores the real outputs of z, packed [Bt][out_dim]
 struct FwdEpi {
+  static constexpr bool F16 = false;
   const float* bias;
   int last, Bt, ld, out_dim;
   bf16* H;   // [Bt][ld]
@@ -94,6 +95,7 @@ struct FwdEpi {
 
 // weight gradient: rows are output units; rows beyond the padded width are not stored
 struct DwEpi {
+  static constexpr bool F16 = false;
   float* G;  // [out_p][ld]
   int out_p, ld;
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
@@ -113,6 +115,7 @@ struct DwEpi {
 
 // input gradient of a hidden layer: dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1}), BF16, both layouts
 struct DhEpi {
+  static constexpr bool F16 = false;
   const float* S;  // [Bt][ld]
   bf16* dZ;        // [Bt][ld]
   bf16* dZT;       // [ld][Bt]
@@ -546,13 +549,13 @@ extern "C" int kura_mlp_create(int32_t in_dim, int32_t hidden, int32_t out_dim, 
   // tensor maps of every GEMM operand (the buffers never move)
   for (int l = 0; l < NL; ++l) {
     const Layer& L = m->L[l];
-    int bad = kura::make_tmap_bf16(&m->fA[l], m->H[l], L.in_p, Bt, kura::TG_BM);
-    bad |= kura::make_tmap_bf16(&m->fX[l], m->W[l], L.in_p, L.out_p, kura::MLP_NC);
-    bad |= kura::make_tmap_bf16(&m->wA[l], m->dZT[l], Bt, L.out_m, kura::TG_BM);
-    bad |= kura::make_tmap_bf16(&m->wX[l], m->HT[l], Bt, L.in_p, kura::MLP_NC);
+    int bad = kura::make_tmap_16(&m->fA[l], false, m->H[l], L.in_p, Bt, kura::TG_BM);
+    bad |= kura::make_tmap_16(&m->fX[l], false, m->W[l], L.in_p, L.out_p, kura::MLP_NC);
+    bad |= kura::make_tmap_16(&m->wA[l], false, m->dZT[l], Bt, L.out_m, kura::TG_BM);
+    bad |= kura::make_tmap_16(&m->wX[l], false, m->HT[l], Bt, L.in_p, kura::MLP_NC);
     if (l > 0) {
-      bad |= kura::make_tmap_bf16(&m->hA[l], m->dZ[l], L.out_p, Bt, kura::TG_BM);
-      bad |= kura::make_tmap_bf16(&m->hX[l], m->WT[l], L.out_p, L.in_p, kura::MLP_NC);
+      bad |= kura::make_tmap_16(&m->hA[l], false, m->dZ[l], L.out_p, Bt, kura::TG_BM);
+      bad |= kura::make_tmap_16(&m->hX[l], false, m->WT[l], L.out_p, L.in_p, kura::MLP_NC);
     }
     if (bad) return bail(mlp_fail(KURA_ERR_CUDA, "cuTensorMapEncodeTiled failed for an MLP operand"));
   }

@@ -4,18 +4,19 @@
 // their own phases, coupling constants and adaptive steps.  Each RHS of the batch is
 // one GEMM over A:
 //   F[i][(cos|sin), b] = sum_j A_ij (cos, sin)(theta_jb)
-// computed as (N A) x [X_hi | X_lo] with X = [cos | sin] split into BF16 hi + lo and FP32
+// computed as (N A) x [X_hi | X_lo] with X = [cos | sin] split into F16 hi + lo and FP32
 // accumulation in TMEM; the GEMM epilogue forms g = c_b (sin F_c - cos F_s) / N directly.
-// For the reference's volcano rule N*A_ij is an integer in [-K, K], exact in BF16, so the
-// product carries the precision of the hi+lo split of X (about 2^-16).  A general
-// adjacency is split as N A = A_hi + A_lo and the term A_lo X_hi comes from a second GEMM
-// pass (split-BF16 hi + lo operands, FP32 accumulation).
+// For the reference's volcano rule N*A_ij is an integer in [-K, K], exact in F16 up to 2048, so
+// the product carries the precision of the hi+lo split of X: 2^-25 absolute, where BF16 parts of
+// the same size and rate hold 2^-18.  A general adjacency is split as 2^p_i N A_ij = A_hi + A_lo
+// with a power of two per row, which keeps a row's largest entry near 2^14 (22 significant bits,
+// and 2^-40 of the largest for the small ones), and the term A_lo X_hi is added by further K steps.
 //
 // The DP45 attempt (dp45_step, dp45.cu:87-141) is a fixed sequence of launches --
 // coefficients, 6 x (stage, GEMM), error norm, controller, outputs -- captured once in a
 // CUDA graph and replayed; every per-trajectory decision (accept/reject, step size, t,
 // output crossings) stays on the device.  The host only polls a completion flag.
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstring>
@@ -26,6 +27,7 @@
 #include "kura_kernels.cuh"
 #include "kura_tensor.h"
 #include "kura_tensor_gemm.cuh"
+#include "kura_tensor_split.cuh"
 
 namespace kura {
 
@@ -58,11 +60,12 @@ struct TView {
   float* ph_lo;
   long long* ph_w;
   float* g;
-  __nv_bfloat16* X;
+  __half* X;
   float2* x32;
   float* fin_theta;
   float* fin_coup;
   float* Flo;  // [2][bp][np] partial couplings of the A_lo pass (general adjacency)
+  const float* rinv;  // [np] 1 / (N 2^p_i): the scale of a row's couplings
 };
 
 // row of X holding column q (0 hi cos, 1 hi sin, 2 lo cos, 3 lo sin) of trajectory b: the
@@ -79,63 +82,56 @@ __device__ __forceinline__ int slot_k7(int rot_g) { return rot_g ? 0 : 6; }
 // ---------------------------------------------------------------- coefficients
 // Per-trajectory sources: src[0] = phases y (first slope, RHS), src[1..6] = stages 2..7
 // of the next attempt (dp45.cu:90-106), src[7] = dense output (set by the output kernels).
-__global__ void k_t_coef(TrajG* traj, TCoef* src, int B, int bp, int fixed, int* any_active) {
-  if (threadIdx.x == 0) {
-    int a0 = 0, a1 = 0;
-    for (int b = 0; b < B; ++b) {
-      const TrajG& T = traj[b];
-      a0 |= (T.status == 0 && T.need_k1);
-      a1 |= (T.status == 0 && T.eval_i >= T.eval_end && T.t < T.t1);
-    }
-    any_active[0] = a0;
-    any_active[1] = a1;
-    any_active[2] = 1;
+// src[0] of the trajectories that still need their first slope; flags[0]: there is one
+__global__ void k_t_first(const TrajG* traj, TCoef* src, int* flags) {
+  const int b = blockIdx.x, j = threadIdx.x;
+  TCoef& S = src[b];
+  const TrajG& T = traj[b];
+  if (j < 7) {
+    S.W[j] = 0.f;
+    S.slot[j] = j;
+  } else if (j == 7) {
+    S.m_hi = S.m_lo = 0.f;
+    S.nW = 0;
+    S.base = T.rot_y;
+    S.gout = slot_k1(T.rot_g);
+    S.active = (T.status == 0 && T.need_k1);
+    S.store_y7 = 0;
+    S.rec = 0;
+    S.c1 = T.c1;
+    if (S.active) flags[0] = 1;
   }
-  for (int t = threadIdx.x; t < 7 * B * 16; t += blockDim.x) {
-    const int j = t & 15, b = (t >> 4) % B, sidx = (t >> 4) / B;  // sidx 0: y; 1..6: stage s = sidx + 1
-    TCoef& S = src[sidx * bp + b];
-    const TrajG& T = traj[b];
-    const double h = T.h;
-    const bool act = (T.status == 0 && T.eval_i >= T.eval_end && T.t < T.t1);
-    if (sidx == 0) {
-      if (j < 7) S.W[j] = 0.f;
-      else if (j == 14) { S.m_hi = 0.f; S.m_lo = 0.f; }
-      else if (j == 15) {
-        S.nW = 0;
-        for (int q = 0; q < 7; ++q) S.slot[q] = q;
-        S.base = T.rot_y;
-        S.gout = slot_k1(T.rot_g);
-        S.active = (T.status == 0 && T.need_k1);
-        S.store_y7 = 0;
-        S.rec = 0;
-        S.c1 = T.c1;
-      }
-      continue;
-    }
-    const int s = sidx + 1;
-    if (j < 7) {
-      S.W[j] = (j < s - 1) ? (float)(h * A_TAB[s - 1][j]) : 0.f;
-    } else if (j < 14) {
-      if (s == 7) S.E[j - 7] = (float)(h * E_TAB[j - 7]);
-    } else if (j == 14) {
-      double mh = C_TAB[s - 1] * h;
-      float hi = (float)mh;
-      S.m_hi = hi;
-      S.m_lo = (float)(mh - (double)hi);
-    } else {
-      S.nW = s - 1;
-      S.slot[0] = slot_k1(T.rot_g);
-      for (int q = 1; q < 6; ++q) S.slot[q] = q;
-      S.slot[6] = slot_k7(T.rot_g);
-      S.base = T.rot_y;
-      S.gout = (s < 7) ? s - 1 : slot_k7(T.rot_g);
-      S.store_y7 = (s == 7);
-      S.rec = 0;
-      S.active = act;
-      S.c1 = T.c1;
-    }
+}
+// the six stages of trajectory b's next attempt, by 16 threads per stage; flags[1]: some
+// trajectory steps in it
+__device__ __forceinline__ void fill_attempt(const TrajG& T, TCoef* src, int bp, int b, int t, int* flags) {
+  const bool act = (T.status == 0 && T.eval_i >= T.eval_end && T.t < T.t1);
+  if (t == 0 && act) flags[1] = 1;
+  if (t >= 6 * 16) return;
+  const int j = t & 15, s = 2 + (t >> 4);
+  TCoef& S = src[(s - 1) * bp + b];
+  const double h = T.h;
+  if (j < 7) {
+    S.W[j] = (j < s - 1) ? (float)(h * A_TAB[s - 1][j]) : 0.f;
+  } else if (j < 14) {
+    if (s == 7) S.E[j - 7] = (float)(h * E_TAB[j - 7]);
+  } else if (j == 14) {
+    double mh = C_TAB[s - 1] * h;
+    float hi = (float)mh;
+    S.m_hi = hi;
+    S.m_lo = (float)(mh - (double)hi);
+  } else {
+    S.nW = s - 1;
+    S.slot[0] = slot_k1(T.rot_g);
+    for (int q = 1; q < 6; ++q) S.slot[q] = q;
+    S.slot[6] = slot_k7(T.rot_g);
+    S.base = T.rot_y;
+    S.gout = (s < 7) ? s - 1 : slot_k7(T.rot_g);
+    S.store_y7 = (s == 7);
+    S.rec = 0;
+    S.active = act;
+    S.c1 = T.c1;
   }
-  (void)fixed;
 }
 
 // source for the end-of-run record (interpolation with k1 replaced by k7, as after the
@@ -172,7 +168,7 @@ __global__ void k_t_coef_final(TrajG* traj, TCoef* src, int B, const float* t_ev
 
 // ---------------------------------------------------------------- stage (elementwise)
 // theta = phase[base] + omega*(m_hi+m_lo) + sum_j W_j g_j for (trajectory b, oscillator i);
-// writes the BF16 hi/lo operand columns (cos, sin) and the FP32 (cos, sin) for the epilogue
+// writes the F16 hi/lo operand columns (cos, sin) and the FP32 (cos, sin) for the epilogue
 __global__ void k_t_stage(TView v, const TCoef* src) {
   const int b = blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -189,9 +185,9 @@ __global__ void k_t_stage(TView v, const TCoef* src) {
   float sn, cs;
   sincos_pair(s2.hi, lo, &sn, &cs);
   v.x32[(size_t)b * v.np + i] = make_float2(cs, sn);
-  const __nv_bfloat16 ch = __float2bfloat16_rn(cs), sh = __float2bfloat16_rn(sn);
-  const __nv_bfloat16 cl = __float2bfloat16_rn(cs - __bfloat162float(ch));
-  const __nv_bfloat16 sl = __float2bfloat16_rn(sn - __bfloat162float(sh));
+  const __half ch = __float2half_rn(cs), sh = __float2half_rn(sn);
+  const __half cl = __float2half_rn(cs - __half2float(ch));
+  const __half sl = __float2half_rn(sn - __half2float(sh));
   v.X[xrow(0, b, v.bp) * v.np + i] = ch;
   v.X[xrow(1, b, v.bp) * v.np + i] = sh;
   v.X[xrow(2, b, v.bp) * v.np + i] = cl;
@@ -217,12 +213,13 @@ __global__ void k_t_stage(TView v, const TCoef* src) {
 // accumulator columns of work unit sp: [hi cos | hi sin | lo cos | lo sin] of trajectories
 // sp*BP .. sp*BP + BP - 1, BP columns each
 template <int BP> struct KuraEpi {
+  static constexpr bool F16 = true;
   TView v;
   const TCoef* src;
-  float invn;
   int has_lo;
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int i = m0 + row;
+    const float rinv = v.rinv[i];
 #pragma unroll 1
     for (int b0 = 0; b0 < BP; b0 += 16) {
       float hc[16], hs[16], lc[16], ls[16];
@@ -243,8 +240,8 @@ template <int BP> struct KuraEpi {
           Fc += v.Flo[((size_t)0 * v.bp + b) * v.np + i];
           Fs += v.Flo[((size_t)1 * v.bp + b) * v.np + i];
         }
-        Fc *= invn;
-        Fs *= invn;
+        Fc *= rinv;
+        Fs *= rinv;
         const float2 x = v.x32[(size_t)b * v.np + i];
         const float gv = s.c1 * (x.y * Fc - x.x * Fs);
         if (s.gout >= 0) v.g[((size_t)s.gout * v.bp + b) * v.np + i] = gv;
@@ -257,8 +254,39 @@ template <int BP> struct KuraEpi {
     }
   }
 };
+// the same for the split GEMM: the couplings (times N) of rows i..i+3 of trajectory b
+struct SplitEpi {
+  static constexpr bool F16 = true;
+  TView v;
+  const TCoef* src;
+  __device__ bool wants(int b) const { return b < v.B && src[b].active; }
+  __device__ void rows4(int i, int b, const float4& c4, const float4& s4) const {
+    if (i >= v.n) return;
+    const TCoef& s = src[b];
+    const size_t o = (size_t)b * v.np + i;
+    // np is a multiple of 4: the last group's loads and stores past n stay in the padding
+    const float4 x01 = *reinterpret_cast<const float4*>(v.x32 + o), x23 = *reinterpret_cast<const float4*>(v.x32 + o + 2);
+    const float4 ri = *reinterpret_cast<const float4*>(v.rinv + i);
+    const float Fc[4] = {c4.x * ri.x, c4.y * ri.y, c4.z * ri.z, c4.w * ri.w};
+    const float Fs[4] = {s4.x * ri.x, s4.y * ri.y, s4.z * ri.z, s4.w * ri.w};
+    const float gv[4] = {s.c1 * (x01.y * Fc[0] - x01.x * Fs[0]), s.c1 * (x01.w * Fc[1] - x01.z * Fs[1]),
+                         s.c1 * (x23.y * Fc[2] - x23.x * Fs[2]), s.c1 * (x23.w * Fc[3] - x23.z * Fs[3])};
+    if (s.gout >= 0)
+      *reinterpret_cast<float4*>(v.g + ((size_t)s.gout * v.bp + b) * v.np + i) = make_float4(gv[0], gv[1], gv[2], gv[3]);
+    if (v.mode != 0 && s.rec) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (i + q >= v.n) break;
+        v.fin_coup[(o + q) * 2] = Fc[q];
+        v.fin_coup[(o + q) * 2 + 1] = Fs[q];
+        if (v.mode == 2) v.fin_theta[o + q] = v.omega[i + q] + gv[q];
+      }
+    }
+  }
+};
 // the A_lo pass: columns [hi cos | hi sin]; stores the partial couplings
 template <int BP> struct LoEpi {
+  static constexpr bool F16 = true;
   TView v;
   const TCoef* src;
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
@@ -295,13 +323,49 @@ __device__ __forceinline__ float block_sum(float v, float* sh) {
   return t;  // valid on thread 0
 }
 
-// sum of squared scaled errors of stage 7 (dp45.cu:79-84) -> part[b][blk]
-__global__ void k_t_error(TView v, const TCoef* src7, double atol, double rtol, float* part, int nblk) {
+// whether this block is the last of the gridDim.x blocks of trajectory b to get here; the counter
+// is left at zero for the next kernel
+__device__ __forceinline__ bool last_of(unsigned* cnt, int b) {
+  __shared__ int last;
+  if (threadIdx.x == 0) {
+    __threadfence();  // this block's partial sums before its arrival
+    last = atomicAdd(cnt + b, 1u) == gridDim.x - 1;
+    if (last) {
+      cnt[b] = 0;
+      __threadfence();
+    }
+  }
+  __syncthreads();
+  return last;
+}
+// the nblk values p[q * stride], added in the order of q; every thread of the block calls it
+__device__ __forceinline__ float sum_in_order(const float* p, int nblk, int stride, float* buf) {
+  __syncthreads();
+  for (int q = threadIdx.x; q < nblk; q += blockDim.x) buf[q] = __ldcg(p + (size_t)q * stride);
+  __syncthreads();
+  float s = 0.f;
+  if (threadIdx.x == 0) {
+#pragma unroll 8
+    for (int q = 0; q < nblk; ++q) s += buf[q];
+  }
+  return s;  // valid on thread 0
+}
+constexpr int T_MAXBLK = 1024;  // blocks per trajectory of the two kernels below
+
+// The error norm of stage 7 (dp45.cu:79-84) and the controller (dp45.cu:109-139) of each
+// trajectory, which the last block of the trajectory runs: a launch of its own for the controller
+// and one thread per trajectory over its partial sums cost 6 us of latency per attempt.  flags[1]
+// is cleared for the output kernel, which sets it anew.
+__global__ void k_t_error(TView v, const TCoef* src7, double atol, double rtol, float* part, int nblk, TrajG* traj,
+                          int fixed, const float* t_eval, int n_eval, unsigned* cnt, int* flags) {
   __shared__ float sh[32];
+  __shared__ float buf[T_MAXBLK];
   const int b = blockIdx.y;
   const TCoef& s = src7[b];
+  if (b == 0 && blockIdx.x == 0 && threadIdx.x == 0) flags[1] = 0;
+  if (!s.active) return;
   float acc = 0.f;
-  if (s.active) {
+  if (!fixed) {
     const size_t yb = ((size_t)s.base * v.bp + b) * v.np, y7b = ((size_t)(s.base ^ 1) * v.bp + b) * v.np;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < v.n; i += gridDim.x * blockDim.x) {
       float e = 0.f;
@@ -316,152 +380,138 @@ __global__ void k_t_error(TView v, const TCoef* src7, double atol, double rtol, 
       const float ye = e / tol;
       acc = __fmaf_rn(ye, ye, acc);
     }
+    const float t = block_sum(acc, sh);
+    if (threadIdx.x == 0) part[(size_t)b * nblk + blockIdx.x] = t;
+    if (!last_of(cnt, b)) return;
+  } else if (blockIdx.x > 0) {
+    return;
   }
-  const float t = block_sum(acc, sh);
-  if (threadIdx.x == 0) part[(size_t)b * nblk + blockIdx.x] = t;
-}
-
-// controller of every trajectory (dp45.cu:109-139); writes the completion flag
-__global__ void k_t_decide(TrajG* traj, const TCoef* src7, const float* part, int nblk, int B, int n, int fixed,
-                           const float* t_eval, int n_eval, int* done) {
-  const int b = threadIdx.x;
-  __shared__ int any;
-  if (b == 0) any = 0;
-  __syncthreads();
-  if (b < B) {
-    TrajG& T = traj[b];
-    if (src7[b].active && T.status == 0) {
-      const double h = T.h;
-      bool accept = true;
-      double factor = 1.0;
-      if (!fixed) {
-        float ss = 0.f;
-        for (int q = 0; q < nblk; ++q) ss += part[(size_t)b * nblk + q];
-        const double norm = sqrt((double)ss) / sqrt((double)n);
-        if (isnan(norm)) {
-          T.status = KURA_ERR_NONFINITE;
-        } else {
-          factor = (double)(0.9f * exp2f(-0.2f * log2f((float)norm)));
-          accept = norm < 1.0;
-        }
-      }
-      if (T.status == 0) {
-        if (accept) {
-          T.t_last = T.t;
-          T.t = T.t + h;
-          T.rot_y ^= 1;
-          T.rot_g ^= 1;
-          T.accepted++;
-          if (!fixed) T.h = h * fmin(factor, 10.0);
-          int e = T.eval_i;
-          while (e < n_eval && T.t >= (double)t_eval[e]) e++;
-          T.eval_end = e;
-        } else {
-          T.rejected++;
-          if (factor < 1.0) T.h = h * fmax(factor, 0.2);
-          if (!(T.h >= 1e-14 * fmax(1.0, fabs(T.t)))) T.status = KURA_ERR_STEP_UNDERFLOW;
-        }
-      }
+  const float ss = fixed ? 0.f : sum_in_order(part + (size_t)b * nblk, nblk, 1, buf);
+  if (threadIdx.x != 0) return;
+  TrajG& T = traj[b];
+  const double h = T.h;
+  bool accept = true;
+  double factor = 1.0;
+  if (!fixed) {
+    const double norm = sqrt((double)ss) / sqrt((double)v.n);
+    if (isnan(norm)) {
+      T.status = KURA_ERR_NONFINITE;
+      return;
     }
-    if (T.status == 0 && !(T.t < T.t1) && T.eval_i >= T.eval_end) T.status = 1;
-    if (T.status == 0 || T.eval_i < T.eval_end) atomicOr(&any, 1);
+    factor = (double)(0.9f * exp2f(-0.2f * log2f((float)norm)));
+    accept = norm < 1.0;
   }
-  __syncthreads();
-  if (b == 0) *done = any ? 0 : 1;
+  if (accept) {
+    T.t_last = T.t;
+    T.t = T.t + h;
+    T.rot_y ^= 1;
+    T.rot_g ^= 1;
+    T.accepted++;
+    if (!fixed) T.h = h * fmin(factor, 10.0);
+    int e = T.eval_i;
+    while (e < n_eval && T.t >= (double)t_eval[e]) e++;
+    T.eval_end = e;
+  } else {
+    T.rejected++;
+    if (factor < 1.0) T.h = h * fmax(factor, 0.2);
+    if (!(T.h >= 1e-14 * fmax(1.0, fabs(T.t)))) T.status = KURA_ERR_STEP_UNDERFLOW;
+  }
 }
 
-// order parameter at the pending output times of each trajectory: partial sums of
-// (cos, sin) of the dense output (dp45.cu:70-76, kuramoto.cu:212-220)
-__global__ void k_t_out_partial(TView v, const TrajG* traj, const float* t_eval, float* part, int nblk) {
+// The order parameter at the pending output times of each trajectory (dense output, dp45.cu:70-76,
+// kuramoto.cu:212-220); the last block of the trajectory writes the records, ends the trajectory
+// when it has reached t1 and fills the coefficients of its next attempt (on their own, over all
+// trajectories in one block, these took 4 and 15 us per attempt).  first: the call after the
+// first slopes.
+__global__ void k_t_output(TView v, TrajG* traj, const float* t_eval, float* part, int nblk, float* out_r, int* out_idx,
+                           int ring, TCoef* src, unsigned* cnt, int* flags, int first) {
   __shared__ float sh[32];
+  __shared__ float buf[T_MAXBLK];
   const int b = blockIdx.y;
-  const TrajG& T = traj[b];
+  TrajG& T = traj[b];
   const int ncross = min(T.eval_end - T.eval_i, T_MAXC);
   const bool initial = T.need_init != 0;
-  if (ncross <= 0 && !initial) return;
-  const int nrec = initial ? 1 : ncross;
-  const size_t bl = initial ? ((size_t)T.rot_y * v.bp + b) * v.np : ((size_t)(T.rot_y ^ 1) * v.bp + b) * v.np;
-  // after the accept, k1 of the step sits in the k7 slot and vice versa
-  const int k1s = slot_k7(T.rot_g), k7s = slot_k1(T.rot_g);
-  __shared__ float sw[9];  // the record's weights: W[0..6], then the time offset hi and lo
-  for (int c = 0; c < nrec; ++c) {
-    // the weights in double, once per block (FP64 is a small fraction of this GPU's FP32 rate:
-    // computed by every thread they cost more than the record's memory traffic)
-    if (threadIdx.x == 0) {
-      for (int j = 0; j < 9; ++j) sw[j] = 0.f;
-      if (!initial) {
-        const double hs = T.t - T.t_last, dl = (double)t_eval[T.eval_i + c] - T.t_last, x = dl / hs;
-        for (int j = 0; j < 7; ++j) {
-          const double cc = ((P_TAB[j][3] * x + P_TAB[j][2]) * x + P_TAB[j][1]) * x * x + P_TAB[j][0] * x;
-          sw[j] = (float)(hs * cc);
+  const int nrec = initial ? 1 : max(ncross, 0);
+  if (nrec == 0 && blockIdx.x > 0) return;
+  if (nrec > 0) {
+    const size_t bl = initial ? ((size_t)T.rot_y * v.bp + b) * v.np : ((size_t)(T.rot_y ^ 1) * v.bp + b) * v.np;
+    // after the accept, k1 of the step sits in the k7 slot and vice versa
+    const int k1s = slot_k7(T.rot_g), k7s = slot_k1(T.rot_g);
+    __shared__ float sw[9];  // the record's weights: W[0..6], then the time offset hi and lo
+    for (int c = 0; c < nrec; ++c) {
+      // the weights in double, once per block (FP64 is a small fraction of this GPU's FP32 rate:
+      // computed by every thread they cost more than the record's memory traffic)
+      if (threadIdx.x == 0) {
+        for (int j = 0; j < 9; ++j) sw[j] = 0.f;
+        if (!initial) {
+          const double hs = T.t - T.t_last, dl = (double)t_eval[T.eval_i + c] - T.t_last, x = dl / hs;
+          for (int j = 0; j < 7; ++j) {
+            const double cc = ((P_TAB[j][3] * x + P_TAB[j][2]) * x + P_TAB[j][1]) * x * x + P_TAB[j][0] * x;
+            sw[j] = (float)(hs * cc);
+          }
+          const float mh0 = (float)dl;
+          sw[7] = mh0;
+          sw[8] = (float)(dl - (double)mh0);
         }
-        const float mh0 = (float)dl;
-        sw[7] = mh0;
-        sw[8] = (float)(dl - (double)mh0);
       }
-    }
-    __syncthreads();
-    float W[7];
+      __syncthreads();
+      float W[7];
 #pragma unroll
-    for (int j = 0; j < 7; ++j) W[j] = sw[j];
-    const float mh = sw[7], ml = sw[8];
-    float ax = 0.f, ay = 0.f;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < v.n; i += gridDim.x * blockDim.x) {
-      float gsum = 0.f;
-      if (!initial) {
-        gsum = __fmaf_rn(W[0], v.g[((size_t)k1s * v.bp + b) * v.np + i], gsum);
-        for (int j = 1; j < 6; ++j) gsum = __fmaf_rn(W[j], v.g[((size_t)j * v.bp + b) * v.np + i], gsum);
-        gsum = __fmaf_rn(W[6], v.g[((size_t)k7s * v.bp + b) * v.np + i], gsum);
+      for (int j = 0; j < 7; ++j) W[j] = sw[j];
+      const float mh = sw[7], ml = sw[8];
+      float ax = 0.f, ay = 0.f;
+      for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < v.n; i += gridDim.x * blockDim.x) {
+        float gsum = 0.f;
+        if (!initial) {
+          gsum = __fmaf_rn(W[0], v.g[((size_t)k1s * v.bp + b) * v.np + i], gsum);
+          for (int j = 1; j < 6; ++j) gsum = __fmaf_rn(W[j], v.g[((size_t)j * v.bp + b) * v.np + i], gsum);
+          gsum = __fmaf_rn(W[6], v.g[((size_t)k7s * v.bp + b) * v.np + i], gsum);
+        }
+        const float om = v.omega[i];
+        const f2 pr = two_prod(om, mh);
+        const f2 s1 = two_sum(v.ph_hi[bl + i], pr.hi);
+        const f2 s2 = two_sum(s1.hi, gsum);
+        const float lo = v.ph_lo[bl + i] + ((s1.lo + s2.lo) + __fmaf_rn(om, ml, pr.lo));
+        float sn, cs;
+        sincos_pair(s2.hi, lo, &sn, &cs);
+        ax += cs;
+        ay += sn;
       }
-      const float om = v.omega[i];
-      const f2 pr = two_prod(om, mh);
-      const f2 s1 = two_sum(v.ph_hi[bl + i], pr.hi);
-      const f2 s2 = two_sum(s1.hi, gsum);
-      const float lo = v.ph_lo[bl + i] + ((s1.lo + s2.lo) + __fmaf_rn(om, ml, pr.lo));
-      float sn, cs;
-      sincos_pair(s2.hi, lo, &sn, &cs);
-      ax += cs;
-      ay += sn;
+      const float tx = block_sum(ax, sh);
+      const float ty = block_sum(ay, sh);
+      if (threadIdx.x == 0) {
+        part[(((size_t)b * T_MAXC + c) * nblk + blockIdx.x) * 2] = tx;
+        part[(((size_t)b * T_MAXC + c) * nblk + blockIdx.x) * 2 + 1] = ty;
+      }
     }
-    const float tx = block_sum(ax, sh);
-    const float ty = block_sum(ay, sh);
+    if (!last_of(cnt, b)) return;
+    for (int c = 0; c < nrec; ++c) {
+      const float* pc = part + ((size_t)b * T_MAXC + c) * nblk * 2;
+      const float X = sum_in_order(pc, nblk, 2, buf), Y = sum_in_order(pc + 1, nblk, 2, buf);
+      if (threadIdx.x == 0 && T.out_count < ring) {
+        const float xn = X / (float)v.n, yn = Y / (float)v.n;
+        out_r[(size_t)b * ring + T.out_count] = sqrtf(xn * xn + yn * yn);
+        out_idx[(size_t)b * ring + T.out_count] = initial ? -1 : T.eval_i;
+        T.out_count++;
+        if (!initial) T.eval_i++;
+      }
+    }
     if (threadIdx.x == 0) {
-      part[(((size_t)b * T_MAXC + c) * nblk + blockIdx.x) * 2] = tx;
-      part[(((size_t)b * T_MAXC + c) * nblk + blockIdx.x) * 2 + 1] = ty;
+      if (initial) T.need_init = 0;
+      else if (T.eval_i < T.eval_end) T.status = KURA_ERR_UNSUPPORTED;  // more than T_MAXC crossings in a step
     }
   }
-}
-__global__ void k_t_out_final(TrajG* traj, const float* part, int nblk, int B, int n, float* out_r, int* out_idx,
-                              int ring) {
-  const int b = threadIdx.x;
-  if (b >= B) return;
-  TrajG& T = traj[b];
-  const bool initial = T.need_init != 0;
-  int nrec = initial ? 1 : min(T.eval_end - T.eval_i, T_MAXC);
-  if (nrec <= 0) return;
-  if (!initial && T.eval_end - T.eval_i > T_MAXC) T.status = KURA_ERR_UNSUPPORTED;
-  for (int c = 0; c < nrec && T.out_count < ring; ++c) {
-    float X = 0.f, Y = 0.f;
-    for (int q = 0; q < nblk; ++q) {
-      X += part[(((size_t)b * T_MAXC + c) * nblk + q) * 2];
-      Y += part[(((size_t)b * T_MAXC + c) * nblk + q) * 2 + 1];
-    }
-    const float xn = X / (float)n, yn = Y / (float)n;
-    out_r[(size_t)b * ring + T.out_count] = sqrtf(xn * xn + yn * yn);
-    out_idx[(size_t)b * ring + T.out_count] = initial ? -1 : T.eval_i;
-    T.out_count++;
-    if (!initial) T.eval_i++;
+  if (threadIdx.x == 0) {
+    if (first) T.need_k1 = 0;
+    if (T.status == 0 && !(T.t < T.t1) && T.eval_i >= T.eval_end) T.status = 1;
   }
-  if (initial) T.need_init = 0;
-}
-__global__ void k_t_clear_k1(TrajG* traj, int B) {
-  const int b = threadIdx.x;
-  if (b < B) traj[b].need_k1 = 0;
+  __syncthreads();
+  fill_attempt(T, src, v.bp, b, threadIdx.x, flags);
 }
 
-// N*A for the volcano rule, exact in BF16 (integers in [-K, K])
-__global__ void k_t_volcano_bf16(const uint32_t* __restrict__ bits, int n, int k, int words, int np,
-                                 __nv_bfloat16* __restrict__ A, __nv_bfloat16* __restrict__ Alo) {
+// N*A for the volcano rule, exact in F16 (integers in [-K, K], K <= 2048; hi + lo above)
+__global__ void k_t_volcano_f16(const uint32_t* __restrict__ bits, int n, int k, int words, int np,
+                                __half* __restrict__ A, __half* __restrict__ Alo) {
   for (int i = blockIdx.y; i < np; i += gridDim.y)
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < np; j += gridDim.x * blockDim.x) {
       int kk = 0;
@@ -474,28 +524,53 @@ __global__ void k_t_volcano_bf16(const uint32_t* __restrict__ bits, int n, int k
           kk += __popc(even) - __popc(odd) - 2 * __popc(dis & even) + 2 * __popc(dis & odd);
         }
       }
-      const __nv_bfloat16 hi = __float2bfloat16_rn((float)kk);
+      const __half hi = __float2half_rn((float)kk);
       A[(size_t)i * np + j] = hi;
-      if (Alo) Alo[(size_t)i * np + j] = __float2bfloat16_rn((float)kk - __bfloat162float(hi));
+      if (Alo) Alo[(size_t)i * np + j] = __float2half_rn((float)kk - __half2float(hi));
     }
 }
-// general adjacency: N*A = hi + lo in BF16
-__global__ void k_t_split(const float* __restrict__ adj, int n, int np, float scale, __nv_bfloat16* hi,
-                          __nv_bfloat16* lo) {
-  for (int i = blockIdx.y; i < np; i += gridDim.y)
-    for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < np; j += gridDim.x * blockDim.x) {
-      const float a = (i < n && j < n) ? adj[(size_t)i * n + j] * scale : 0.f;
-      const __nv_bfloat16 h = __float2bfloat16_rn(a);
+__global__ void k_t_fill(float* p, int n, float v) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) p[i] = v;
+}
+// general adjacency, one block per row: 2^p N A = hi + lo in F16, with 2^p so that the row's largest
+// entry lies in [2^13, 2^14) (1 for a row of zeros or one that holds an infinity)
+__global__ void k_t_split(const float* __restrict__ adj, int n, int np, float scale, __half* hi, __half* lo,
+                          float* rinv) {
+  __shared__ float sh[32];
+  __shared__ float smax;
+  for (int i = blockIdx.x; i < np; i += gridDim.x) {
+    float m = 0.f;
+    if (i < n)
+      for (int j = threadIdx.x; j < n; j += blockDim.x) m = fmaxf(m, fabsf(adj[(size_t)i * n + j] * scale));
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, sh[w]);
+      int e = 14;  // frexp's exponent: m in [2^(e-1), 2^e)
+      if (m > 0.f && m <= 3.4028235e38f) frexpf(m, &e);
+      e = max(-110, min(e, 120));  // 2^(14-e) and its reciprocal stay normal floats
+      smax = ldexpf(1.f, 14 - e);
+      rinv[i] = (1.f / scale) * ldexpf(1.f, e - 14);
+    }
+    __syncthreads();
+    const float p = smax;
+    for (int j = threadIdx.x; j < np; j += blockDim.x) {
+      const float a = (i < n && j < n) ? adj[(size_t)i * n + j] * scale * p : 0.f;
+      const __half h = __float2half_rn(a);
       hi[(size_t)i * np + j] = h;
-      lo[(size_t)i * np + j] = __float2bfloat16_rn(a - __bfloat162float(h));
+      lo[(size_t)i * np + j] = __float2half_rn(a - __half2float(h));
     }
+  }
 }
-__global__ void k_t_adj_out(const __nv_bfloat16* hi, const __nv_bfloat16* lo, int n, int np, float invn, float* adj) {
+__global__ void k_t_adj_out(const __half* hi, const __half* lo, int n, int np, const float* rinv, float* adj) {
   for (int i = blockIdx.y; i < n; i += gridDim.y)
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-      float a = __bfloat162float(hi[(size_t)i * np + j]);
-      if (lo) a += __bfloat162float(lo[(size_t)i * np + j]);
-      adj[(size_t)i * n + j] = __fmul_rn(a, invn);
+      float a = __half2float(hi[(size_t)i * np + j]);
+      if (lo) a += __half2float(lo[(size_t)i * np + j]);
+      adj[(size_t)i * n + j] = __fmul_rn(a, rinv[i]);
     }
 }
 
@@ -511,11 +586,12 @@ struct TensorEngine::Impl {
   float* ph_lo = nullptr;
   long long* ph_w = nullptr;
   float* g = nullptr;
-  __nv_bfloat16* X = nullptr;
+  __half* X = nullptr;
   float2* x32 = nullptr;
-  __nv_bfloat16* Ahi = nullptr;
-  __nv_bfloat16* Alo = nullptr;
+  __half* Ahi = nullptr;
+  __half* Alo = nullptr;
   float* Flo = nullptr;
+  float* rinv = nullptr;  // [np] scale of each row's couplings
   float* fin_theta = nullptr;
   float* fin_coup = nullptr;
   TrajG* traj = nullptr;
@@ -524,10 +600,10 @@ struct TensorEngine::Impl {
   float* t_eval = nullptr;
   float* out_r = nullptr;
   int* out_idx = nullptr;
-  int* done = nullptr;
   int* err = nullptr;
-  int* any_active = nullptr;  // written by the coefficient kernels; the GEMMs skip when 0
-  int* h_done = nullptr;      // pinned
+  int* flags = nullptr;     // [0]: a trajectory needs its first slope, [1]: one steps in the next attempt; the GEMMs skip on 0
+  unsigned* cnt = nullptr;  // [bp] arrivals of a trajectory's blocks
+  int* h_run = nullptr;     // pinned: flags[1] and the error code
   int ring = 0, n_eval = 0, nblk = 1;
   CUtensorMap tmA, tmAlo, tmX, tmXhi;
   bool has_lo = false, adj_set = false;
@@ -562,12 +638,11 @@ template <typename T> static cudaError_t zalloc(T** p, size_t count) {
 
 TensorEngine::TensorEngine() : d(new Impl) {}
 TensorEngine::~TensorEngine() {
-  void* ptrs[] = {d->omega, d->ph_hi, d->ph_lo, d->ph_w, d->g, d->X, d->x32, d->Ahi, d->Alo, d->Flo, d->fin_theta,
-                  d->fin_coup, d->traj, d->src, d->part, d->t_eval, d->out_r, d->out_idx, d->done, d->err,
-                  d->any_active};
+  void* ptrs[] = {d->omega, d->ph_hi, d->ph_lo, d->ph_w, d->g, d->X, d->x32, d->Ahi, d->Alo, d->Flo, d->rinv, d->fin_theta,
+                  d->fin_coup, d->traj, d->src, d->part, d->t_eval, d->out_r, d->out_idx, d->err, d->flags, d->cnt};
   for (void* p : ptrs)
     if (p) cudaFree(p);
-  if (d->h_done) cudaFreeHost(d->h_done);
+  if (d->h_run) cudaFreeHost(d->h_run);
   if (d->graph) cudaGraphExecDestroy(d->graph);
   if (d->ev0) cudaEventDestroy(d->ev0);
   if (d->ev1) cudaEventDestroy(d->ev1);
@@ -588,7 +663,7 @@ int TensorEngine::init(int64_t n, int k, int batch, int seed, double atol, doubl
   I.bp = 16;
   while (I.bp < batch) I.bp *= 2;
   const size_t np = I.np, bp = I.bp;
-  I.nblk = std::min(1024, (I.n + T_RBLK - 1) / T_RBLK);
+  I.nblk = std::min(T_MAXBLK, (I.n + T_RBLK - 1) / T_RBLK);
   TCU(zalloc(&I.omega, np));
   TCU(zalloc(&I.ph_hi, 2 * bp * np));
   TCU(zalloc(&I.ph_lo, 2 * bp * np));
@@ -597,15 +672,16 @@ int TensorEngine::init(int64_t n, int k, int batch, int seed, double atol, doubl
   TCU(zalloc(&I.X, 4 * bp * np));
   TCU(zalloc(&I.x32, bp * np));
   TCU(zalloc(&I.Ahi, np * np));
+  TCU(zalloc(&I.rinv, np));
   TCU(zalloc(&I.fin_theta, bp * np));
   TCU(zalloc(&I.fin_coup, 2 * bp * np));
   TCU(zalloc(&I.traj, bp));
   TCU(zalloc(&I.src, 8 * bp));
   TCU(zalloc(&I.part, (size_t)bp * T_MAXC * I.nblk * 2));
-  TCU(zalloc(&I.done, 4));
-  TCU(zalloc(&I.any_active, 16));
+  TCU(zalloc(&I.flags, 2));
+  TCU(zalloc(&I.cnt, bp));
   TCU(zalloc(&I.err, 4));
-  TCU(cudaHostAlloc((void**)&I.h_done, sizeof(int), cudaHostAllocDefault));
+  TCU(cudaHostAlloc((void**)&I.h_run, 2 * sizeof(int), cudaHostAllocDefault));
   TCU(cudaEventCreate(&I.ev0));
   TCU(cudaEventCreate(&I.ev1));
   const char* tg = getenv("KURA_TIME_COUPLING");
@@ -614,9 +690,9 @@ int TensorEngine::init(int64_t n, int k, int batch, int seed, double atol, doubl
     for (cudaEvent_t& e : I.gev) TCU(cudaEventCreate(&e));
   // X is [4 bp][np]: a work unit's column block is 4 * x_bph(bp) rows (its hi + lo columns),
   // of which the A_lo pass reads the first half
-  if (make_tmap_bf16(&I.tmA, I.Ahi, np, np, TG_BM, TE_BK) ||
-      make_tmap_bf16(&I.tmX, I.X, np, 4 * bp, 4 * x_bph(I.bp), TE_BK) ||
-      make_tmap_bf16(&I.tmXhi, I.X, np, 4 * bp, 2 * x_bph(I.bp), TE_BK)) {
+  if (make_tmap_16(&I.tmA, true, I.Ahi, np, np, TG_BM, TE_BK) ||
+      make_tmap_16(&I.tmX, true, I.X, np, 4 * bp, 4 * x_bph(I.bp), TE_BK) ||
+      make_tmap_16(&I.tmXhi, true, I.X, np, 4 * bp, 2 * x_bph(I.bp), TE_BK)) {
     g_terr = "cuTensorMapEncodeTiled failed";
     return KURA_ERR_CUDA;
   }
@@ -626,7 +702,7 @@ int TensorEngine::init(int64_t n, int k, int batch, int seed, double atol, doubl
 size_t TensorEngine::memory_required(int64_t n, int batch) {
   size_t np = ((size_t)n + 255) / 256 * 256, bp = 16;
   while ((int)bp < batch) bp *= 2;
-  return np * np * 2 + np * bp * (2 * 16 + 7 * 4 + 4 * 2 + 8 + 4 + 8) + np * 4;
+  return np * np * 2 + np * bp * (2 * 16 + 7 * 4 + 4 * 2 + 8 + 4 + 8) + np * 8;
 }
 
 int TensorEngine::set_frequencies(const float* omega) {
@@ -643,16 +719,17 @@ int TensorEngine::generate_adjacency() {
     TCU(cudaMalloc((void**)&bits, sizeof(uint32_t) * (size_t)words * I.n));
     TCU(launch_volcano_words(I.seed, I.n, I.K, words, bits, I.st));
   }
-  // N*A_ij is an integer in [-K, K]: exact in BF16 for K <= 256, else exact as hi + lo
-  const bool need_lo = I.K > 256;
+  // N*A_ij is an integer in [-K, K]: exact in F16 for K <= 2048, else as hi + lo
+  const bool need_lo = I.K > 2048;
   if (need_lo && !I.Alo) TCU(zalloc(&I.Alo, (size_t)I.np * I.np));
   if (need_lo && !I.Flo) TCU(zalloc(&I.Flo, (size_t)2 * I.bp * I.np));
   dim3 grid((unsigned)std::min((I.np + 255) / 256, 64), (unsigned)std::min(I.np, 65535));
-  k_t_volcano_bf16<<<grid, 256, 0, I.st>>>(bits, I.n, I.K, words, I.np, I.Ahi, need_lo ? I.Alo : nullptr);
+  k_t_volcano_f16<<<grid, 256, 0, I.st>>>(bits, I.n, I.K, words, I.np, I.Ahi, need_lo ? I.Alo : nullptr);
+  k_t_fill<<<(I.np + 255) / 256, 256, 0, I.st>>>(I.rinv, I.np, 1.0f / (float)I.n);
   TCU(cudaGetLastError());
   TCU(cudaStreamSynchronize(I.st));
   if (bits) cudaFree(bits);
-  if (need_lo && make_tmap_bf16(&I.tmAlo, I.Alo, I.np, I.np, TG_BM, TE_BK)) {
+  if (need_lo && make_tmap_16(&I.tmAlo, true, I.Alo, I.np, I.np, TG_BM, TE_BK)) {
     g_terr = "cuTensorMapEncodeTiled failed";
     return KURA_ERR_CUDA;
   }
@@ -668,12 +745,11 @@ int TensorEngine::set_adjacency(const float* adj_host) {
   TCU(cudaMemcpyAsync(dadj, adj_host, sizeof(float) * (size_t)I.n * I.n, cudaMemcpyHostToDevice, I.st));
   if (!I.Alo) TCU(zalloc(&I.Alo, (size_t)I.np * I.np));
   if (!I.Flo) TCU(zalloc(&I.Flo, (size_t)2 * I.bp * I.np));
-  dim3 grid((unsigned)std::min((I.np + 255) / 256, 64), (unsigned)std::min(I.np, 65535));
-  k_t_split<<<grid, 256, 0, I.st>>>(dadj, I.n, I.np, (float)I.n, I.Ahi, I.Alo);
+  k_t_split<<<(unsigned)std::min(I.np, 65535), 256, 0, I.st>>>(dadj, I.n, I.np, (float)I.n, I.Ahi, I.Alo, I.rinv);
   TCU(cudaGetLastError());
   TCU(cudaStreamSynchronize(I.st));
   cudaFree(dadj);
-  if (make_tmap_bf16(&I.tmAlo, I.Alo, I.np, I.np, TG_BM, TE_BK)) {
+  if (make_tmap_16(&I.tmAlo, true, I.Alo, I.np, I.np, TG_BM, TE_BK)) {
     g_terr = "cuTensorMapEncodeTiled failed";
     return KURA_ERR_CUDA;
   }
@@ -687,7 +763,7 @@ int TensorEngine::get_adjacency(float* adj_host) {
   float* dadj = nullptr;
   TCU(cudaMalloc((void**)&dadj, sizeof(float) * (size_t)I.n * I.n));
   dim3 grid((unsigned)std::min((I.n + 255) / 256, 64), (unsigned)std::min(I.n, 65535));
-  k_t_adj_out<<<grid, 256, 0, I.st>>>(I.Ahi, I.has_lo ? I.Alo : nullptr, I.n, I.np, 1.0f / (float)I.n, dadj);
+  k_t_adj_out<<<grid, 256, 0, I.st>>>(I.Ahi, I.has_lo ? I.Alo : nullptr, I.n, I.np, I.rinv, dadj);
   TCU(cudaGetLastError());
   TCU(cudaMemcpyAsync(adj_host, dadj, sizeof(float) * (size_t)I.n * I.n, cudaMemcpyDeviceToHost, I.st));
   TCU(cudaStreamSynchronize(I.st));
@@ -727,15 +803,42 @@ int TensorEngine::set_horizon(const std::vector<float>& t_eval, int ring, std::v
   return KURA_OK;
 }
 
+template <int NCOL, int MT>
+static cudaError_t launch_split(TensorEngine::Impl& I, const TView& v, const TCoef* src, int s, int ktiles, int nsplit,
+                                int xstride, const int* run_flag) {
+  using C = TSCfg<NCOL, MT>;
+  auto k = k_split_gemm<NCOL, MT, SplitEpi>;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+  if (e != cudaSuccess) return e;
+  const int tiles = (I.n + TG_BM - 1) / TG_BM;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = s;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)((tiles + MT - 1) / MT * nsplit * s));
+  cfg.blockDim = dim3(TS_THREADS);
+  cfg.dynamicSmemBytes = C::SMEM;
+  cfg.stream = I.st;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, I.tmA, I.has_lo ? I.tmAlo : I.tmA, I.tmX, I.tmXhi, ktiles, s, nsplit, xstride,
+                            I.has_lo ? 1 : 0, SplitEpi{v, src}, I.err, 20000000000ull, run_flag);
+}
+
 template <int NCOL>
 static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode, const int* run_flag) {
   TView v{I.n, I.np, I.bp, I.B, mode, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, I.fin_theta, I.fin_coup,
-          I.Flo};
+          I.Flo, I.rinv};
   constexpr int BP = NCOL / 4;  // trajectories per work unit
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, I.device);
   const int mtiles = I.np / (2 * TG_BM), ktiles = I.np / TE_BK;  // groups of two row tiles
   const int nsplit = I.bp / BP, xstride = 4 * BP;
+  const SplitShape sh = split_shape((I.n + TG_BM - 1) / TG_BM, nsplit, NCOL, ktiles, sms);
+  if (sh.mt == 1) return launch_split<NCOL, 1>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag);
+  if (sh.mt == 2) return launch_split<NCOL, 2>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag);
   const int grid = std::min(mtiles * nsplit, sms);
   // Units of two row tiles fill whole waves of the grid; the rest run as one-tile units, when
   // that shortens the last wave (in unit times: a one-tile unit is half of a two-tile one)
@@ -760,7 +863,7 @@ static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode
   }
   auto k = k_tensor_gemm<NCOL, KuraEpi<BP>, 2, TE_BK>;
   cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TGCfg<NCOL, 2, TE_BK>::SMEM);
-  KuraEpi<BP> ep{v, src, 1.0f / (float)I.n, I.has_lo ? 1 : 0};
+  KuraEpi<BP> ep{v, src, I.has_lo ? 1 : 0};
   k<<<grid, TG_THREADS, TGCfg<NCOL, 2, TE_BK>::SMEM, I.st>>>(I.tmA, I.tmX, mtiles, big, ktiles, nsplit, xstride, ep, I.err, limit,
                                                    run_flag);
   return cudaGetLastError();
@@ -779,7 +882,7 @@ static cudaError_t gemm(TensorEngine::Impl& I, const TCoef* src, int mode, const
 static cudaError_t coupling(TensorEngine::Impl& I, const TCoef* src, int mode, float* fin_theta, const int* run_flag,
                             int timed = -1) {
   TView v{I.n, I.np, I.bp, I.B, mode, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, fin_theta, I.fin_coup,
-          I.Flo};
+          I.Flo, I.rinv};
   dim3 grid((unsigned)((I.n + 255) / 256), (unsigned)I.B);
   k_t_stage<<<grid, 256, 0, I.st>>>(v, src);
   cudaError_t e = cudaGetLastError();
@@ -791,46 +894,39 @@ static cudaError_t coupling(TensorEngine::Impl& I, const TCoef* src, int mode, f
   return e;
 }
 
-// one attempt of every trajectory, then its outputs
+static cudaError_t output(TensorEngine::Impl& I, int first) {
+  TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo, I.rinv};
+  k_t_output<<<dim3((unsigned)I.nblk, (unsigned)I.B), T_RBLK, 0, I.st>>>(v, I.traj, I.t_eval, I.part, I.nblk, I.out_r,
+                                                                       I.out_idx, I.ring, I.src, I.cnt, I.flags, first);
+  return cudaGetLastError();
+}
+
+// one attempt of every trajectory, its outputs, and the coefficients of the next
 static cudaError_t attempt(TensorEngine::Impl& I) {
-  TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo};
-  k_t_coef<<<1, 512, 0, I.st>>>(I.traj, I.src, I.B, I.bp, I.fixed, I.any_active);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo, I.rinv};
+  cudaError_t e = cudaSuccess;
   for (int s = 2; s <= 7; ++s) {
-    e = coupling(I, I.src + (size_t)(s - 1) * I.bp, 0, nullptr, I.any_active + 1, s - 2);
+    e = coupling(I, I.src + (size_t)(s - 1) * I.bp, 0, nullptr, I.flags + 1, s - 2);
     if (e != cudaSuccess) return e;
   }
-  if (!I.fixed) {
-    k_t_error<<<dim3((unsigned)I.nblk, (unsigned)I.B), T_RBLK, 0, I.st>>>(v, I.src + 6 * (size_t)I.bp, I.atol, I.rtol,
-                                                                        I.part, I.nblk);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  }
-  k_t_decide<<<1, 128, 0, I.st>>>(I.traj, I.src + 6 * (size_t)I.bp, I.part, I.nblk, I.B, I.n, I.fixed, I.t_eval,
-                                  I.n_eval, I.done);
+  k_t_error<<<dim3((unsigned)(I.fixed ? 1 : I.nblk), (unsigned)I.B), T_RBLK, 0, I.st>>>(
+      v, I.src + 6 * (size_t)I.bp, I.atol, I.rtol, I.part, I.nblk, I.traj, I.fixed, I.t_eval, I.n_eval, I.cnt, I.flags);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  k_t_out_partial<<<dim3((unsigned)I.nblk, (unsigned)I.B), T_RBLK, 0, I.st>>>(v, I.traj, I.t_eval, I.part, I.nblk);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  k_t_out_final<<<1, 128, 0, I.st>>>(I.traj, I.part, I.nblk, I.B, I.n, I.out_r, I.out_idx, I.ring);
-  return cudaGetLastError();
+  return output(I, 0);
 }
 
 int TensorEngine::run(std::vector<TrajG>& traj, kura_stats& stats, long long max_replays) {
   Impl& I = *d;
   if (!I.adj_set) { g_terr = "adjacency not set"; return KURA_ERR_INVALID; }
   TCU(cudaMemsetAsync(I.err, 0, sizeof(int), I.st));
+  TCU(cudaMemsetAsync(I.flags, 0, 2 * sizeof(int), I.st));
+  TCU(cudaMemsetAsync(I.cnt, 0, sizeof(unsigned) * I.bp, I.st));
   TCU(cudaEventRecord(I.ev0, I.st));
-  // first slope of the run and the record at t0
-  {
-    TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo};
-    k_t_coef<<<1, 512, 0, I.st>>>(I.traj, I.src, I.B, I.bp, I.fixed, I.any_active);
-    TCU(cudaGetLastError());
-    TCU(coupling(I, I.src, 0, nullptr, I.any_active));
-    k_t_clear_k1<<<1, 128, 0, I.st>>>(I.traj, I.B);
-    k_t_out_partial<<<dim3((unsigned)I.nblk, (unsigned)I.B), T_RBLK, 0, I.st>>>(v, I.traj, I.t_eval, I.part, I.nblk);
-    k_t_out_final<<<1, 128, 0, I.st>>>(I.traj, I.part, I.nblk, I.B, I.n, I.out_r, I.out_idx, I.ring);
-    TCU(cudaGetLastError());
-  }
+  // first slope of the run, the record at t0 and the coefficients of the first attempt
+  k_t_first<<<I.B, 32, 0, I.st>>>(I.traj, I.src, I.flags);
+  TCU(cudaGetLastError());
+  TCU(coupling(I, I.src, 0, nullptr, I.flags));
+  TCU(output(I, 1));
   if (!I.graph) {
     cudaGraph_t gr;
     TCU(cudaStreamBeginCapture(I.st, cudaStreamCaptureModeThreadLocal));
@@ -849,12 +945,11 @@ int TensorEngine::run(std::vector<TrajG>& traj, kura_stats& stats, long long max
       TCU(cudaGraphLaunch(I.graph, I.st));
       launches++;
     }
-    TCU(cudaMemcpyAsync(I.h_done, I.done, sizeof(int), cudaMemcpyDeviceToHost, I.st));
+    TCU(cudaMemcpyAsync(I.h_run, I.flags + 1, sizeof(int), cudaMemcpyDeviceToHost, I.st));
+    TCU(cudaMemcpyAsync(I.h_run + 1, I.err, sizeof(int), cudaMemcpyDeviceToHost, I.st));
     TCU(cudaStreamSynchronize(I.st));
-    int errv = 0;
-    TCU(cudaMemcpy(&errv, I.err, sizeof(int), cudaMemcpyDeviceToHost));
-    if (errv) { g_terr = "tensor GEMM aborted (wait time limit)"; return KURA_ERR_BARRIER_TIMEOUT; }
-    if (*I.h_done) break;
+    if (I.h_run[1]) { g_terr = "tensor GEMM aborted (wait time limit)"; return KURA_ERR_BARRIER_TIMEOUT; }
+    if (!I.h_run[0]) break;
     if (I.time_gemm) {  // every replay of this batch stepped some trajectory: sample the last one
       for (int q = 0; q < 6; ++q) {
         float gm = 0.f;

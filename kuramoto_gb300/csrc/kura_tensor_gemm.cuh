@@ -1,10 +1,10 @@
 // kura_tensor_gemm.cuh -- tcgen05 GEMM with a fused epilogue:
-//   C[m][c] = sum_k A[m][k] * X[c][k]      (A: M x K BF16, X: NCOL x K BF16, both K-major)
+//   C[m][c] = sum_k A[m][k] * X[c][k]      (A: M x K, X: NCOL x K, both F16 or both BF16, K-major)
 // accumulated in FP32 in tensor memory.  A work unit is a 128-row tile times one block of
 // NCOL columns (NCOL <= 512); CTAs loop over units (persistent).
 //
 // Roles (192 threads): warp 0 lane 0 streams A and X tiles with TMA (64-byte swizzle, 32
-// BF16 of K per stage, so that even NCOL = 512 keeps 5 stages in flight) into a ring of
+// values of K per stage, so that even NCOL = 512 keeps 5 stages in flight) into a ring of
 // STAGES shared-memory stages; warp 1 lane 0 issues the MMAs (M = 128, N = min(NCOL,
 // 256), K = 16 per instruction) and commits each stage back to the producer; warps 2-5
 // read the accumulator (warp w owns TMEM lanes 32*(w%4)..+31, one tile row per thread)
@@ -48,7 +48,8 @@ template <int NCOL, int MT = 1, int BK = TG_BK> struct TGCfg {
 // sp * xstride .. + NCOL; mtiles counts groups of MT * 128 rows.  The first big_tiles groups
 // run as units of MT row tiles; the rest run one row tile per unit, so that the last wave of
 // a persistent grid holds units of half the work (a tail of one-tile units instead of a
-// partly filled wave of MT-tile units).  Epilogue interface:
+// partly filled wave of MT-tile units).  Epilogue interface: Epi::F16 says which 16-bit type the
+// operands have, and
 // Epi::row(taddr, row, m0, sp) is called by
 // every thread of warps 1-4 with taddr = TMEM address of this thread's accumulator row
 // (lane field set, column 0).  With NCOL <= 256 the accumulator is double-buffered in TMEM,
@@ -105,7 +106,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t idesc = umma::idesc_bf16_f32(TG_BM, C::NMMA);
+  const uint32_t idesc = umma::idesc_f32(Epi::F16, TG_BM, C::NMMA);
 
   if (warp == 0) {
     // ---------------- TMA producer
@@ -180,7 +181,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
               for (int h = 0; h < C::NH; ++h) {
                 const uint32_t xa = x0 + h * C::NMMA * C::ROWB + kk * 32;
                 const uint64_t xd = BK == 64 ? umma::sw128_desc(xa) : umma::sw64_desc(xa);
-                umma::mma_bf16(tacc + mt * NCOL + h * C::NMMA, ad, xd, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
+                umma::mma_16(tacc + mt * NCOL + h * C::NMMA, ad, xd, idesc, (kt > 0 || kk > 0) ? 1u : 0u);
               }
             }
           }
@@ -222,14 +223,14 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
   }
 }
 
-// host: 2-D tensor map of a K-major BF16 matrix [rows][k] (row stride k elements) with a
+// host: 2-D tensor map of a K-major F16 or BF16 matrix [rows][k] (row stride k elements) with a
 // (TG_BK x box_rows) box and the 64-byte swizzle.  cuTensorMapEncodeTiled is fetched from
 // the driver at run time, so the library does not link libcuda.
 typedef CUresult (*PFN_encodeTiled)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                     const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-inline int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows,
-                          int bk = TG_BK) {
+inline int make_tmap_16(CUtensorMap* map, bool f16, const void* base, uint64_t k, uint64_t rows, uint32_t box_rows,
+                        int bk = TG_BK) {
   static PFN_encodeTiled fn = nullptr;
   if (!fn) {
     void* f = nullptr;
@@ -243,7 +244,7 @@ inline int make_tmap_bf16(CUtensorMap* map, const void* base, uint64_t k, uint64
   cuuint64_t strides[1] = {k * 2};
   cuuint32_t box[2] = {(cuuint32_t)bk, box_rows};
   cuuint32_t es[2] = {1, 1};
-  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
+  CUresult r = fn(map, f16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dims, strides, box, es,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, bk == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);

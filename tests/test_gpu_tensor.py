@@ -56,6 +56,42 @@ def test_tensor_rhs_matches_oracle(native, oracle_lib, n, batch, k):
     net.close()
 
 
+# units of one and of two row tiles, clusters of 1 to 8 CTAs along K, part-filled tiles, several
+# waves of clusters, every column width; the tolerance is the test's above
+@pytest.mark.parametrize("n,batch", [(1, 2), (127, 3), (129, 16), (500, 17), (1000, 32), (3001, 64), (3001, 128),
+                                     (6100, 33), (12700, 11), (20000, 128), (38000, 2)])
+def test_tensor_split_gemm_matches_oracle(native, oracle_lib, n, batch):
+    th, om = cauchy_inputs(n, 4)
+    thetas = [(th + 0.1 * b).astype(np.float32) for b in range(batch)]
+    net = make(native, n, 5, thetas, om, [2.5] * batch, seed=3)
+    for b in (0, batch - 1):
+        f, cp = net.rhs(b, thetas[b])
+        fr, cpr = oracle_lib.rhs(thetas[b], om, k=5, c1=2.5, seed=3, fp64=True, onthefly=n > 4096)
+        scale = np.max(np.abs(cpr)) + 1e-3
+        assert np.max(np.abs(cp - cpr)) <= 3e-5 * scale + 1e-7, np.max(np.abs(cp - cpr))
+        assert np.all(np.abs(f - fr) <= 1e-4 * scale + 1e-6 * np.abs(fr))
+    net.close()
+
+
+# the A_lo pass inside the split GEMM's K loop; N*A = hi + lo holds 16 significant bits of an entry
+@pytest.mark.parametrize("n,batch", [(130, 2), (1500, 40), (2100, 128)])
+def test_tensor_split_gemm_general_adjacency(native, oracle_lib, n, batch):
+    rng = np.random.default_rng(n)
+    adj = (rng.random((n, n)) * (rng.random((n, n)) < 0.2) / (0.1 * n)).astype(np.float32)
+    th, om = normal_inputs(n, 5)
+    thetas = [(th + 0.1 * b).astype(np.float32) for b in range(batch)]
+    net = make(native, n, 5, thetas, om, [2.0] * batch, adj=adj)
+    for b in (0, batch - 1):
+        _, cp = net.rhs(b, thetas[b])
+        x = np.stack([np.cos(thetas[b].astype(np.float64)), np.sin(thetas[b].astype(np.float64))], 1)
+        ref = adj.astype(np.float64) @ x
+        # relative errors per term: 2^-17 of the entry, 2^-17 of (cos, sin), 2^-16 of the dropped
+        # lo * lo part and the sums, on the absolute row sums
+        bound = 3 * 2.0**-16 * np.abs(adj.astype(np.float64)).sum(1)
+        assert np.all(np.abs(cp.reshape(n, 2) - ref) <= bound[:, None])
+    net.close()
+
+
 def test_tensor_general_adjacency_split(native, oracle_lib):
     n, batch = 200, 16
     rng = np.random.default_rng(5)
