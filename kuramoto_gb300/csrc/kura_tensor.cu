@@ -7,10 +7,10 @@
 // computed as (N A) x [X_hi | X_lo] with X = [cos | sin] split into F16 hi + lo and FP32
 // accumulation in TMEM; the GEMM epilogue forms g = c_b (sin F_c - cos F_s) / N directly.
 // For the reference's volcano rule N*A_ij is an integer in [-K, K], exact in F16 up to 2048, so
-// the product carries the precision of the hi+lo split of X: 2^-25 absolute, where BF16 parts of
+// the product carries the precision of the hi+lo split of X: 2^-21 absolute, where BF16 parts of
 // the same size and rate hold 2^-18.  A general adjacency is split as 2^p_i N A_ij = A_hi + A_lo
-// with a power of two per row, which keeps a row's largest entry near 2^14 (22 significant bits,
-// and 2^-40 of the largest for the small ones), and the term A_lo X_hi is added by further K steps.
+// with a power of two per row, which keeps a row's largest entry near 2^14: A_hi has 7 significant
+// bits, A_lo 11 more.  The term A_lo X_hi is added by further K steps.
 //
 // The DP45 attempt (dp45_step, dp45.cu:87-141) is a fixed sequence of launches --
 // coefficients, 6 x (stage, GEMM), error norm, controller, outputs -- captured once in a
@@ -41,6 +41,12 @@ constexpr int T_MAXC = 32;  // output crossings handled per step
 #define KURA_GEMM_BK 64
 #endif
 constexpr int TE_BK = KURA_GEMM_BK;
+// X_hi is a multiple of 2^-8 and X_lo the rest to 11 bits (2^-21 absolute): the tensor core cuts each
+// product off at the accumulator's last bit, always toward zero, and the coarse steps leave it
+// nothing to cut from A_hi X_hi.  With X_hi and A_hi of 11 bits each the couplings of n = 6007
+// positive weights were 2.8e-6 off, 2.0e-6 of it bias; they are
+// 2.7e-7 off now (BF16 parts: 1.8e-6), and 3.7e-7 for the volcano rule at n = 20000 (2.3e-6).
+constexpr float X_STEPS = 256.f;
 constexpr int T_RBLK = 256; // rows per block of the reduction kernels
 
 struct TCoef {
@@ -185,7 +191,8 @@ __global__ void k_t_stage(TView v, const TCoef* src) {
   float sn, cs;
   sincos_pair(s2.hi, lo, &sn, &cs);
   v.x32[(size_t)b * v.np + i] = make_float2(cs, sn);
-  const __half ch = __float2half_rn(cs), sh = __float2half_rn(sn);
+  const __half ch = __float2half_rn(rintf(cs * X_STEPS) * (1.f / X_STEPS));
+  const __half sh = __float2half_rn(rintf(sn * X_STEPS) * (1.f / X_STEPS));
   const __half cl = __float2half_rn(cs - __half2float(ch));
   const __half sl = __float2half_rn(sn - __half2float(sh));
   v.X[xrow(0, b, v.bp) * v.np + i] = ch;
@@ -533,7 +540,7 @@ __global__ void k_t_fill(float* p, int n, float v) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
 }
-// general adjacency, one block per row: 2^p N A = hi + lo in F16, with 2^p so that the row's largest
+// general adjacency, one block per row: 2^p N A = hi (7 bits) + lo (11 bits) in F16, with 2^p so that the row's largest
 // entry lies in [2^13, 2^14) (1 for a row of zeros or one that holds an infinity)
 __global__ void k_t_split(const float* __restrict__ adj, int n, int np, float scale, __half* hi, __half* lo,
                           float* rinv) {
@@ -559,7 +566,9 @@ __global__ void k_t_split(const float* __restrict__ adj, int n, int np, float sc
     const float p = smax;
     for (int j = threadIdx.x; j < np; j += blockDim.x) {
       const float a = (i < n && j < n) ? adj[(size_t)i * n + j] * scale * p : 0.f;
-      const __half h = __float2half_rn(a);
+      // Veltkamp's split: the upper 24 - 17 = 7 bits of a (an infinity or NaN stays itself)
+      const float t = 131073.f * a, up = t - (t - a);
+      const __half h = __float2half_rn(isfinite(a) ? up : a);
       hi[(size_t)i * np + j] = h;
       lo[(size_t)i * np + j] = __float2half_rn(a - __half2float(h));
     }

@@ -7,7 +7,7 @@
 // CTAs of a cluster each accumulate K/S of the same unit in their own TMEM, leave the sums in
 // shared memory and finish 1/S of the unit's (row, trajectory) pairs each, adding the S parts in
 // rank order out of the peers' shared memory.  The A_lo pass of a general adjacency runs in the
-// same K loop and accumulates into the X_hi columns.  Measured per launch (ncu): 52 -> 19 us at
+// same K loop and accumulates into the X_lo columns, whose small sums it joins.  Measured per launch (ncu): 52 -> 19 us at
 // n = 3000 with 24 trajectories (24 units x 6 CTAs), 159 -> 59 us at n = 6007 with 64 (24 x 6).
 //
 // Roles (256 threads): warp 0 lane 0 feeds the ring with TMA, warp 1 lane 0 issues the MMAs; then
@@ -137,11 +137,12 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
         const uint32_t a0 = umma::smem_u32(smem + s * C::STAGE_BYTES);
         const uint32_t x0 = a0 + C::A_BYTES;
         const uint32_t idesc = q >= nk ? id_lo : id_hi;
+        const uint32_t acc = tmem + (q >= nk ? NCOL / 2 : 0);
 #pragma unroll
         for (int kk = 0; kk < TS_BK / 16; ++kk)
 #pragma unroll
           for (int mt = 0; mt < MT; ++mt)
-            umma::mma_16(tmem + mt * NCOL, umma::sw128_desc(a0 + mt * C::A1_BYTES + kk * 32),
+            umma::mma_16(acc + mt * NCOL, umma::sw128_desc(a0 + mt * C::A1_BYTES + kk * 32),
                            umma::sw128_desc(x0 + kk * 32), idesc, (q > 0 || kk > 0) ? 1u : 0u);
         umma::mma_commit(&empty[s]);
         if (++s == C::STAGES) { s = 0; ph ^= 1; }
