@@ -47,6 +47,7 @@ def build(verbose: bool = False, ptxas_info: bool = False) -> str:
         cu_flags += ["-Xptxas", "-v"]
     objs = {
         "kura_kernels.o": [nv, *cu_flags, "-c", os.path.join(SRC, "kura_kernels.cu")],
+        "kura_resident.o": [nv, *cu_flags, "-c", os.path.join(SRC, "kura_resident.cu")],
         "kura_api.o": [nv, *cu_flags, "-c", os.path.join(SRC, "kura_api.cu")],
         "kura_noalloc.o": [nv, *cu_flags, "-c", os.path.join(SRC, "kura_noalloc.cu")],
         "kura_tensor.o": [nv, *cu_flags, "-c", os.path.join(SRC, "kura_tensor.cu")],

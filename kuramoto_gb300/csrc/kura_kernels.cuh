@@ -47,6 +47,7 @@ struct KParams {
   float* g;            // [7][B][ld] coupling part of the stage slopes k_j - omega
   float2* xbuf;        // [2][B][ld] (cos, sin) exchanged between CTAs
   float* part;         // [2][grid][B][PW_MAX] per-CTA partial sums
+  unsigned long long* fix;  // [3][B][16] fixed-point sums of the resident integrator (zeroed before each launch)
   unsigned* bar;       // grid barrier arrival counter (zeroed before each launch)
   int* err;            // launch-wide abort code
   TrajG* traj;         // [B]
@@ -90,6 +91,22 @@ cudaError_t launch_volcano_adjacency_i8(const uint32_t* bits, int n, int k, int 
                                         cudaStream_t st);
 cudaError_t launch_volcano_adjacency(const uint32_t* bits, int n, int k, int words, int ld, float* adj,
                                      cudaStream_t st);
+// The resident integrator of a volcano network (kura_resident.cu): how it runs one, mode < 0 where
+// it does not (k > 8, or state that fits no CTA's shared memory).
+// How the rows of a network are split and summed (kura_resident.cuh).
+struct ResSplit {
+  int B, k, rows, vrows, vblocks, ctas;  // rows: the most a CTA holds
+};
+constexpr int RES_MODE_FIXED = 2;  // the form that needs KParams::fix
+struct ResPlan {
+  int mode = -1, hl = 0, grid = 0;
+  ResSplit split{};
+  size_t smem = 0;
+};
+// blocks, rows: the persistent kernel's grid for this network and its rows per CTA
+ResPlan resident_plan(int64_t n, int batch, int k, int blocks, int rows);
+cudaError_t launch_resident(const KParams& p, const ResPlan& r, cudaStream_t st);
+
 // sets the message returned by kura_last_error() for the calling thread
 void set_last_error(const char* msg);
 cudaError_t launch_unwrap(const float* hi, const float* lo, const long long* w, int n, float* out,
