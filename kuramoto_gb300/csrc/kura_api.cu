@@ -267,7 +267,11 @@ extern "C" int kura_create(const kura_config* cfg, kura_handle** out) {
   if (bps < 1) return bail(fail(KURA_ERR_UNSUPPORTED, "persistent kernel shared memory exceeds an SM"));
   h->grid = G;
   h->rows = rows;
-  if (h->coupling == KURA_COUPLING_VOLCANO) h->res = kura::resident_plan(h->n, h->B, h->K, G, rows);
+  if (h->coupling == KURA_COUPLING_VOLCANO)
+    h->res = kura::resident_plan(h->n, h->B, h->K, G, rows);
+  else if (h->B == 1)
+    h->res = uses_i8(cfg) ? kura::resident_plan_dense(kura::RES_I8, (h->n + 15) / 16 * 16, G, rows)
+                          : kura::resident_plan_dense(kura::RES_F32, h->ld, G, rows);
 
   size_t ld = h->ld, B = h->B;
   CUH(dalloc(&h->omega, ld));
@@ -306,7 +310,7 @@ extern "C" int kura_create(const kura_config* cfg, kura_handle** out) {
   h->finished.assign(B, 0);
   h->order.assign(B, {});
   h->stats.grid = h->res.mode >= 0 ? h->res.grid : G;
-  h->stats.block = kura::KT;
+  h->stats.block = h->res.split.den == kura::RES_F32 ? 576 : kura::KT;
   *out = h;
   return KURA_OK;
 #undef CUH

@@ -31,6 +31,7 @@
 #include "kura.h"
 #include "kura_kernels.cuh"
 #include "kura_device.cuh"
+#include "kura_matvec.cuh"
 
 namespace kura {
 
@@ -66,50 +67,6 @@ __device__ __forceinline__ uint4 ld_stream_u4(const int8_t* p) {
 __device__ __forceinline__ float i8_to_f(uint32_t w_biased, int j) {
   return __int_as_float((int)__byte_perm(w_biased, 0x4B000000u, 0x7540u + (unsigned)j)) - 8388736.0f;
 }
-// Packed FP32 pairs (sm_100 and later): one instruction, each half rounded as the scalar
-// operation.  (a.lo*b.lo + c.lo, a.hi*b.hi + c.hi):
-__device__ __forceinline__ unsigned long long ffma2(unsigned long long a, unsigned long long b,
-                                                    unsigned long long c) {
-  unsigned long long d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ float2 unpack_f2(unsigned long long v) {
-  float2 r;
-  asm("mov.b64 {%0,%1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
-// byte j of w0 and of w1 (biased by 0x80, as for i8_to_f) as the exact float pair
-// (lo: w0, hi: w1): both placed under the exponent of 2^23, then 2^23 + 128 subtracted from
-// the pair in one packed add
-__device__ __forceinline__ unsigned long long i8_pair_to_f2(uint32_t w0, uint32_t w1, int j) {
-  const uint32_t lo = __byte_perm(w0, 0x4B000000u, 0x7540u + (unsigned)j);
-  const uint32_t hi = __byte_perm(w1, 0x4B000000u, 0x7540u + (unsigned)j);
-  const unsigned long long bias = 0xCB000080CB000080ull;  // (-8388736.0f, -8388736.0f)
-  unsigned long long d;
-  asm("{\n\t.reg .b64 t;\n\tmov.b64 t, {%1,%2};\n\tadd.rn.f32x2 %0, t, %3;\n\t}"
-      : "=l"(d) : "r"(lo), "r"(hi), "l"(bias));
-  return d;
-}
-// 16 bytes global -> shared without a register round trip (L2 only); src_bytes 0 zero-fills
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, int src_bytes) {
-  const unsigned d = (unsigned)__cvta_generic_to_shared(smem_dst);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(gsrc), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-__device__ __forceinline__ float4 ld_stream4(const float* p) {
-  float4 v;
-  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
-               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-               : "l"(p));
-  return v;
-}
-
 // ------------------------------------------------------------------ per-evaluation source
 // What one coupling evaluation integrates for one trajectory:
 //   theta = phase[base] + omega*(m_hi + m_lo) + sum_j W[j] * g[slot[j]]
@@ -202,8 +159,6 @@ __device__ __forceinline__ int scatter16_index(int lane) {
 template <int COUP, int BMAX, int KMAX>
 struct Engine {
   static constexpr int PW = pw_of(COUP, KMAX);
-  // rows per warp and pass of the dense coupling: each staged x value is reused RG times
-  static constexpr int RG = A_ROWS;
 
   const KParams& p;
   TrajG* tr;
@@ -221,6 +176,7 @@ struct Engine {
   int G, gi, tid, lane, warp, r0, r1, B;
   unsigned target;
   int nbar, xpar;
+  double sqrt_n;
 
   __device__ Engine(const KParams& pp, unsigned char* smem) : p(pp) {
     int off[10], total;
@@ -240,6 +196,7 @@ struct Engine {
     tid = threadIdx.x;
     lane = tid & 31;
     warp = tid >> 5;
+    sqrt_n = sqrt((double)p.n);
     r0 = min(p.n, gi * p.rows);
     r1 = min(p.n, r0 + p.rows);
     B = p.batch;
@@ -279,7 +236,9 @@ struct Engine {
     __syncthreads();
     target += (unsigned)G;
     if (tid == 0) {
-      __threadfence();
+      // The release covers what the CTA's other threads wrote before the block barrier, and the
+      // acquire below what the block reads after the next one: no further fence on either side
+      // (two membars cost about 1 us per barrier).
       red_release_add(p.bar, 1u);
       unsigned long long t0 = global_ns();
       int abort = 0;
@@ -294,7 +253,6 @@ struct Engine {
           break;
         }
       }
-      __threadfence();
       flag[0] = abort;
     }
     __syncthreads();
@@ -682,7 +640,15 @@ struct Engine {
       need_F |= sbb.active && (sbb.gout >= 0 || (sbb.rec && (p.dense_level >= 2 || p.mode != MODE_INTEGRATE)));
     }
     if (need_part) publish_partials(npw);
-    if (!grid_sync()) return false;
+    bool ahead = false;
+    if constexpr (COUP == KURA_COUPLING_DENSE) {
+      // the first chunks of A do not depend on the other CTAs: they land during the barrier
+      if ((ahead = need_F)) matvec().first_chunks();
+    }
+    if (!grid_sync()) {
+      if (ahead) cp_async_wait<0>();
+      return false;
+    }
     if (need_part) gather_partials(npw);
 
     // phase C: couplings for the CTA's rows
@@ -790,262 +756,25 @@ struct Engine {
     return true;
   }
 
-  // A (rows r0..r1 of this CTA) times the (cos, sin) of every trajectory.  x is
-  // staged in shared memory one column tile at a time; each warp works on up to RG rows,
-  // each lane on 16-byte chunks of them.
+  // A (rows r0..r1 of this CTA) times the (cos, sin) of every trajectory (kura_matvec.cuh)
   static constexpr int CTF = BMAX == 1 ? CT_F1 : CT;  // columns per x tile of the float product
-  // A lane's 4 columns of x are 32 bytes from the next lane's, so back to back they would
-  // fall on four of the eight 16-byte bank groups; a stride of F_CHUNK = 6 (cos, sin) pairs
-  // (48 bytes) per 4 columns uses all eight.
-  static constexpr int CTFP = CTF / 4 * F_CHUNK;
-  // One x tile for the NR rows this warp holds.  A streams through the warp's ring of
-  // A_STAGES * RG chunk slots with cp.async: every lane copies its own 16 bytes of each
-  // row, ST = A_STAGES * RG / NR column steps ahead, and reads back only what it copied,
-  // so the ring needs no barrier and holds no registers per byte in flight.  A warp with
-  // fewer rows (small N, the last pass) keeps as many bytes in flight with more steps.
-  // The prologue's copies start before the x tile has landed; neither part holds a barrier,
-  // so warps with different NR run side by side between the caller's barriers.
-  template <int NR>
-  __device__ __forceinline__ void mv_f32_prologue(float4* my, const float* const (&src)[RG], int c0, int nit) {
-    constexpr int ST = A_STAGES * RG / NR;
-    static_assert(ST * NR <= A_STAGES * RG, "ring slots");
-#pragma unroll
-    for (int s = 0; s < ST - 1; ++s) {
-      if (s < nit)
-#pragma unroll
-        for (int q = 0; q < NR; ++q) cp_async16(my + (s * NR + q) * 32, src[q] + c0 + 128 * s, 16);
-      cp_async_commit();
-    }
-    cp_async_wait<ST - 1>();  // this thread's copies of the x tile, committed before, have landed
+  __device__ __forceinline__ MatvecF32<BMAX, CTF> matvec() const {
+    return {p.adj, p.ld, r0, r1, B, xt, ring, tid, KT, lane, warp, KW};
   }
-  template <int NR>
-  __device__ __forceinline__ void mv_f32_steps(float4* my, const float* const (&src)[RG], int c0, int nit,
-                                               float (&acc)[RG][BMAX][2]) {
-    constexpr int ST = A_STAGES * RG / NR;
-    for (int it = 0; it < nit; ++it) {
-      const int ahead = it + ST - 1;
-      if (ahead < nit) {
-        const int sl = ahead % ST;
-#pragma unroll
-        for (int q = 0; q < NR; ++q) cp_async16(my + (sl * NR + q) * 32, src[q] + c0 + 128 * ahead, 16);
-      }
-      cp_async_commit();
-      cp_async_wait<ST - 1>();  // the chunks of step it have landed
-      const int sl = it % ST;
-      float4 a[NR];
-#pragma unroll
-      for (int q = 0; q < NR; ++q) a[q] = my[(sl * NR + q) * 32];
-      const int cc = lane * 4 + 128 * it;
-#pragma unroll
-      for (int b = 0; b < BMAX; ++b) {
-        if (b < B) {
-          const float4* xp = reinterpret_cast<const float4*>(xt + b * CTFP + (cc >> 2) * F_CHUNK);
-          float4 x01 = xp[0], x23 = xp[1];  // (c0,s0,c1,s1), (c2,s2,c3,s3)
-#pragma unroll
-          for (int q = 0; q < NR; ++q) {
-            acc[q][b][0] += a[q].x * x01.x + a[q].y * x01.z + a[q].z * x23.x + a[q].w * x23.z;
-            acc[q][b][1] += a[q].x * x01.y + a[q].y * x01.w + a[q].z * x23.y + a[q].w * x23.w;
-          }
-        }
-      }
-    }
-    cp_async_wait<0>();
-  }
-
   __device__ void dense_matvec() {
-    const int ld = p.ld;
-    const int rows_per_pass = KW * RG;
-    float4* my = ring + (size_t)warp * (A_STAGES * RG * 32) + lane;
-    for (int pr0 = r0; pr0 < r1; pr0 += rows_per_pass) {
-      float acc[RG][BMAX][2];
-#pragma unroll
-      for (int q = 0; q < RG; ++q)
-#pragma unroll
-        for (int b = 0; b < BMAX; ++b) acc[q][b][0] = acc[q][b][1] = 0.f;
-      // warp w takes rows pr0 + w + KW*q of the pass, so small row blocks keep every warp
-      // busy; its nr rows in the CTA's block are q < nr
-      const int row0 = pr0 + warp;
-      const int nr = r1 > row0 ? min(RG, (r1 - row0 + KW - 1) / KW) : 0;
-      const float* src[RG];
-#pragma unroll
-      for (int q = 0; q < RG; ++q) {
-        const int row = row0 + KW * q;
-        src[q] = p.adj + (size_t)(row < r1 ? row : r0) * ld + lane * 4;
-      }
-      int c0 = 0;
-      for (; c0 < ld; c0 += CTF) {
-        __syncthreads();  // the previous tile's readers are done
-        const int cw = min(CTF, ld - c0);  // a multiple of 32
-        // the x tile, 16 bytes (two columns) per copy, in one commit group ahead of the ring's
-        for (int b = 0; b < B; ++b)
-          for (int c = 2 * tid; c < cw; c += 2 * KT)
-            cp_async16(xt + b * CTFP + (c >> 2) * F_CHUNK + (c & 3), p.xbuf + ((size_t)xpar * B + b) * ld + c0 + c,
-                       16);
-        cp_async_commit();
-        // column steps of this lane: cc = lane*4 + 128*it < cw
-        const int nit = (cw - lane * 4 + 127) >> 7;
-        if (nr == 4) mv_f32_prologue<4>(my, src, c0, nit);
-        else if (nr == 3) mv_f32_prologue<3>(my, src, c0, nit);
-        else if (nr == 2) mv_f32_prologue<2>(my, src, c0, nit);
-        else if (nr == 1) mv_f32_prologue<1>(my, src, c0, nit);
-        else cp_async_wait<0>();
-        __syncthreads();  // every thread's part of the x tile has landed
-        if (nr == 4) mv_f32_steps<4>(my, src, c0, nit, acc);
-        else if (nr == 3) mv_f32_steps<3>(my, src, c0, nit, acc);
-        else if (nr == 2) mv_f32_steps<2>(my, src, c0, nit, acc);
-        else if (nr == 1) mv_f32_steps<1>(my, src, c0, nit, acc);
-      }
-      const int xt_c0 = c0 - CTF;  // first column of the tile still staged
-#pragma unroll
-      for (int q = 0; q < RG; ++q)
-        if (q < nr)
-#pragma unroll
-          for (int b = 0; b < BMAX; ++b) {
-            acc[q][b][0] = warp_sum(acc[q][b][0]);
-            acc[q][b][1] = warp_sum(acc[q][b][1]);
-          }
-      // lane q*BMAX+b finishes row row0+q of trajectory b; its own (cos, sin) come from the
-      // staged tile when the last tile holds the row
-#pragma unroll
-      for (int q = 0; q < RG; ++q)
-#pragma unroll
-        for (int b = 0; b < BMAX; ++b) {
-          int row = row0 + KW * q;
-          if (lane == q * BMAX + b && b < B && row < r1 && sb[b].active) {
-            const int c = row - xt_c0;
-            const float2 x = c >= 0 ? xt[b * CTFP + (c >> 2) * F_CHUNK + (c & 3)]
-                                    : __ldcg(&p.xbuf[((size_t)xpar * B + b) * ld + row]);
-            epilogue(b, row, acc[q][b][0], acc[q][b][1], x.x, x.y);
-          }
-        }
-    }
+    matvec().run(p.xbuf + (size_t)xpar * B * p.ld, [&](int b, int row, float Fc, float Fs, float2 x) {
+      if (sb[b].active) epilogue(b, row, Fc, Fs, x.x, x.y);
+    });
+  }
+  __device__ void dense_matvec_i8_one() {
+    const MatvecI8 mv{p.adj8, p.invn, p.ld8, r0, r1, reinterpret_cast<float4*>(xt), reinterpret_cast<uint4*>(ring),
+                      tid, KT, lane, warp, KW};
+    mv.run(p.xbuf + (size_t)xpar * p.ld, [&](int row, float Fc, float Fs, float2 x) {
+      if (sb[0].active) epilogue(0, row, Fc, Fs, x.x, x.y);
+    });
   }
 
-  static constexpr int CTX = BMAX == 1 ? CT_I8 : CT;  // columns per x tile of the int8 product
-  // The int8 product's x tile holds per column the float4 (cos, cos, sin, sin), so that one
-  // packed FP32 FMA multiplies the converted bytes of two rows by the same column.  A lane's
-  // 16 columns start I8_CHUNK4 = 17 float4 (272 bytes) after the previous lane's, which puts
-  // the 8 lanes of each phase of a 16-byte shared-memory read on distinct banks.
-  static constexpr int CTXP = CTX / 16 * I8_CHUNK4;  // float4 per trajectory
-  // The columns [c0, c0 + cw) of the staged tile for the first RGT of the pass's RG_I8 rows of
-  // this warp (rows pr0 + warp + KW*q), 16 int8 columns per lane and step; rows 2qp and 2qp+1
-  // share the packed accumulators acc[qp].  A streams through the warp's ring of I8_SLOTS
-  // chunk slots (16 bytes per lane) with cp.async, I8_SLOTS / RGT steps deep, so the loads of
-  // the next step are in flight during this step's conversion and FMAs.  No barrier inside:
-  // warps with different RGT run side by side between the tile barriers of the caller.
-  static constexpr int RG_I8 = 8;
-  template <int RGT>
-  __device__ __forceinline__ void mv_i8_tile(unsigned long long (&acc)[RG_I8 / 2][2], int row0, int c0, int cw) {
-    static_assert(RGT % 2 == 0 && RGT <= RG_I8 && I8_SLOTS % RGT == 0, "rows are taken in pairs");
-    constexpr int ST = I8_SLOTS / RGT;
-    const int ld8 = p.ld8;
-    const float4* xt4 = reinterpret_cast<const float4*>(xt);
-    uint4* my = reinterpret_cast<uint4*>(ring) + (size_t)warp * (I8_SLOTS * 32) + lane;
-    const int8_t* src[RGT];
-    int nb[RGT];
-#pragma unroll
-    for (int q = 0; q < RGT; ++q) {
-      const int row = row0 + KW * q;
-      nb[q] = row < r1 ? 16 : 0;  // rows past the CTA's block are zero-filled
-      src[q] = p.adj8 + (size_t)(row < r1 ? row : r0) * ld8 + c0 + lane * 16;
-    }
-    // steps of this lane: columns cc = lane*16 + 512*it < cw (cw is a multiple of 16)
-    const int nit = cw > lane * 16 ? (cw - lane * 16 + 511) >> 9 : 0;
-#pragma unroll
-    for (int s = 0; s < ST - 1; ++s) {
-      if (s < nit)
-#pragma unroll
-        for (int q = 0; q < RGT; ++q) cp_async16(my + (s * RGT + q) * 32, src[q] + 512 * s, nb[q]);
-      cp_async_commit();
-    }
-    for (int it = 0; it < nit; ++it) {
-      const int ahead = it + ST - 1;
-      if (ahead < nit) {
-        const int sl = ahead % ST;
-#pragma unroll
-        for (int q = 0; q < RGT; ++q) cp_async16(my + (sl * RGT + q) * 32, src[q] + 512 * ahead, nb[q]);
-      }
-      cp_async_commit();
-      cp_async_wait<ST - 1>();  // the chunks of step it have landed
-      const int sl = it % ST;
-      uint32_t a[RGT][4];
-#pragma unroll
-      for (int q = 0; q < RGT; ++q) {
-        const uint4 v = my[(sl * RGT + q) * 32];
-        a[q][0] = v.x ^ 0x80808080u;
-        a[q][1] = v.y ^ 0x80808080u;
-        a[q][2] = v.z ^ 0x80808080u;
-        a[q][3] = v.w ^ 0x80808080u;
-      }
-      const int cc = lane * 16 + 512 * it;
-#pragma unroll
-      for (int wd = 0; wd < 4; ++wd) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          // ((cos, cos), (sin, sin)) of column cc + 4*wd + j
-          const ulonglong2 xj = *reinterpret_cast<const ulonglong2*>(xt4 + (cc >> 4) * I8_CHUNK4 + 4 * wd + j);
-#pragma unroll
-          for (int qp = 0; qp < RGT / 2; ++qp) {
-            const unsigned long long kp = i8_pair_to_f2(a[2 * qp][wd], a[2 * qp + 1][wd], j);
-            acc[qp][0] = ffma2(kp, xj.x, acc[qp][0]);
-            acc[qp][1] = ffma2(kp, xj.y, acc[qp][1]);
-          }
-        }
-      }
-    }
-    cp_async_wait<0>();
-  }
-  // one pass over the RG_I8 rows per warp of one trajectory
-  __device__ void mv_i8_pass(int pr0) {
-    const int ld = p.ld, ld8 = p.ld8;
-    float4* xt4 = reinterpret_cast<float4*>(xt);
-    // [qp][0]: (sum k cos) of rows (2qp, 2qp+1); [qp][1]: the same for sin
-    unsigned long long acc[RG_I8 / 2][2];
-#pragma unroll
-    for (int q = 0; q < RG_I8 / 2; ++q) acc[q][0] = acc[q][1] = 0ull;
-    const int row0 = pr0 + warp;
-    const int nr = r1 > row0 ? min(RG_I8, (r1 - row0 + KW - 1) / KW) : 0;
-    int c0 = 0;
-    for (; c0 < ld8; c0 += CTX) {
-      __syncthreads();
-      const int cw = min(CTX, ld8 - c0);  // a multiple of 16
-      for (int c = tid; c < cw; c += KT) {
-        const float2 x = __ldcg(&p.xbuf[(size_t)xpar * ld + c0 + c]);
-        xt4[(c >> 4) * I8_CHUNK4 + (c & 15)] = make_float4(x.x, x.x, x.y, x.y);
-      }
-      __syncthreads();
-      // a warp with at most 4 rows in the pass (small N, the last pass) converts no bytes of
-      // the absent ones
-      if (nr <= 4) mv_i8_tile<4>(acc, row0, c0, cw);
-      else mv_i8_tile<RG_I8>(acc, row0, c0, cw);
-    }
-    float accf[RG_I8][2];
-#pragma unroll
-    for (int qp = 0; qp < RG_I8 / 2; ++qp)
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const float2 u = unpack_f2(acc[qp][v]);
-        accf[2 * qp][v] = warp_sum(u.x);
-        accf[2 * qp + 1][v] = warp_sum(u.y);
-      }
-    // the row's own (cos, sin) from the staged tile when the last tile holds it
-    const int xt_c0 = c0 - CTX;
-#pragma unroll
-    for (int q = 0; q < RG_I8; ++q) {
-      const int row = row0 + KW * q;
-      if (lane == q && row < r1 && sb[0].active) {
-        const int c = row - xt_c0;
-        float2 x;
-        if (c >= 0) {
-          const float4 v = xt4[(c >> 4) * I8_CHUNK4 + (c & 15)];
-          x = make_float2(v.x, v.z);
-        } else {
-          x = __ldcg(&p.xbuf[(size_t)xpar * ld + row]);
-        }
-        epilogue(0, row, accf[q][0] * p.invn, accf[q][1] * p.invn, x.x, x.y);
-      }
-    }
-  }
+  static constexpr int CTX = CT;  // columns per x tile of the int8 product of a batch
   // The batch form: x tile of (cos, sin) pairs, I8_CHUNK = 18 pairs (144 bytes) per 16
   // columns, and one scalar FMA per byte, trajectory and sum; the register budget of eight
   // trajectories leaves no room for the packed form's operands.
@@ -1126,19 +855,12 @@ struct Engine {
         }
       }
   }
-  // The same product with A stored as the integers N*A (int8, exact for the reference's
-  // volcano rule, K <= 127): a quarter of the HBM bytes.  Each lane streams 16 columns of
-  // 8 rows (one trajectory) or 2 rows (a batch) per load; the sums are scaled by 1/N
-  // before the epilogue.  One trajectory converts the bytes of two rows at a time into a
-  // packed float pair and multiplies it by a column's (cos, cos) and (sin, sin) with packed
-  // FMAs: 2.5 instructions per byte and trajectory instead of 4.  (16 rows of 8 columns
-  // halves the shared-memory reads of x but measured 2x slower at N=65536: half the bytes in
-  // flight per load.)
   __device__ void dense_matvec_i8() {
-    constexpr int RG = BMAX == 1 ? 8 : 2;
-    for (int pr0 = r0; pr0 < r1; pr0 += KW * RG) {
-      if constexpr (BMAX > 1) mv_i8_pass_batch<RG, 16>(pr0);
-      else mv_i8_pass(pr0);
+    if constexpr (BMAX > 1) {
+      constexpr int RG = 2;
+      for (int pr0 = r0; pr0 < r1; pr0 += KW * RG) mv_i8_pass_batch<RG, 16>(pr0);
+    } else {
+      dense_matvec_i8_one();
     }
   }
 
@@ -1283,7 +1005,7 @@ struct Engine {
     bool accept = true;
     double factor = 1.0;
     if (!p.fixed) {
-      double norm = sqrt((double)rsum[b * PW]) / sqrt((double)p.n);
+      double norm = sqrt((double)rsum[b * PW]) / sqrt_n;
       if (isnan(norm)) {
         T.status = KURA_ERR_NONFINITE;
         return;

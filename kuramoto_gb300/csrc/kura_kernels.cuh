@@ -91,12 +91,14 @@ cudaError_t launch_volcano_adjacency_i8(const uint32_t* bits, int n, int k, int 
                                         cudaStream_t st);
 cudaError_t launch_volcano_adjacency(const uint32_t* bits, int n, int k, int words, int ld, float* adj,
                                      cudaStream_t st);
-// The resident integrator of a volcano network (kura_resident.cu): how it runs one, mode < 0 where
-// it does not (k > 8, or state that fits no CTA's shared memory).
+// The resident integrator (kura_resident.cu): how it runs a network, mode < 0 where it does not
+// (volcano rank above 8, a stored adjacency with a batch, or state that fits no CTA's shared memory).
 // How the rows of a network are split and summed (kura_resident.cuh).
 struct ResSplit {
   int B, k, rows, vrows, vblocks, ctas;  // rows: the most a CTA holds
+  int den, ld;  // stored adjacency: RES_F32 or RES_I8 with rows of ld values; 0: regenerated coupling
 };
+enum { RES_F32 = 1, RES_I8 = 2 };
 constexpr int RES_MODE_FIXED = 2;  // the form that needs KParams::fix
 struct ResPlan {
   int mode = -1, hl = 0, grid = 0;
@@ -105,6 +107,7 @@ struct ResPlan {
 };
 // blocks, rows: the persistent kernel's grid for this network and its rows per CTA
 ResPlan resident_plan(int64_t n, int batch, int k, int blocks, int rows);
+ResPlan resident_plan_dense(int den, int ld, int blocks, int rows);
 cudaError_t launch_resident(const KParams& p, const ResPlan& r, cudaStream_t st);
 
 // sets the message returned by kura_last_error() for the calling thread

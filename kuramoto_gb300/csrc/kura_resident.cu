@@ -1,5 +1,6 @@
 // kura_resident.cu -- the resident integrator (kura_resident.cuh) for one volcano network and its
-// batch of trajectories: kernels, the choice of shape, and the launch.  Stands in for the persistent
+// batch of trajectories, or one trajectory of a stored adjacency: kernels, the choice of shape, and
+// the launch.  Stands in for the persistent
 // kernel in MODE_INTEGRATE wherever a CTA's share of the state fits in shared memory.
 #include "kura_resident.cuh"
 
@@ -7,14 +8,18 @@ namespace kura {
 namespace {
 
 constexpr int NT = 512;
+// 18 warps for the float product: 33 rows per CTA (N = 5000) are two rows per warp, where 16 warps
+// would wait for the one that has three
+constexpr int NT_F32 = 576;
+__host__ __device__ constexpr int threads_of(int den) { return den == RES_F32 ? NT_F32 : NT; }
 constexpr size_t SMEM_CAP = 227 * 1024 - 256;
 
-template <int MODE, bool HL>
-__global__ void __launch_bounds__(NT, 1) k_resident(const KParams p, const ResSplit split) {
-  extern __shared__ __align__(16) unsigned char smem[];
+template <int MODE, bool HL, int DEN = 0>
+__global__ void __launch_bounds__(threads_of(DEN), 1) k_resident(const KParams p, const ResSplit split) {
+  extern __shared__ __align__(128) unsigned char smem[];
   __shared__ ResNet net;
   if (threadIdx.x == 0) {
-    net.n = p.n; net.k = p.k; net.B = p.batch; net.seed = p.seed; net.split = split;
+    net.n = p.n; net.k = split.k; net.B = p.batch; net.seed = p.seed; net.split = split;
     net.omega = p.omega;
     net.hi = p.ph_hi; net.lo = p.ph_lo; net.w = p.ph_w; net.g = p.g;
     net.ld = p.ld;
@@ -24,9 +29,10 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const KParams p, const ResSp
     net.out_ld = p.ld; net.ring = p.ring;
     net.log_t = p.log_t; net.log_h = p.log_h; net.log_cap = p.log_cap;
     net.max_attempts = p.max_attempts;
+    net.adj = p.adj; net.adj8 = p.adj8; net.invn = p.invn; net.x = p.xbuf;
   }
   __syncthreads();
-  Resident<MODE, HL, NT> e(net, smem, blockIdx.x, gridDim.x);
+  Resident<MODE, HL, threads_of(DEN), DEN> e(net, smem, blockIdx.x, gridDim.x);
   e.bar = p.bar;
   e.bar_extra = p.bar_extra;
   e.err = p.err;
@@ -46,7 +52,9 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const KParams p, const ResSp
   }
 }
 
-const void* pick(int mode, int hl) {
+const void* pick(int mode, int hl, int den) {
+  if (den == RES_F32) return (const void*)&k_resident<RES_GRIDX, true, RES_F32>;
+  if (den == RES_I8) return (const void*)&k_resident<RES_GRIDX, true, RES_I8>;
   if (mode == RES_ONE) return hl ? (const void*)&k_resident<RES_ONE, true> : nullptr;
   if (mode == RES_CLUSTER) return hl ? (const void*)&k_resident<RES_CLUSTER, true> : nullptr;
   if (mode == RES_GRIDX) return hl ? (const void*)&k_resident<RES_GRIDX, true> : nullptr;
@@ -54,12 +62,12 @@ const void* pick(int mode, int hl) {
 }
 
 cudaError_t configure(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const ResPlan& r, cudaStream_t st) {
-  const void* f = pick(r.mode, r.hl);
+  const void* f = pick(r.mode, r.hl, r.split.den);
   cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem);
   if (e == cudaSuccess && r.mode == RES_CLUSTER && r.grid > 8)
     e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cfg->gridDim = dim3((unsigned)r.grid);
-  cfg->blockDim = dim3(NT);
+  cfg->blockDim = dim3(threads_of(r.split.den));
   cfg->dynamicSmemBytes = r.smem;
   cfg->stream = st;
   cfg->attrs = attr;
@@ -80,13 +88,13 @@ cudaError_t configure(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const 
 
 // fills *r for a launch of `ctas` CTAs; blocks, rows: the grid of the persistent kernel and its rows
 // per CTA.  False when the state does not fit.
-bool shape(ResPlan* r, int B, int k, int blocks, int rows, int mode, int ctas, int hl) {
+bool shape(ResPlan* r, int B, int k, int blocks, int rows, int mode, int ctas, int hl, int den = 0, int ld = 0) {
   r->mode = mode;
   r->hl = hl;
   r->grid = ctas;
-  r->split = {B, k, mode == RES_GRID ? rows : (blocks + ctas - 1) / ctas * rows, rows, blocks, ctas};
-  int off[16];
-  r->smem = res_layout(r->split, hl, mode, NT, off);
+  r->split = {B, k, mode == RES_GRID ? rows : (blocks + ctas - 1) / ctas * rows, rows, blocks, ctas, den, ld};
+  int off[18];
+  r->smem = res_layout(r->split, hl, mode, threads_of(den), off);
   return r->smem <= SMEM_CAP && (mode == RES_GRID || r->split.rows < 65536);
 }
 
@@ -121,7 +129,7 @@ ResPlan resident_plan(int64_t n, int B, int k, int blocks, int rows) {
       cudaLaunchAttribute attr[1];
       int fit = 0;
       if (configure(&cfg, attr, r, nullptr) == cudaSuccess &&
-          cudaOccupancyMaxActiveClusters(&fit, pick(r.mode, r.hl), &cfg) == cudaSuccess && fit >= 1)
+          cudaOccupancyMaxActiveClusters(&fit, pick(r.mode, r.hl, r.split.den), &cfg) == cudaSuccess && fit >= 1)
         return r;
       cudaGetLastError();
     }
@@ -129,6 +137,15 @@ ResPlan resident_plan(int64_t n, int B, int k, int blocks, int rows) {
   if (n < FIXED_N) return rows < 1024 && shape(&r, B, k, blocks, rows, RES_GRIDX, blocks, 1) ? r : ResPlan();
   for (int hl = 1; hl >= 0; --hl)
     if (shape(&r, B, k, blocks, rows, RES_GRID, blocks, hl)) return r;
+  return ResPlan();
+}
+
+// One trajectory of a stored adjacency: wherever the state fits beside the x tile and the ring (N up
+// to about 80000 in float32, 70000 in int8) and a CTA has fewer than 1024 rows, from where on the
+// persistent kernel forms its sums in another order.
+ResPlan resident_plan_dense(int den, int ld, int blocks, int rows) {
+  ResPlan r;
+  if (rows < 1024 && shape(&r, 1, 0, blocks, rows, RES_GRIDX, blocks, 1, den, ld)) return r;
   return ResPlan();
 }
 
@@ -140,7 +157,7 @@ cudaError_t launch_resident(const KParams& p, const ResPlan& r, cudaStream_t st)
   cudaError_t e = configure(&cfg, attr, r, st);
   if (e != cudaSuccess) return e;
   void* args[] = {&q, &split};
-  return cudaLaunchKernelExC(&cfg, pick(r.mode, r.hl), args);
+  return cudaLaunchKernelExC(&cfg, pick(r.mode, r.hl, r.split.den), args);
 }
 
 }  // namespace kura

@@ -1,5 +1,4 @@
-// kura_resident.cuh -- DP45 of the regenerated-volcano network with the state of a CTA's rows held in
-// shared memory for the whole launch.
+// kura_resident.cuh -- DP45 with the state of a CTA's rows held in shared memory for the whole launch.
 //
 // The persistent kernel (kura_kernels.cu) keeps phases and slopes in L2 and reads up to nine values
 // per oscillator and stage from there; with 64-bit addressing, a second pass over the rows for the
@@ -24,6 +23,12 @@
 // heavy-tailed frequencies the controller of a small network amplifies a rounding of its sums
 // (1e-8 becomes 1e-6 of the phases within a hundred steps at n = 1000), so another order, although
 // as exact, would be another run.  RES_GRID, for large networks, adds in fixed point.
+//
+// One trajectory of a stored adjacency runs the same way (template DEN) in the RES_GRIDX form: the
+// CTAs publish (cos, sin) instead of sums, and after the barrier each forms its rows' couplings with
+// kura_matvec.cuh in the place of the table.  Per attempt, against the persistent kernel: 49 -> 36 us
+// at N = 997, 106 -> 89 at 5000 (A from L2 at 12 TB/s is 58 of them), 14.9 -> 14.1 ms at 65536
+// (7.3 TB/s of A).
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>
@@ -31,6 +36,7 @@
 #include "kura.h"
 #include "kura_device.cuh"
 #include "kura_kernels.cuh"
+#include "kura_matvec.cuh"
 
 namespace kura {
 
@@ -65,7 +71,13 @@ struct ResNet {
   double *log_t, *log_h;
   int log_cap;
   long long max_attempts;
+  // stored adjacency
+  const float* adj;
+  const int8_t* adj8;
+  float invn;
+  float2* x;  // [2][ld] (cos, sin) of all rows, by parity of the exchange
 };
+constexpr int RES_CTF = 7168;  // columns per x tile of the float product: leaves room for the state at N = 65536
 
 // How the rows of a network are split and summed.  RES_GRID: CTA i owns rows i * rows ..; the
 // others: the sums are formed over blocks of vrows rows, vblocks of them, as a grid of vblocks CTAs
@@ -89,7 +101,7 @@ __host__ __device__ inline size_t res_layout(const ResSplit& s, int hl, int mode
   };
   take(B * (int)sizeof(TrajG));            // 0 controllers
   take(B * RES_ROWS_WT * RES_WT * 4);      // 1 weights
-  take(16);                                // 2 (free)
+  take(B * 8);                             // 2 next output time
   take((mode == RES_GRID ? (nt / 32) * 2 : B * nu) * RES_RED * 4);  // 3 warps' or units' sums
   take(B * RES_RED * 4);                   // 4 totals
   take(mode >= RES_GRID ? 0 : (mode == RES_CLUSTER ? 2 : 1) * s.vblocks * B * RES_RED * 4);  // 5 totals of every block
@@ -102,10 +114,18 @@ __host__ __device__ inline size_t res_layout(const ResSplit& s, int hl, int mode
   take(np * 8);                            // 12 (cos, sin)
   take(6 * np * 4);                        // 13 slopes
   take(hl ? np * 8 : 0);                   // 14 phases (hi, lo)
+  if (s.den) {
+    const int warps = nt / 32, cf = s.ld < RES_CTF ? s.ld : RES_CTF, ci = s.ld < CT_I8 ? s.ld : CT_I8;
+    take(s.rows * 8);                                                                    // 15 couplings
+    o = (o + 127) & ~127;  // copies into the ring are faster from a line boundary (1.2x at N = 65536)
+    take(s.den == RES_F32 ? (cf + 3) / 4 * F_CHUNK * 8 : (ci + 15) / 16 * I8_CHUNK4 * 16);  // 16 x tile
+    o = (o + 127) & ~127;
+    take(warps * 32 * 16 * (s.den == RES_F32 ? A_STAGES * A_ROWS : I8_SLOTS));             // 17 ring of A
+  }
   return (size_t)o;
 }
 
-template <int MODE, bool HL, int NT>
+template <int MODE, bool HL, int NT, int DEN = 0>
 struct Resident {
   static constexpr int NW = NT / 32;
   static constexpr bool EX = MODE != RES_GRID;  // sums in the persistent kernel's order
@@ -114,6 +134,9 @@ struct Resident {
   float *wt, *red, *rsum, *ex, *slice;
   uint32_t* ut;  // of a unit: first row and the end of its block
   float2* tab;
+  float2* Fr;  // DEN: couplings of the rows
+  float4 *xt, *ring;
+  double* te;  // per trajectory: the next output time
   int* flag;
   int* ps;  // per trajectory: phase buffer, candidate state, record slot, record index
   int* wr;  // per trajectory: first and last warp that hold rows of it, and the first one's entry in red
@@ -134,11 +157,12 @@ struct Resident {
   int* err;
   float* part;
   unsigned long long timeout_ns;
-  int nbar, par, nfix;
+  int nbar, par, nfix, xpar;
+  bool rec0;  // the pass over y (kind 0) records r
 
   __device__ Resident(const ResNet& net, unsigned char* smem, int gi_, int G_) : N(net), gi(gi_), G(G_) {
     const ResSplit& sp = net.split;
-    int off[16];
+    int off[18];
     res_layout(sp, HL, MODE, NT, off);
     tr = (TrajG*)(smem + off[0]);
     wt = (float*)(smem + off[1]);
@@ -156,6 +180,13 @@ struct Resident {
     xs = (float2*)(smem + off[12]);
     g = (float*)(smem + off[13]);
     yy = (float2*)(smem + off[14]);
+    te = (double*)(smem + off[2]);
+    if (DEN) {
+      Fr = (float2*)(smem + off[15]);
+      xt = (float4*)(smem + off[16]);
+      ring = (float4*)(smem + off[17]);
+    }
+    xpar = 0;
     tid = threadIdx.x;
     lane = tid & 31;
     warp = tid >> 5;
@@ -277,8 +308,9 @@ struct Resident {
   // blocks -> rsum: the same additions in the same order as a grid of vblocks CTAs of the persistent
   // kernel, so that a run gives the same bits however many CTAs carry it.
   // npw: the values per trajectory that the persistent kernel would gather at once.
-  __device__ __forceinline__ bool exchange_blocks(int v0, int nv, bool proj, int npw) {
-    __syncthreads();
+  // DEN, want_F: the couplings of the rows as well; nv may be 0 then.
+  __device__ __forceinline__ bool exchange_blocks(int v0, int nv, bool proj, int npw, bool want_F = false) {
+    if (!DEN || nv) __syncthreads();
     const int NV = B * nv, VB = N.split.vblocks;
     float* mine = ex + (MODE == RES_CLUSTER ? par * VB * B * RES_RED : 0);
     // thread t of a round: value q of block vb; a block's NV values fill vstep threads
@@ -316,7 +348,11 @@ struct Resident {
       // a CTA reaches only when it has read them
       par ^= 1;
     } else if (MODE == RES_GRIDX) {
-      if (!grid_sync()) return false;
+      if (DEN == RES_F32 && want_F) mv_f32().first_chunks();  // they land during the barrier
+      if (!grid_sync()) {
+        if (DEN) cp_async_wait<0>();
+        return false;
+      }
       mine = part + (size_t)((nbar - 1) & 1) * VB * NV;
     } else {
       __syncthreads();
@@ -324,7 +360,7 @@ struct Resident {
     int S = 128 / npw;
     if (S < 1) S = 1;
     if (S > (VB + 15) / 16) S = (VB + 15) / 16;
-    if (S > 1) {
+    if (S > 1 && NV) {
       for (int sl = tid / vstep; sl < S; sl += NT / vstep) {
         if (q >= NV) break;
         const int g0 = sl * VB / S, g1 = (sl + 1) * VB / S;
@@ -340,8 +376,22 @@ struct Resident {
       rsum[b * RES_RED + v] = finish(s, v, proj);
     }
     if (MODE != RES_GRIDX) nbar++;
+    if (DEN && want_F) {
+      const float2* x = N.x + (size_t)xpar * N.ld;
+      if (DEN == RES_F32)
+        mv_f32().run(x, [&](int, int row, float Fc, float Fs, float2) { Fr[row - r0] = make_float2(Fc, Fs); });
+      else
+        mv_i8().run(x, [&](int row, float Fc, float Fs, float2) { Fr[row - r0] = make_float2(Fc, Fs); });
+    }
+    if (DEN) xpar ^= 1;
     __syncthreads();
     return true;
+  }
+  __device__ __forceinline__ MatvecF32<1, RES_CTF> mv_f32() const {
+    return {N.adj, N.split.ld, r0, r0 + nr, 1, reinterpret_cast<float2*>(xt), ring, tid, NT, lane, warp, NW};
+  }
+  __device__ __forceinline__ MatvecI8 mv_i8() const {
+    return {N.adj8, N.invn, N.split.ld, r0, r0 + nr, xt, reinterpret_cast<uint4*>(ring), tid, NT, lane, warp, NW};
   }
   // s + p[0] + p[stride] + .. of n <= 16 values, in that order
   template <bool L2 = false>
@@ -513,11 +563,11 @@ struct Resident {
         ok[u] = r < end[u];
         rr[u] = ok[u] ? r : 0;  // an idle lane reads row 0 and stores nothing
         P[u] = P0 + rr[u];
-        bits[u] = ub[rr[u]];
+        bits[u] = DEN ? 0u : ub[rr[u]];
         gn[u] = gs[u] = omr[u] = 0.f;
         y[u] = make_float2(0.f, 0.f);
         if (SLOPE) {
-          const float2 F = tb[bits[u]], x = xs[P[u]];
+          const float2 F = DEN ? Fr[rr[u]] : tb[bits[u]], x = xs[P[u]];
           gn[u] = c1b * (x.y * F.x - x.x * F.y);
         }
         if (ARG) {
@@ -593,9 +643,10 @@ struct Resident {
         }
         if (ARG && ok[u]) {
           xs[P[u]] = make_float2(cs[u], sn[u]);
+          if (DEN) N.x[(size_t)xpar * N.ld + r0 + rr[u]] = make_float2(cs[u], sn[u]);
           sx[a] += cs[u];
           sy[a] += sn[u];
-          if (KIND != 9 || N.dense_level >= 2) {
+          if (!DEN && (KIND != 9 || N.dense_level >= 2)) {
             // sums over the rows with u_mn = +1 (the factor bits from k on are zero)
 #pragma unroll
             for (int m = 0; m < 4; ++m)
@@ -630,7 +681,8 @@ struct Resident {
   // instruction caches do not hold (a stage of a small network took twice as long); with one body
   // for all kinds its loads no longer run ahead of the arithmetic (1.4 times as long at 5 x 200000).
   __device__ __forceinline__ void pass(const int kind) {
-    const bool full = kind != 1 && kind != 8 && (kind != 9 || N.dense_level >= 2);  // with projections
+    const bool full = !DEN && kind != 1 && kind != 8 && (kind != 9 || N.dense_level >= 2);  // with projections
+    const bool flush = kind != 1 && (!DEN || kind >= 8 || (kind == 0 && rec0));
     const int pairs = EX ? (nu + U - 1) / U : 0;  // EX: a warp takes U units at a time
     int e = 0;
 #pragma unroll 1
@@ -680,16 +732,18 @@ struct Resident {
         case 8: rows<8>(b, base, end, step, todo, acc, sx, sy); break;
         default: rows<9>(b, base, end, step, todo, acc, sx, sy); break;
       }
-      if (kind == 1) continue;
+      if (!flush) continue;
       float* dst = red + (EX ? b * nu + q0 : warp * 2 + e) * RES_RED;
       e = 1;
       __syncwarp();
       // sum_n u_mn x_n = 2 (sum over u_mn = +1) - sum_n x_n on every lane, where it costs no digits
       // (of a CTA's totals it did: the error norm of a small step came out three times too large)
+      if (full) {
 #pragma unroll
-      for (int a = 0; a < NA; ++a)
+        for (int a = 0; a < NA; ++a)
 #pragma unroll
-        for (int j = 0; j < 16; ++j) acc[a][j] = 2.f * acc[a][j] - ((j & 1) ? sy[a] : sx[a]);
+          for (int j = 0; j < 16; ++j) acc[a][j] = 2.f * acc[a][j] - ((j & 1) ? sy[a] : sx[a]);
+      }
       if (!full || k == 8) {  // the plain sums, or the error, alone
 #pragma unroll
         for (int a = 0; a < NA; ++a) {
@@ -744,6 +798,7 @@ struct Resident {
     }
     __syncthreads();
   }
+  // (read from L2: an acquire at every barrier empties L1, so the controller compares with te first)
   __device__ __forceinline__ double eval_time(int i) const {
     return N.t_eval ? (double)N.t_eval[i] : (double)(N.dtf * (float)(i + 1));
   }
@@ -787,7 +842,8 @@ struct Resident {
       T.accepted++;
       if (!N.fixed) T.h = h * fmin(factor, 10.0);
       int e = T.eval_i;
-      while (e < N.n_eval && T.t >= eval_time(e)) e++;
+      if (T.t >= te[b])
+        while (e < N.n_eval && T.t >= eval_time(e)) e++;
       T.eval_end = e;
       if (N.log_cap > 0 && gi == 0) {
         N.log_t[(size_t)b * N.log_cap + T.log_count] = T.t;
@@ -813,7 +869,7 @@ struct Resident {
     for (int b = 0; b < B; ++b) {
       if (!((act >> b) & 1) || ps[b * 4 + 2] < 0) continue;
       float2* dst = reinterpret_cast<float2*>(N.out_coup + ((size_t)b * N.ring + ps[b * 4 + 2]) * 2 * N.out_ld) + r0;
-      for (int r = tid; r < nr; r += NT) dst[r] = tab[(b << k) + ub[r]];
+      for (int r = tid; r < nr; r += NT) dst[r] = DEN ? Fr[r] : tab[(b << k) + ub[r]];
     }
   }
 
@@ -826,10 +882,12 @@ struct Resident {
   __device__ bool run(bool fresh_theta, const float* theta0) {
     for (int r = tid; r < nr; r += NT) {
       const int i = r0 + r;
-      uint32_t w = 0;
-      for (int m = 0; m < k; ++m)
-        w |= (stream_word(N.seed, (unsigned long long)m * (unsigned long long)N.n + (unsigned long long)i) & 1u) << m;
-      ub[r] = (uint8_t)w;
+      if (!DEN) {
+        uint32_t w = 0;
+        for (int m = 0; m < k; ++m)
+          w |= (stream_word(N.seed, (unsigned long long)m * (unsigned long long)N.n + (unsigned long long)i) & 1u) << m;
+        ub[r] = (uint8_t)w;
+      }
       om[r] = N.omega[i];
     }
     if (tid < B) {
@@ -864,6 +922,7 @@ struct Resident {
     }
     __syncthreads();
 
+    if (tid < B) te[tid] = tr[tid].eval_i < N.n_eval ? eval_time(tr[tid].eval_i) : INFINITY;
     // first slope (dp45.cu:151) and the record at t0 (kuramoto.cu:587-626)
     act = 0;
     bool want_r = false;
@@ -874,6 +933,7 @@ struct Resident {
         want_r |= T.need_init && T.out_count < N.ring;
       }
     }
+    rec0 = want_r;
     const bool coup = N.dense_level >= 2;
     const int np1 = max(2 * k, 1);
     long long attempts = 0;
@@ -894,6 +954,11 @@ struct Resident {
       pass(kind);
       if (kind == 1 || (kind == 8 && N.fixed)) {
         __syncthreads();
+      } else if (DEN) {
+        const bool sums = kind >= 8 || (kind == 0 && want_r);
+        if (!exchange_blocks(2 * RES_KMAX, !sums ? 0 : kind == 8 ? 1 : 2, false, kind == 8 ? 1 : 2,
+                             kind < 8 || (kind == 9 && coup)))
+          return false;
       } else {
         const bool st = kind >= 2 && kind <= 7, all = kind == 0 || (kind == 9 && coup);
         if (!exchange(st || all ? 0 : 2 * RES_KMAX, st ? np1 : all ? RES_RED : kind == 8 ? 1 : 2, st || all,
@@ -920,7 +985,8 @@ struct Resident {
         if (coup) record_couplings();
         __syncthreads();
         if (mine) {
-          tr[tid].eval_i++;
+          const int i = ++tr[tid].eval_i;
+          te[tid] = i < N.n_eval ? eval_time(i) : INFINITY;
           tr[tid].out_count++;
           ps[tid * 4 + 2] = -1;
         }

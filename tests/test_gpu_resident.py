@@ -134,3 +134,51 @@ def test_cut_into_launches_gives_the_same_bits(native, n, k, batch):
     for x, y in zip(sorted(a[3], key=key), sorted(c[3], key=key)):
         assert x[:3] == y[:3] and np.array_equal(x[3], y[3])
         assert level < 2 or np.array_equal(x[4], y[4])
+
+
+# ------------------------------------------------------------------ stored adjacency, one trajectory
+def dense_run(native, n, k, th, om, c, t1, dt, storage, batch=1, level=2, attempts=0):
+    net = native.Network(n, k=k, coupling=0, batch=batch, seed=7, dense_level=level, adj_storage=storage,
+                         engine=native.ENGINE_PERSISTENT)
+    net.set_frequencies(om)
+    net.generate_adjacency()
+    for b in range(batch):
+        net.set_coupling(b, c)
+        net.set_state(b, th, 0.0, dt / 100)
+    net.set_horizon(t1, dt, True)
+    if attempts:
+        net.set_launch_attempts(attempts)
+    rec = []
+    net.run(on_output=lambda b, i, t, r, theta, cp: rec.append((i, r, theta, cp)) and False if b == 0 else False)
+    out = rec, net.state(0)[0], net.stats()
+    net.close()
+    return out
+
+
+# one row per CTA, rows that leave warps idle, two and three rows of a warp, one and two x tiles
+@pytest.mark.parametrize("n", [1, 31, 100, 997, 5000, 7169, 8300])
+def test_dense_same_bits_as_the_persistent_kernel(native, n):
+    """The persistent kernel, which takes a batch of two, adds a row's product and a CTA's sums in the
+    same order."""
+    th, om = cauchy_inputs(n, 3 + n)
+    a, ta, _ = dense_run(native, n, 5, th, om, 2.0, 0.25, 0.0625, native.ADJ_F32)
+    b, tb, _ = dense_run(native, n, 5, th, om, 2.0, 0.25, 0.0625, native.ADJ_F32, batch=2)
+    assert len(a) == len(b) == 5 and np.array_equal(ta, tb)
+    for x, y in zip(a, b):
+        assert x[:2] == y[:2] and np.array_equal(x[2], y[2]) and np.array_equal(x[3], y[3])
+
+
+@pytest.mark.parametrize("storage", ["ADJ_F32", "ADJ_I8"])
+@pytest.mark.parametrize("n", [1, 33, 700, 4100, 7300])
+def test_dense_runs_match_fp64_and_cut_runs_their_bits(native, oracle_lib, n, storage):
+    th, om = normal_inputs(n, 12, init=np.pi)
+    rec, end, st = dense_run(native, n, 6, th, om, 1.5, 2.0, 0.25, getattr(native, storage))
+    cut, cend, cst = dense_run(native, n, 6, th, om, 1.5, 2.0, 0.25, getattr(native, storage), attempts=3)
+    assert st["launches"] == 1 and cst["launches"] > 1 and np.array_equal(end, cend)
+    ref = oracle_lib.run(th, om, k=6, c1=1.5, onthefly=True, seed=7, fp64=True, t1=2.0, dt=0.25, dense=2)
+    assert len(rec) == len(cut) == 9
+    for q, (x, y) in enumerate(zip(rec, cut)):
+        assert x[:2] == y[:2] and np.array_equal(x[2], y[2]) and np.array_equal(x[3], y[3])
+        assert abs(x[1] - ref.order[q]) < 1e-5
+        assert np.max(np.abs(x[2] - ref.thetas[q])) < 1e-4
+        assert np.max(np.abs(x[3] - np.asarray(ref.couplings[q]).reshape(-1))) < 1e-4
