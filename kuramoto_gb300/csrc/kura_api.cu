@@ -48,6 +48,7 @@ struct kura_handle {
   long long* ph_w = nullptr;
   float* g = nullptr;
   float2* xbuf = nullptr;
+  int8_t* xdig = nullptr;  // digits of (cos, sin) for the int8 product on the integer tensor pipe
   float* part = nullptr;
   unsigned long long* fix = nullptr;
   unsigned* bar = nullptr;
@@ -170,7 +171,7 @@ extern "C" int kura_memory_required(const kura_config* c, int64_t* bytes) {
 extern "C" void kura_destroy(kura_handle* h) {
   if (!h) return;
   cudaSetDevice(h->cfg.device);
-  void* ptrs[] = {h->omega, h->adj, h->adj8, h->ph_hi, h->ph_lo, h->ph_w, h->g, h->xbuf, h->part, h->fix, h->bar, h->err,
+  void* ptrs[] = {h->omega, h->adj, h->adj8, h->ph_hi, h->ph_lo, h->ph_w, h->g, h->xbuf, h->xdig, h->part, h->fix, h->bar, h->err,
                   h->traj, h->t_eval, h->out_r, h->out_idx, h->out_theta, h->out_coup, h->log_t, h->log_h,
                   h->fin_theta, h->fin_coup, h->counters};
   for (void* p : ptrs)
@@ -270,8 +271,8 @@ extern "C" int kura_create(const kura_config* cfg, kura_handle** out) {
   if (h->coupling == KURA_COUPLING_VOLCANO)
     h->res = kura::resident_plan(h->n, h->B, h->K, G, rows);
   else if (h->B == 1)
-    h->res = uses_i8(cfg) ? kura::resident_plan_dense(kura::RES_I8, (h->n + 15) / 16 * 16, G, rows)
-                          : kura::resident_plan_dense(kura::RES_F32, h->ld, G, rows);
+    h->res = uses_i8(cfg) ? kura::resident_plan_dense(kura::RES_I8, h->n, (h->n + 15) / 16 * 16, G, rows)
+                          : kura::resident_plan_dense(kura::RES_F32, h->n, h->ld, G, rows);
 
   size_t ld = h->ld, B = h->B;
   CUH(dalloc(&h->omega, ld));
@@ -286,6 +287,7 @@ extern "C" int kura_create(const kura_config* cfg, kura_handle** out) {
   CUH(dalloc(&h->ph_w, 2 * B * ld));
   CUH(dalloc(&h->g, 7 * B * ld));
   CUH(dalloc(&h->xbuf, 2 * B * ld));
+  if (h->res.split.den == kura::RES_IMMA) CUH(dalloc(&h->xdig, 16 * ld));
   CUH(dalloc(&h->part, 2 * (size_t)G * B * kura::PW_MAX));
   if (h->res.mode == kura::RES_MODE_FIXED) CUH(dalloc(&h->fix, 3 * B * 16));
   CUH(dalloc(&h->bar, 4));
@@ -600,6 +602,7 @@ static int launch_begin(kura_handle* h, int mode, bool log_steps) {
   p.xs_smem = h->xs_smem;
   p.counters = h->counters;
   p.adj8 = h->adj8;
+  p.xdig = h->xdig;
   p.ld8 = h->ld8;
   p.invn = 1.0f / (float)h->n;
   std::memcpy(h->traj_pin, h->htraj.data(), sizeof(TrajG) * h->B);

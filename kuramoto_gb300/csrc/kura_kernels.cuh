@@ -72,6 +72,7 @@ struct KParams {
   const int8_t* adj8;  // [n][ld8] N*A as int8 (dense coupling stored as integers), or null
   int ld8;             // row stride of adj8 (a multiple of 16)
   float invn;          // 1/N in float, the scale of adj8
+  int8_t* xdig;        // [2][8][ld] base-256 digits of (cos, sin) (RES_IMMA)
 };
 
 // kernel selector for a dense adjacency stored as the integers N*A (int8); the public
@@ -98,7 +99,7 @@ struct ResSplit {
   int B, k, rows, vrows, vblocks, ctas;  // rows: the most a CTA holds
   int den, ld;  // stored adjacency: RES_F32 or RES_I8 with rows of ld values; 0: regenerated coupling
 };
-enum { RES_F32 = 1, RES_I8 = 2 };
+enum { RES_F32 = 1, RES_I8 = 2, RES_IMMA = 3 };  // RES_IMMA: int8 on the integer tensor pipe
 constexpr int RES_MODE_FIXED = 2;  // the form that needs KParams::fix
 struct ResPlan {
   int mode = -1, hl = 0, grid = 0;
@@ -107,7 +108,7 @@ struct ResPlan {
 };
 // blocks, rows: the persistent kernel's grid for this network and its rows per CTA
 ResPlan resident_plan(int64_t n, int batch, int k, int blocks, int rows);
-ResPlan resident_plan_dense(int den, int ld, int blocks, int rows);
+ResPlan resident_plan_dense(int den, int64_t n, int ld, int blocks, int rows);
 cudaError_t launch_resident(const KParams& p, const ResPlan& r, cudaStream_t st);
 
 // sets the message returned by kura_last_error() for the calling thread

@@ -345,4 +345,158 @@ struct MatvecI8 {
   }
 };
 
+// ---------------------------------------------------------------- int8 on the integer tensor pipe
+// The int8 product of a large network as integers: x = X 2^-30 with X = round(x 2^30) in four signed
+// base-256 digits, so the 8 digits of (cos, sin) are the 8 columns of mma.m16n8k32.s8 and one
+// instruction multiplies 512 bytes of A.  The sums are exact (|sum| <= 127 128 n < 2^31 for
+// n <= 132000); the product's only errors are the 2^-31 of X and the final rounding.  The byte
+// conversions and packed FMAs of MatvecI8 cost 20 issue slots per 8 bytes and lane and held A at 4.1
+// to 5.1 TB/s (N = 40009, 65536); here 512 bytes take 16 clocks of an SM's integer pipe (measured) of
+// the 23 that HBM needs to deliver them, and A arrives at 5.6 / 6.0 / 6.8 TB/s at N = 16384 / 40009 /
+// 65536.
+//
+// Work: a pass holds up to 8 tiles of 16 rows; the warps split the columns, warp w takes the 64-column
+// chunks w, w + 16, .. and all rows of the pass, so that any number of rows keeps all warps busy and a
+// chunk of x is read once per pass.  K order: in a chunk, lane (g, t) = (lane / 4, lane % 4) holds
+// columns 16 t .. 16 t + 15 of rows g and g + 8 and of digit plane g, 16 bytes each; the words 0, 1 and
+// 2, 3 of A and x meet in one MMA each.  A streams through the warp's ring of IM_SLOTS units (one row
+// tile of a chunk, 32 bytes per lane), across chunks and x tiles; x arrives in two tiles of IM_TC
+// columns, one ahead.  The warps' sums meet in shared memory by integer atomics.
+constexpr int IM_TC = 4096;           // columns per x tile
+constexpr int IM_XS = IM_TC + 64;     // bytes per digit plane of a tile: a phase's two planes on distinct banks
+constexpr int IM_SLOTS = 8;           // units in a warp's ring
+constexpr int IM_MT = 8;              // row tiles per pass
+constexpr int IM_SMEM_X = 2 * 8 * IM_XS;
+constexpr int IM_SMEM_ACC = IM_MT * 16 * 8 * 4;
+
+// the four signed base-256 digits of round(x 2^30), lowest first, |x| <= 1
+__device__ __forceinline__ uint32_t x_digits(float x) {
+  const int X = __float2int_rn(x * 1073741824.f);
+  return ((uint32_t)X + 0x00808080u) ^ 0x00808080u;
+}
+
+struct MatvecImma {
+  const int8_t* adj8;
+  float invn;
+  int ld8, r0, r1;
+  int xld;     // bytes per digit plane of x
+  int8_t* xt;  // [2][8][IM_XS]
+  int* sums;   // [IM_MT * 16][8]
+  uint4* ring;
+  int tid, nt, lane, warp, nw;
+
+  // the digits of tile `t` of x into buffer t & 1
+  __device__ __forceinline__ void load_x(const int8_t* x, int t) const {
+    int8_t* dst = xt + (t & 1) * 8 * IM_XS;
+    const int c0 = t * IM_TC;
+    for (int i = tid; i < 8 * IM_TC / 16; i += nt) {
+      const int pl = i / (IM_TC / 16), c = i % (IM_TC / 16) * 16;
+      const bool in = c0 + c < xld;
+      cp_async16(dst + pl * IM_XS + c, x + (size_t)pl * xld + (in ? c0 + c : 0), in ? 16 : 0);
+    }
+  }
+  // rows row0 .. row0 + 16 MT: sums[row][digit]
+  template <int MT>
+  __device__ __forceinline__ void pass(const int8_t* x, int row0) const {
+    const int g = lane >> 2, t = lane & 3;
+    int acc[MT][4];
+#pragma unroll
+    for (int m = 0; m < MT; ++m) acc[m][0] = acc[m][1] = acc[m][2] = acc[m][3] = 0;
+    uint4* my = ring + (size_t)warp * (IM_SLOTS * 64) + lane;
+    const int nch = (ld8 + 63) / 64;  // chunks
+    const int mine = warp < nch ? (nch - warp + nw - 1) / nw : 0, units = mine * MT;
+    // unit u: chunk u / MT of this warp, row tile u % MT
+    int lc = 64 * warp + 16 * t, lm = 0, lu = 0;  // the next unit to load
+    auto load = [&]() {
+      if (lu < units) {
+        const int ra = row0 + 16 * lm + g, rb = ra + 8;
+        const bool in = lc < ld8;
+        uint4* s = my + (lu % IM_SLOTS) * 64;
+        cp_async16(s, adj8 + (size_t)(ra < r1 ? ra : r0) * ld8 + (in ? lc : 0), in && ra < r1 ? 16 : 0);
+        cp_async16(s + 32, adj8 + (size_t)(rb < r1 ? rb : r0) * ld8 + (in ? lc : 0), in && rb < r1 ? 16 : 0);
+        if (++lm == MT) {
+          lm = 0;
+          lc += 64 * nw;
+        }
+        ++lu;
+      }
+      cp_async_commit();
+    };
+    const int tiles = (ld8 + IM_TC - 1) / IM_TC;
+    load_x(x, 0);
+    cp_async_commit();
+#pragma unroll 1
+    for (int s = 0; s < IM_SLOTS - 1; ++s) load();
+    int u = 0;
+#pragma unroll 1
+    for (int tl = 0; tl < tiles; ++tl) {
+      // this tile of x has landed: the first was committed before the ring's units, a later one with
+      // the first unit of the tile before, IM_SLOTS units or more ago where that had so many
+      if (tl > 0 && MT * (IM_TC / 64 / 16) < IM_SLOTS) cp_async_wait<0>();
+      else cp_async_wait<IM_SLOTS - 1>();
+      __syncthreads();  // every thread's part of it, and the tile before is no longer read
+      if (tl + 1 < tiles) load_x(x, tl + 1);
+      const int8_t* xb = xt + (tl & 1) * 8 * IM_XS + g * IM_XS + 16 * t;
+      const int cend = min(nch, (tl + 1) * (IM_TC / 64));
+#pragma unroll 1
+      for (int c = warp + (u / MT) * nw; c < cend; c += nw) {
+        const uint4 b = *reinterpret_cast<const uint4*>(xb + (c * 64 - tl * IM_TC));
+#pragma unroll
+        for (int m = 0; m < MT; ++m, ++u) {
+          load();
+          cp_async_wait<IM_SLOTS - 1>();  // unit u has landed
+          const uint4* s = my + (u % IM_SLOTS) * 64;
+          const uint4 a = s[0], h = s[32];
+          asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                       : "+r"(acc[m][0]), "+r"(acc[m][1]), "+r"(acc[m][2]), "+r"(acc[m][3])
+                       : "r"(a.x), "r"(h.x), "r"(a.y), "r"(h.y), "r"(b.x), "r"(b.y));
+          asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                       : "+r"(acc[m][0]), "+r"(acc[m][1]), "+r"(acc[m][2]), "+r"(acc[m][3])
+                       : "r"(a.z), "r"(h.z), "r"(a.w), "r"(h.w), "r"(b.z), "r"(b.w));
+        }
+      }
+    }
+    cp_async_wait<0>();
+#pragma unroll
+    for (int m = 0; m < MT; ++m) {
+      int* d = sums + (16 * m + g) * 8 + 2 * t;
+      atomicAdd(d, acc[m][0]);
+      atomicAdd(d + 1, acc[m][1]);
+      atomicAdd(d + 64, acc[m][2]);
+      atomicAdd(d + 65, acc[m][3]);
+    }
+  }
+  // x: [8][xld] digit planes.  done(row, Fc, Fs) is called by one thread for each row.
+  template <class Done>
+  __device__ __forceinline__ void run(const int8_t* x, Done done) const {
+    int left = (r1 - r0 + 15) / 16;
+    for (int row0 = r0; left > 0;) {
+      const int passes = (left + IM_MT - 1) / IM_MT, mt = (left + passes - 1) / passes;  // passes of even height
+      for (int i = tid; i < mt * 16 * 8; i += nt) sums[i] = 0;
+      __syncthreads();
+      switch (mt) {
+        case 1: pass<1>(x, row0); break;
+        case 2: pass<2>(x, row0); break;
+        case 3: pass<3>(x, row0); break;
+        case 4: pass<4>(x, row0); break;
+        case 5: pass<5>(x, row0); break;
+        case 6: pass<6>(x, row0); break;
+        case 7: pass<7>(x, row0); break;
+        default: pass<8>(x, row0); break;
+      }
+      __syncthreads();
+      for (int r = tid; r < mt * 16 && row0 + r < r1; r += nt) {
+        const int* d = sums + r * 8;
+        const long long c = 16777216ll * d[3] + 65536ll * d[2] + 256ll * d[1] + d[0];
+        const long long s = 16777216ll * d[7] + 65536ll * d[6] + 256ll * d[5] + d[4];
+        constexpr float S = 1.f / 1073741824.f;
+        done(row0 + r, __ll2float_rn(c) * S * invn, __ll2float_rn(s) * S * invn);
+      }
+      __syncthreads();  // before the sums and the x tiles are written again
+      row0 += 16 * mt;
+      left -= mt;
+    }
+  }
+};
+
 }  // namespace kura

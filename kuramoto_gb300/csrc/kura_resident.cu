@@ -29,7 +29,7 @@ __global__ void __launch_bounds__(threads_of(DEN), 1) k_resident(const KParams p
     net.out_ld = p.ld; net.ring = p.ring;
     net.log_t = p.log_t; net.log_h = p.log_h; net.log_cap = p.log_cap;
     net.max_attempts = p.max_attempts;
-    net.adj = p.adj; net.adj8 = p.adj8; net.invn = p.invn; net.x = p.xbuf;
+    net.adj = p.adj; net.adj8 = p.adj8; net.invn = p.invn; net.x = p.xbuf; net.xdig = p.xdig;
   }
   __syncthreads();
   Resident<MODE, HL, threads_of(DEN), DEN> e(net, smem, blockIdx.x, gridDim.x);
@@ -55,6 +55,7 @@ __global__ void __launch_bounds__(threads_of(DEN), 1) k_resident(const KParams p
 const void* pick(int mode, int hl, int den) {
   if (den == RES_F32) return (const void*)&k_resident<RES_GRIDX, true, RES_F32>;
   if (den == RES_I8) return (const void*)&k_resident<RES_GRIDX, true, RES_I8>;
+  if (den == RES_IMMA) return (const void*)&k_resident<RES_GRIDX, true, RES_IMMA>;
   if (mode == RES_ONE) return hl ? (const void*)&k_resident<RES_ONE, true> : nullptr;
   if (mode == RES_CLUSTER) return hl ? (const void*)&k_resident<RES_CLUSTER, true> : nullptr;
   if (mode == RES_GRIDX) return hl ? (const void*)&k_resident<RES_GRIDX, true> : nullptr;
@@ -143,8 +144,13 @@ ResPlan resident_plan(int64_t n, int B, int k, int blocks, int rows) {
 // One trajectory of a stored adjacency: wherever the state fits beside the x tile and the ring (N up
 // to about 80000 in float32, 70000 in int8) and a CTA has fewer than 1024 rows, from where on the
 // persistent kernel forms its sums in another order.
-ResPlan resident_plan_dense(int den, int ld, int blocks, int rows) {
+// int8: the integer product from 12000 oscillators on (FIXED_N above; it adds in another order than
+// the float one): us per attempt at N = 16384 377 -> 286, 40009 2347 -> 1607, 65536 4992 -> 3800.
+ResPlan resident_plan_dense(int den, int64_t n, int ld, int blocks, int rows) {
   ResPlan r;
+  if (den == RES_I8 && n >= FIXED_N && n <= 131072) {
+    if (rows < 1024 && shape(&r, 1, 0, blocks, rows, RES_GRIDX, blocks, 1, RES_IMMA, ld)) return r;
+  }
   if (rows < 1024 && shape(&r, 1, 0, blocks, rows, RES_GRIDX, blocks, 1, den, ld)) return r;
   return ResPlan();
 }

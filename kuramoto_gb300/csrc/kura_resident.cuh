@@ -76,6 +76,7 @@ struct ResNet {
   const int8_t* adj8;
   float invn;
   float2* x;  // [2][ld] (cos, sin) of all rows, by parity of the exchange
+  int8_t* xdig;  // [2][8][ld] their digits (RES_IMMA)
 };
 constexpr int RES_CTF = 7168;  // columns per x tile of the float product: leaves room for the state at N = 65536
 
@@ -118,9 +119,11 @@ __host__ __device__ inline size_t res_layout(const ResSplit& s, int hl, int mode
     const int warps = nt / 32, cf = s.ld < RES_CTF ? s.ld : RES_CTF, ci = s.ld < CT_I8 ? s.ld : CT_I8;
     take(s.rows * 8);                                                                    // 15 couplings
     o = (o + 127) & ~127;  // copies into the ring are faster from a line boundary (1.2x at N = 65536)
-    take(s.den == RES_F32 ? (cf + 3) / 4 * F_CHUNK * 8 : (ci + 15) / 16 * I8_CHUNK4 * 16);  // 16 x tile
+    take(s.den == RES_F32    ? (cf + 3) / 4 * F_CHUNK * 8
+         : s.den == RES_IMMA ? IM_SMEM_X + IM_SMEM_ACC
+                             : (ci + 15) / 16 * I8_CHUNK4 * 16);  // 16 x tile
     o = (o + 127) & ~127;
-    take(warps * 32 * 16 * (s.den == RES_F32 ? A_STAGES * A_ROWS : I8_SLOTS));             // 17 ring of A
+    take(warps * 32 * 16 * (s.den == RES_F32 ? A_STAGES * A_ROWS : s.den == RES_IMMA ? 2 * IM_SLOTS : I8_SLOTS));             // 17 ring of A
   }
   return (size_t)o;
 }
@@ -380,6 +383,9 @@ struct Resident {
       const float2* x = N.x + (size_t)xpar * N.ld;
       if (DEN == RES_F32)
         mv_f32().run(x, [&](int, int row, float Fc, float Fs, float2) { Fr[row - r0] = make_float2(Fc, Fs); });
+      else if (DEN == RES_IMMA)
+        mv_imma().run(N.xdig + (size_t)xpar * 8 * N.ld,
+                      [&](int row, float Fc, float Fs) { Fr[row - r0] = make_float2(Fc, Fs); });
       else
         mv_i8().run(x, [&](int row, float Fc, float Fs, float2) { Fr[row - r0] = make_float2(Fc, Fs); });
     }
@@ -389,6 +395,11 @@ struct Resident {
   }
   __device__ __forceinline__ MatvecF32<1, RES_CTF> mv_f32() const {
     return {N.adj, N.split.ld, r0, r0 + nr, 1, reinterpret_cast<float2*>(xt), ring, tid, NT, lane, warp, NW};
+  }
+  __device__ __forceinline__ MatvecImma mv_imma() const {
+    int8_t* t = reinterpret_cast<int8_t*>(xt);
+    return {N.adj8, N.invn, N.split.ld, r0, r0 + nr, (int)N.ld, t, reinterpret_cast<int*>(t + IM_SMEM_X),
+            reinterpret_cast<uint4*>(ring), tid, NT, lane, warp, NW};
   }
   __device__ __forceinline__ MatvecI8 mv_i8() const {
     return {N.adj8, N.invn, N.split.ld, r0, r0 + nr, xt, reinterpret_cast<uint4*>(ring), tid, NT, lane, warp, NW};
@@ -643,7 +654,17 @@ struct Resident {
         }
         if (ARG && ok[u]) {
           xs[P[u]] = make_float2(cs[u], sn[u]);
-          if (DEN) N.x[(size_t)xpar * N.ld + r0 + rr[u]] = make_float2(cs[u], sn[u]);
+          if (DEN == RES_IMMA) {
+            int8_t* xd = N.xdig + (size_t)xpar * 8 * N.ld + r0 + rr[u];
+            const uint32_t dc = x_digits(cs[u]), ds = x_digits(sn[u]);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              xd[j * N.ld] = (int8_t)(dc >> (8 * j));
+              xd[(4 + j) * N.ld] = (int8_t)(ds >> (8 * j));
+            }
+          } else if (DEN) {
+            N.x[(size_t)xpar * N.ld + r0 + rr[u]] = make_float2(cs[u], sn[u]);
+          }
           sx[a] += cs[u];
           sy[a] += sn[u];
           if (!DEN && (KIND != 9 || N.dense_level >= 2)) {

@@ -182,3 +182,20 @@ def test_dense_runs_match_fp64_and_cut_runs_their_bits(native, oracle_lib, n, st
         assert abs(x[1] - ref.order[q]) < 1e-5
         assert np.max(np.abs(x[2] - ref.thetas[q])) < 1e-4
         assert np.max(np.abs(x[3] - np.asarray(ref.couplings[q]).reshape(-1))) < 1e-4
+
+
+# the integer product: one to eight row tiles per pass, two passes, rows and columns that end inside a
+# tile, ranks whose entries reach the ends of int8
+@pytest.mark.parametrize("n,k", [(12000, 5), (12001, 127), (16400, 6), (20011, 64), (30002, 3)])
+def test_integer_product_matches_fp64(native, oracle_lib, n, k):
+    th, om = normal_inputs(n, 9, init=np.pi)
+    rec, end, st = dense_run(native, n, k, th, om, 1.5, 0.5, 0.25, native.ADJ_I8)
+    cut, cend, _ = dense_run(native, n, k, th, om, 1.5, 0.5, 0.25, native.ADJ_I8, attempts=2)
+    ref = oracle_lib.run(th, om, k=k, c1=1.5, onthefly=True, seed=7, fp64=True, t1=0.5, dt=0.25, dense=2)
+    assert len(rec) == 3 and np.array_equal(end, cend)
+    scale = np.max(np.abs(ref.couplings))
+    for q, (x, y) in enumerate(zip(rec, cut)):
+        assert x[:2] == y[:2] and np.array_equal(x[2], y[2]) and np.array_equal(x[3], y[3])
+        assert abs(x[1] - ref.order[q]) < 1e-6
+        # (cos, sin) in FP32 are 1e-7 off, at random; the sums of their digits are exact
+        assert np.max(np.abs(x[3] - np.asarray(ref.couplings[q]).reshape(-1))) < 3e-6 * scale + 1e-6
