@@ -173,45 +173,97 @@ __global__ void k_t_coef_final(TrajG* traj, TCoef* src, int B, const float* t_ev
 }
 
 // ---------------------------------------------------------------- stage (elementwise)
-// theta = phase[base] + omega*(m_hi+m_lo) + sum_j W_j g_j for (trajectory b, oscillator i);
-// writes the F16 hi/lo operand columns (cos, sin) and the FP32 (cos, sin) for the epilogue
-__global__ void k_t_stage(TView v, const TCoef* src) {
+// theta = phase[base] + omega*(m_hi+m_lo) + sum_j W_j g_j for trajectory b and four oscillators
+// i .. i + 3; writes the F16 hi/lo operand columns (cos, sin) and the FP32 (cos, sin) for the
+// epilogue.  A thread takes four oscillators because the kernel is bound by the bytes it has in
+// flight: one at a time moved 336 MB at N = 65536, B = 128 in 99 us, four in about 62.  The last
+// group may reach into the padding (np is a multiple of 256), whose state stays finite and meets
+// zero columns of A.
+constexpr int ST_THREADS = 128;
+__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
+  *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
+}
+// A kernel that the previous one's launch may overlap: what it reads and writes of the previous
+// one's data comes after pdl_wait(), which returns when that one has completed.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+__global__ void __launch_bounds__(ST_THREADS) k_t_stage(TView v, const TCoef* src) {
+  pdl_launch();
+  pdl_wait();
   const int b = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (blockIdx.x * ST_THREADS + threadIdx.x) * 4;
   const TCoef& s = src[b];
   if (!s.active || i >= v.n) return;
-  const size_t boff = ((size_t)s.base * v.bp + b) * v.np;
-  const float om = v.omega[i];
-  float gsum = 0.f;
-  for (int j = 0; j < s.nW; ++j) gsum = __fmaf_rn(s.W[j], v.g[((size_t)s.slot[j] * v.bp + b) * v.np + i], gsum);
-  const f2 pr = two_prod(om, s.m_hi);
-  const f2 s1 = two_sum(v.ph_hi[boff + i], pr.hi);
-  const f2 s2 = two_sum(s1.hi, gsum);
-  const float lo = v.ph_lo[boff + i] + ((s1.lo + s2.lo) + __fmaf_rn(om, s.m_lo, pr.lo));
-  float sn, cs;
-  sincos_pair(s2.hi, lo, &sn, &cs);
-  v.x32[(size_t)b * v.np + i] = make_float2(cs, sn);
-  const __half ch = __float2half_rn(rintf(cs * X_STEPS) * (1.f / X_STEPS));
-  const __half sh = __float2half_rn(rintf(sn * X_STEPS) * (1.f / X_STEPS));
-  const __half cl = __float2half_rn(cs - __half2float(ch));
-  const __half sl = __float2half_rn(sn - __half2float(sh));
-  v.X[xrow(0, b, v.bp) * v.np + i] = ch;
-  v.X[xrow(1, b, v.bp) * v.np + i] = sh;
-  v.X[xrow(2, b, v.bp) * v.np + i] = cl;
-  v.X[xrow(3, b, v.bp) * v.np + i] = sl;
+  const size_t boff = ((size_t)s.base * v.bp + b) * v.np + i;
+  const float4 om4 = ld4(v.omega + i), hi4 = ld4(v.ph_hi + boff), lo4 = ld4(v.ph_lo + boff);
+  float4 gk[6];
+#pragma unroll
+  for (int j = 0; j < 6; ++j) {
+    gk[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (j < s.nW) gk[j] = ld4(v.g + ((size_t)s.slot[j] * v.bp + b) * v.np + i);
+  }
+  float gs[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+  for (int j = 0; j < 6; ++j)
+    if (j < s.nW) {
+      gs[0] = __fmaf_rn(s.W[j], gk[j].x, gs[0]);
+      gs[1] = __fmaf_rn(s.W[j], gk[j].y, gs[1]);
+      gs[2] = __fmaf_rn(s.W[j], gk[j].z, gs[2]);
+      gs[3] = __fmaf_rn(s.W[j], gk[j].w, gs[3]);
+    }
+  if (s.nW > 6) {  // the end-of-run record uses all seven
+    const float4 g6 = ld4(v.g + ((size_t)s.slot[6] * v.bp + b) * v.np + i);
+    gs[0] = __fmaf_rn(s.W[6], g6.x, gs[0]);
+    gs[1] = __fmaf_rn(s.W[6], g6.y, gs[1]);
+    gs[2] = __fmaf_rn(s.W[6], g6.z, gs[2]);
+    gs[3] = __fmaf_rn(s.W[6], g6.w, gs[3]);
+  }
+  const float om[4] = {om4.x, om4.y, om4.z, om4.w}, yh[4] = {hi4.x, hi4.y, hi4.z, hi4.w}, yl[4] = {lo4.x, lo4.y, lo4.z, lo4.w};
+  float cs[4], sn[4], zh[4], zl[4];
+  __half ch[4], sh[4], cl[4], sl[4];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const f2 pr = two_prod(om[q], s.m_hi);
+    const f2 s1 = two_sum(yh[q], pr.hi);
+    const f2 s2 = two_sum(s1.hi, gs[q]);
+    zh[q] = s2.hi;
+    zl[q] = yl[q] + ((s1.lo + s2.lo) + __fmaf_rn(om[q], s.m_lo, pr.lo));
+    sincos_pair(zh[q], zl[q], &sn[q], &cs[q]);
+    ch[q] = __float2half_rn(rintf(cs[q] * X_STEPS) * (1.f / X_STEPS));
+    sh[q] = __float2half_rn(rintf(sn[q] * X_STEPS) * (1.f / X_STEPS));
+    cl[q] = __float2half_rn(cs[q] - __half2float(ch[q]));
+    sl[q] = __float2half_rn(sn[q] - __half2float(sh[q]));
+  }
+  float* x = reinterpret_cast<float*>(v.x32 + (size_t)b * v.np + i);
+  st4(x, cs[0], sn[0], cs[1], sn[1]);
+  st4(x + 4, cs[2], sn[2], cs[3], sn[3]);
+  auto put = [&](int q, const __half (&h)[4]) {
+    const __half2 a = __halves2half2(h[0], h[1]), c = __halves2half2(h[2], h[3]);
+    *reinterpret_cast<uint2*>(v.X + xrow(q, b, v.bp) * v.np + i) =
+        make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&c));
+  };
+  put(0, ch);
+  put(1, sh);
+  put(2, cl);
+  put(3, sl);
   if (s.store_y7 || s.rec) {
-    f2 y = two_sum(s2.hi, lo);
-    long long w = v.ph_w[boff + i];
-    if (s.store_y7) {
-      float hi7 = y.hi, lo7 = y.lo;
-      long long w7 = w;
-      wrap_phase(hi7, lo7, w7);
-      const size_t o = ((size_t)(s.base ^ 1) * v.bp + b) * v.np + i;
-      v.ph_hi[o] = hi7;
-      v.ph_lo[o] = lo7;
-      v.ph_w[o] = w7;
-    } else if (v.fin_theta) {
-      v.fin_theta[(size_t)b * v.np + i] = (float)((double)w * TWO_PI_D + (double)y.hi + (double)y.lo);
+    const size_t o = ((size_t)(s.base ^ 1) * v.bp + b) * v.np + i;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      f2 y = two_sum(zh[q], zl[q]);
+      long long w = v.ph_w[boff + q];
+      if (s.store_y7) {
+        float hi7 = y.hi, lo7 = y.lo;
+        long long w7 = w;
+        wrap_phase(hi7, lo7, w7);
+        v.ph_hi[o + q] = hi7;
+        v.ph_lo[o + q] = lo7;
+        v.ph_w[o + q] = w7;
+      } else if (v.fin_theta) {
+        v.fin_theta[(size_t)b * v.np + i + q] = (float)((double)w * TWO_PI_D + (double)y.hi + (double)y.lo);
+      }
     }
   }
 }
@@ -367,6 +419,8 @@ __global__ void k_t_error(TView v, const TCoef* src7, double atol, double rtol, 
                           int fixed, const float* t_eval, int n_eval, unsigned* cnt, int* flags) {
   __shared__ float sh[32];
   __shared__ float buf[T_MAXBLK];
+  pdl_launch();
+  pdl_wait();
   const int b = blockIdx.y;
   const TCoef& s = src7[b];
   if (b == 0 && blockIdx.x == 0 && threadIdx.x == 0) flags[1] = 0;
@@ -434,6 +488,8 @@ __global__ void k_t_output(TView v, TrajG* traj, const float* t_eval, float* par
                            int ring, TCoef* src, unsigned* cnt, int* flags, int first) {
   __shared__ float sh[32];
   __shared__ float buf[T_MAXBLK];
+  pdl_launch();
+  pdl_wait();
   const int b = blockIdx.y;
   TrajG& T = traj[b];
   const int ncross = min(T.eval_end - T.eval_i, T_MAXC);
@@ -616,6 +672,8 @@ struct TensorEngine::Impl {
   int ring = 0, n_eval = 0, nblk = 1;
   CUtensorMap tmA, tmAlo, tmX, tmXhi;
   bool has_lo = false, adj_set = false;
+  SplitShape shape;  // how the coupling GEMM runs, chosen at its first launch
+  bool shaped = false;
   cudaGraphExec_t graph = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // KURA_TIME_COUPLING=1: event nodes around the six coupling GEMMs of the attempt graph; the
@@ -812,6 +870,49 @@ int TensorEngine::set_horizon(const std::vector<float>& t_eval, int ring, std::v
   return KURA_OK;
 }
 
+// a launch that may overlap the end of the one before it (the kernel calls pdl_wait)
+template <class... P, class... A>
+static cudaError_t launch_pdl(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
+template <int NCOL, int MT>
+static int clusters_at_once(int s) {
+  auto k = k_split_gemm<NCOL, MT, SplitEpi>;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TSCfg<NCOL, MT>::SMEM) != cudaSuccess) return 0;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = s;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.gridDim = dim3((unsigned)s);
+  cfg.blockDim = dim3(TS_THREADS);
+  cfg.dynamicSmemBytes = TSCfg<NCOL, MT>::SMEM;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, (void*)k, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return n;
+}
+
 template <int NCOL, int MT>
 static cudaError_t launch_split(TensorEngine::Impl& I, const TView& v, const TCoef* src, int s, int ktiles, int nsplit,
                                 int xstride, const int* run_flag) {
@@ -820,20 +921,9 @@ static cudaError_t launch_split(TensorEngine::Impl& I, const TView& v, const TCo
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
   if (e != cudaSuccess) return e;
   const int tiles = (I.n + TG_BM - 1) / TG_BM;
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = s;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.gridDim = dim3((unsigned)((tiles + MT - 1) / MT * nsplit * s));
-  cfg.blockDim = dim3(TS_THREADS);
-  cfg.dynamicSmemBytes = C::SMEM;
-  cfg.stream = I.st;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, k, I.tmA, I.has_lo ? I.tmAlo : I.tmA, I.tmX, I.tmXhi, ktiles, s, nsplit, xstride,
-                            I.has_lo ? 1 : 0, SplitEpi{v, src}, I.err, 20000000000ull, run_flag);
+  return launch_pdl(k, dim3((unsigned)((tiles + MT - 1) / MT * nsplit * s)), TS_THREADS, C::SMEM, I.st, s, I.tmA,
+                    I.has_lo ? I.tmAlo : I.tmA, I.tmX, I.tmXhi, ktiles, s, nsplit, xstride, I.has_lo ? 1 : 0,
+                    SplitEpi{v, src}, I.err, 20000000000ull, run_flag);
 }
 
 template <int NCOL>
@@ -845,13 +935,11 @@ static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, I.device);
   const int mtiles = I.np / (2 * TG_BM), ktiles = I.np / TE_BK;  // groups of two row tiles
   const int nsplit = I.bp / BP, xstride = 4 * BP;
-  const SplitShape sh = split_shape((I.n + TG_BM - 1) / TG_BM, nsplit, NCOL, ktiles, sms);
-  if (sh.mt == 1) return launch_split<NCOL, 1>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag);
-  if (sh.mt == 2) return launch_split<NCOL, 2>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag);
   const int grid = std::min(mtiles * nsplit, sms);
   // Units of two row tiles fill whole waves of the grid; the rest run as one-tile units, when
   // that shortens the last wave (in unit times: a one-tile unit is half of a two-tile one)
   int big = mtiles;
+  double waves = 0;
   {
     const int full = (mtiles * nsplit) / grid;
     const int b = full * grid / nsplit;
@@ -859,7 +947,16 @@ static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode
     const double t_split = full + 0.5 * ((tail + grid - 1) / grid);
     const double t_big = (mtiles * nsplit + grid - 1) / grid;
     if (b < mtiles && t_split < t_big) big = b;
+    waves = std::min(t_split, t_big);
   }
+  if (!I.shaped) {
+    I.shape = split_shape((I.n + TG_BM - 1) / TG_BM, nsplit, NCOL, ktiles, waves,
+                          [&](int mt, int s) { return mt == 1 ? clusters_at_once<NCOL, 1>(s) : clusters_at_once<NCOL, 2>(s); });
+    I.shaped = true;
+  }
+  const SplitShape sh = I.shape;
+  if (sh.mt == 1) return launch_split<NCOL, 1>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag);
+  if (sh.mt == 2) return launch_split<NCOL, 2>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag);
   const unsigned long long limit = 20000000000ull;
   if (I.has_lo) {
     auto kl = k_tensor_gemm<NCOL / 2, LoEpi<BP>, 2, TE_BK>;
@@ -892,9 +989,8 @@ static cudaError_t coupling(TensorEngine::Impl& I, const TCoef* src, int mode, f
                             int timed = -1) {
   TView v{I.n, I.np, I.bp, I.B, mode, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, fin_theta, I.fin_coup,
           I.Flo, I.rinv};
-  dim3 grid((unsigned)((I.n + 255) / 256), (unsigned)I.B);
-  k_t_stage<<<grid, 256, 0, I.st>>>(v, src);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_pdl(k_t_stage, dim3((unsigned)((I.n + 4 * ST_THREADS - 1) / (4 * ST_THREADS)), (unsigned)I.B),
+                             ST_THREADS, 0, I.st, 1, v, src);
   if (e != cudaSuccess) return e;
   const bool tm = I.time_gemm && timed >= 0;
   if (tm && (e = cudaEventRecordWithFlags(I.gev[2 * timed], I.st, cudaEventRecordExternal)) != cudaSuccess) return e;
@@ -905,9 +1001,8 @@ static cudaError_t coupling(TensorEngine::Impl& I, const TCoef* src, int mode, f
 
 static cudaError_t output(TensorEngine::Impl& I, int first) {
   TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo, I.rinv};
-  k_t_output<<<dim3((unsigned)I.nblk, (unsigned)I.B), T_RBLK, 0, I.st>>>(v, I.traj, I.t_eval, I.part, I.nblk, I.out_r,
-                                                                       I.out_idx, I.ring, I.src, I.cnt, I.flags, first);
-  return cudaGetLastError();
+  return launch_pdl(k_t_output, dim3((unsigned)I.nblk, (unsigned)I.B), T_RBLK, 0, I.st, 1, v, I.traj, I.t_eval, I.part,
+                    I.nblk, I.out_r, I.out_idx, I.ring, I.src, I.cnt, I.flags, first);
 }
 
 // one attempt of every trajectory, its outputs, and the coefficients of the next
@@ -918,9 +1013,9 @@ static cudaError_t attempt(TensorEngine::Impl& I) {
     e = coupling(I, I.src + (size_t)(s - 1) * I.bp, 0, nullptr, I.flags + 1, s - 2);
     if (e != cudaSuccess) return e;
   }
-  k_t_error<<<dim3((unsigned)(I.fixed ? 1 : I.nblk), (unsigned)I.B), T_RBLK, 0, I.st>>>(
-      v, I.src + 6 * (size_t)I.bp, I.atol, I.rtol, I.part, I.nblk, I.traj, I.fixed, I.t_eval, I.n_eval, I.cnt, I.flags);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
+  e = launch_pdl(k_t_error, dim3((unsigned)(I.fixed ? 1 : I.nblk), (unsigned)I.B), T_RBLK, 0, I.st, 1, v,
+                 I.src + 6 * (size_t)I.bp, I.atol, I.rtol, I.part, I.nblk, I.traj, I.fixed, I.t_eval, I.n_eval, I.cnt, I.flags);
+  if (e != cudaSuccess) return e;
   return output(I, 0);
 }
 

@@ -7,8 +7,8 @@
 // CTAs of a cluster each accumulate K/S of the same unit in their own TMEM, leave the sums in
 // shared memory and finish 1/S of the unit's (row, trajectory) pairs each, adding the S parts in
 // rank order out of the peers' shared memory.  The A_lo pass of a general adjacency runs in the
-// same K loop and accumulates into the X_lo columns, whose small sums it joins.  Measured per launch (ncu): 52 -> 19 us at
-// n = 3000 with 24 trajectories (24 units x 6 CTAs), 159 -> 59 us at n = 6007 with 64 (24 x 6).
+// same K loop and accumulates into the X_lo columns, whose small sums it joins.  split_shape below
+// gives the measured times.
 //
 // Roles (256 threads): warp 0 lane 0 feeds the ring with TMA, warp 1 lane 0 issues the MMAs; then
 // all eight warps read TMEM (warp w owns lanes 32 (w % 4).., and half of the trajectories) and
@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
                  const int* run_flag) {
   using C = TSCfg<NCOL, MT>;
   constexpr int BP = C::BP;
-  if (run_flag && *run_flag == 0) return;  // nothing to compute: the same for every CTA of the cluster
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + C::STAGES * C::STAGE_BYTES);
@@ -87,6 +87,9 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
     umma::prefetch_tmap(&tmA);
     umma::prefetch_tmap(&tmX);
   }
+  // all that ran while the launch before this one (the stage kernel) was still going
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (run_flag && *run_flag == 0) return;  // nothing to compute: the same for every CTA of the cluster
   if (warp == 2) umma::tmem_alloc(tmem_slot, C::TMEM_COLS);  // warp 2 also frees it
   umma::tc_fence_before();
   __syncthreads();
@@ -196,12 +199,20 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
       const int b = sp * BP + bl;
       if (!epi.wants(b)) continue;
       const uint32_t ac = part_s + 4u * ((uint32_t)((mt * 2) * BP + bl) * TG_BM + rg * 4), as = ac + 4u * BP * TG_BM;
-      float4 c = ld_peer4(ac, 0), s4 = ld_peer4(as, 0);
-      for (int r = 1; r < S; ++r) {
-        const float4 c2 = ld_peer4(ac, r), s2 = ld_peer4(as, r);
-        c.x += c2.x; c.y += c2.y; c.z += c2.z; c.w += c2.w;
-        s4.x += s2.x; s4.y += s2.y; s4.z += s2.z; s4.w += s2.w;
-      }
+      float4 pc[TS_MAX_SPLIT], ps[TS_MAX_SPLIT];  // every peer's part is on its way before the first is added
+#pragma unroll
+      for (int r = 0; r < TS_MAX_SPLIT; ++r)
+        if (r < S) {
+          pc[r] = ld_peer4(ac, r);
+          ps[r] = ld_peer4(as, r);
+        }
+      float4 c = pc[0], s4 = ps[0];
+#pragma unroll
+      for (int r = 1; r < TS_MAX_SPLIT; ++r)
+        if (r < S) {
+          c.x += pc[r].x; c.y += pc[r].y; c.z += pc[r].z; c.w += pc[r].w;
+          s4.x += ps[r].x; s4.y += ps[r].y; s4.z += ps[r].z; s4.w += ps[r].w;
+        }
       epi.rows4((rt0 + mt) * TG_BM + rg * 4, b, c, s4);
     }
   if (*sabort && tid == 0 && err) atomicCAS(err, 0, -4);
@@ -221,23 +232,29 @@ struct SplitShape {
   int mt = 0, s = 0;  // mt = 0: the persistent kernel
 };
 // The shape with the shortest predicted time, in clocks, for `tiles` 128-row tiles, nsplit column
-// blocks of ncol columns and ktiles K tiles.  A K tile of a CTA costs the larger of its MMAs
-// (ncol 256: 142 clocks per 128 rows and 16 of K) and its operand bytes at the rate an SM draws
-// from L2 when all of them do (about 55 bytes a clock).  A cluster adds its launch, the fill of
-// the ring and the exchange of the sums.  From a full wave of two-tile units upwards (n about
-// 39000 at up to 64 trajectories) the persistent kernel is the better one: it overlaps the
-// fill of one unit with the MMAs of another, and its X tiles serve two row tiles.
-inline SplitShape split_shape(int tiles, int nsplit, int ncol, int ktiles, int sms) {
+// blocks of ncol columns and ktiles K tiles; fits(mt, s) is the number of clusters of s CTAs that run
+// at once (fewer than sms / s: a cluster stays inside a GPC, and one cluster too many is a second
+// wave).  A K tile of a CTA costs the larger of its MMAs (ncol 256: 142 clocks per 128 rows and 16 of
+// K) and its operand bytes at the rate an SM draws from L2 when all of them do (about 55 bytes a
+// clock).  A cluster adds its launch, the fill of the ring and the exchange of the sums.  The
+// persistent kernel takes `waves` times a two-tile unit and pays its fill once.  Measured per launch
+// (us), chosen against the persistent kernel: n = 1000 with 16 trajectories 10.4 (1 tile x 8) / 28.0;
+// 3000 x 24 14.5 (1 x 4) / 45.3; 6007 x 64 28.0 (1 x 3) / 117.7, general 43.6 / 200.0; 20000 x 128
+// 303 (2 x 4) / 467; 30000 x 20 292 (2 x 1) / 310; 65536 x 128 stays with the persistent kernel.
+template <class Fits>
+inline SplitShape split_shape(int tiles, int nsplit, int ncol, int ktiles, double waves0, Fits fits) {
   SplitShape best;
-  if (((tiles + 1) / 2) * nsplit >= sms) return best;
-  double tbest = 1e300;
+  const double mma2 = 8.0 * 142.0 * ncol / 256.0, load2 = (2 * 16384.0 + ncol * 128.0) / 55.0;
+  double tbest = waves0 * ktiles * (mma2 > load2 ? mma2 : load2) + 6000.0;
   for (int mt = 1; mt <= 2; ++mt) {
     if (mt * ncol > 512) continue;
     const int units = (tiles + mt - 1) / mt * nsplit;
     const double mma = 4.0 * mt * 142.0 * ncol / 256.0;
     const double load = (mt * 16384.0 + ncol * 128.0) / 55.0;
     for (int s = 1; s <= TS_MAX_SPLIT && s <= ktiles; ++s) {
-      const int waves = (units * s + sms - 1) / sms;
+      const int at_once = fits(mt, s);
+      if (at_once < 1) continue;
+      const int waves = (units + at_once - 1) / at_once;
       const double exchange = 1500.0 + (s > 1 ? 1500.0 + mt * 128.0 * (ncol / 4) * 8.0 / 40.0 : 0.0);
       const double t = waves * (((ktiles + s - 1) / s) * (mma > load ? mma : load) + 4000.0 + exchange);
       if (t < tbest) {
