@@ -119,6 +119,23 @@ struct MatvecF32 {
     }
     cp_async_wait<0>();
   }
+  // The same where the prologue has brought the whole of the rows (N up to 1408 with one row per warp):
+  // no copies and no waits, so that the reads of several steps overlap (340 clocks a step otherwise,
+  // most of it latency: 1.4 of the 5 us of a RHS at N = 997)
+  template <int NR>
+  __device__ __forceinline__ void landed(const float4* my, int nit, float (&acc)[RG][BMAX][2]) const {
+#pragma unroll 4
+    for (int it = 0; it < nit; ++it) {
+      const float4* xp = reinterpret_cast<const float4*>(xt + (lane + 32 * it) * F_CHUNK);
+      const float4 x01 = xp[0], x23 = xp[1];
+#pragma unroll
+      for (int q = 0; q < NR; ++q) {
+        const float4 a = my[(it * NR + q) * 32];
+        acc[q][0][0] += a.x * x01.x + a.y * x01.z + a.z * x23.x + a.w * x23.z;
+        acc[q][0][1] += a.x * x01.y + a.y * x01.w + a.z * x23.y + a.w * x23.w;
+      }
+    }
+  }
   // The product with x (the CTAs' (cos, sin) of trajectory b at x + b*ld), after first_chunks() and the
   // barrier.  done(b, row, Fc, Fs, own (cos, sin)) is called by one lane for each row and trajectory.
   template <class Done>
@@ -151,7 +168,10 @@ struct MatvecF32 {
         else if (nr == 2) cp_async_wait<A_STAGES * RG / 2 - 1>();
         else cp_async_wait<A_STAGES * RG - 1>();
         __syncthreads();  // every thread's part has
-        if (nr == 4) steps<4>(my, src, c0, nit, acc);
+        constexpr int ALL = A_STAGES * RG;  // ring slots: ALL / nr - 1 steps are on their way before a first tile
+        if (BMAX == 1 && first && nr == 1 && cw <= 128 * (ALL - 1)) landed<1>(my, nit, acc);
+        else if (BMAX == 1 && first && nr == 2 && cw <= 128 * (ALL / 2 - 1)) landed<2>(my, nit, acc);
+        else if (nr == 4) steps<4>(my, src, c0, nit, acc);
         else if (nr == 3) steps<3>(my, src, c0, nit, acc);
         else if (nr == 2) steps<2>(my, src, c0, nit, acc);
         else if (nr == 1) steps<1>(my, src, c0, nit, acc);
