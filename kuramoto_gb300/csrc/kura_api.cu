@@ -51,6 +51,7 @@ struct kura_handle {
   int8_t* xdig = nullptr;  // digits of (cos, sin) for the int8 product on the integer tensor pipe
   float* part = nullptr;
   unsigned long long* fix = nullptr;
+  char* ctl = nullptr;  // barrier counter, error flag and launch counters in one piece
   unsigned* bar = nullptr;
   int* err = nullptr;
   TrajG* traj = nullptr;
@@ -171,9 +172,9 @@ extern "C" int kura_memory_required(const kura_config* c, int64_t* bytes) {
 extern "C" void kura_destroy(kura_handle* h) {
   if (!h) return;
   cudaSetDevice(h->cfg.device);
-  void* ptrs[] = {h->omega, h->adj, h->adj8, h->ph_hi, h->ph_lo, h->ph_w, h->g, h->xbuf, h->xdig, h->part, h->fix, h->bar, h->err,
+  void* ptrs[] = {h->omega, h->adj, h->adj8, h->ph_hi, h->ph_lo, h->ph_w, h->g, h->xbuf, h->xdig, h->part, h->fix, h->ctl,
                   h->traj, h->t_eval, h->out_r, h->out_idx, h->out_theta, h->out_coup, h->log_t, h->log_h,
-                  h->fin_theta, h->fin_coup, h->counters};
+                  h->fin_theta, h->fin_coup};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (h->ev0) cudaEventDestroy(h->ev0);
@@ -290,17 +291,19 @@ extern "C" int kura_create(const kura_config* cfg, kura_handle** out) {
   if (h->res.split.den == kura::RES_IMMA) CUH(dalloc(&h->xdig, 16 * ld));
   CUH(dalloc(&h->part, 2 * (size_t)G * B * kura::PW_MAX));
   if (h->res.mode == kura::RES_MODE_FIXED) CUH(dalloc(&h->fix, 3 * B * 16));
-  CUH(dalloc(&h->bar, 4));
-  CUH(dalloc(&h->err, 4));
+  CUH(dalloc(&h->ctl, 256));
+  h->bar = (unsigned*)h->ctl;
+  h->err = (int*)(h->ctl + 128);             // apart from the barrier's line, which every CTA polls
+  h->counters = (long long*)(h->ctl + 136);  // read back with the error flag
   CUH(dalloc(&h->traj, B));
   CUH(dalloc(&h->fin_theta, B * ld));
   CUH(dalloc(&h->fin_coup, 2 * B * ld));
-  CUH(dalloc(&h->counters, 4));
   h->log_cap = 4096;
   CUH(dalloc(&h->log_t, B * (size_t)h->log_cap));
   CUH(dalloc(&h->log_h, B * (size_t)h->log_cap));
   CUH(cudaMallocHost((void**)&h->traj_pin, sizeof(TrajG) * B));
-  CUH(cudaMallocHost((void**)&h->err_h, sizeof(int)));
+  CUH(cudaMallocHost((void**)&h->err_h, 16));
+  std::memset(h->err_h, 0, 16);
   CUH(cudaEventCreateWithFlags(&h->ev_stage, cudaEventDisableTiming));
   h->htraj.assign(B, TrajG{});
   for (auto& T : h->htraj) {
@@ -433,7 +436,8 @@ extern "C" int kura_set_coupling(kura_handle* h, int32_t traj, float c) {
   return KURA_OK;
 }
 
-static int set_state_common(kura_handle* h, int traj, const float* dev_theta, double t, double step) {
+static int set_state_common(kura_handle* h, int traj, const float* dev_theta, double t, double step,
+                            const float* host_theta = nullptr) {
   if (!h->te) {
     size_t off = (size_t)traj * h->ld;  // physical buffer 0
     CU(kura::launch_init_state(dev_theta, h->n, h->ld, h->ph_hi + off, h->ph_lo + off, h->ph_w + off, h->stream));
@@ -453,7 +457,7 @@ static int set_state_common(kura_handle* h, int traj, const float* dev_theta, do
   T.need_init = 0;
   h->horizon_set = false;
   if (h->te) {
-    int rc = h->te->set_state(traj, dev_theta, T);
+    int rc = host_theta ? h->te->upload_state(traj, host_theta, T) : h->te->set_state(traj, dev_theta, T);
     if (rc) return fail(rc, kura::TensorEngine::last_error());
   }
   return KURA_OK;
@@ -465,7 +469,8 @@ extern "C" int kura_set_state(kura_handle* h, int32_t traj, const float* theta, 
   if (!theta) return fail(KURA_ERR_INVALID, "theta is NULL");
   if (!(step > 0)) return fail(KURA_ERR_INVALID, "step must be > 0");
   CU(cudaSetDevice(h->cfg.device));
-  float* tmp = h->te ? h->te->staging(traj) : h->fin_theta + (size_t)traj * h->ld;
+  if (h->te) return set_state_common(h, traj, nullptr, t, step, theta);
+  float* tmp = h->fin_theta + (size_t)traj * h->ld;
   CU(cudaMemcpyAsync(tmp, theta, sizeof(float) * h->n, cudaMemcpyHostToDevice, h->stream));
   return set_state_common(h, traj, tmp, t, step);
 }
@@ -607,8 +612,7 @@ static int launch_begin(kura_handle* h, int mode, bool log_steps) {
   p.invn = 1.0f / (float)h->n;
   std::memcpy(h->traj_pin, h->htraj.data(), sizeof(TrajG) * h->B);
   CU(cudaMemcpyAsync(h->traj, h->traj_pin, sizeof(TrajG) * h->B, cudaMemcpyHostToDevice, h->stream));
-  CU(cudaMemsetAsync(h->bar, 0, sizeof(unsigned), h->stream));
-  CU(cudaMemsetAsync(h->err, 0, sizeof(int), h->stream));
+  CU(cudaMemsetAsync(h->ctl, 0, 132, h->stream));  // barrier and error flag
   // the test hook of the barrier's time limit needs a launch that has a grid barrier
   const bool resident = mode == kura::MODE_INTEGRATE && h->res.mode >= 0 && p.bar_extra == 0;
   if (resident && h->fix)
@@ -619,7 +623,7 @@ static int launch_begin(kura_handle* h, int mode, bool log_steps) {
   else
     CU(kura::launch_persistent(p, h->grid, h->bmax, h->kmax, h->smem, h->stream));
   CU(cudaEventRecord(h->ev1, h->stream));
-  CU(cudaMemcpyAsync(h->err_h, h->err, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+  CU(cudaMemcpyAsync(h->err_h, h->err, 16, cudaMemcpyDeviceToHost, h->stream));
   CU(cudaMemcpyAsync(h->traj_pin, h->traj, sizeof(TrajG) * h->B, cudaMemcpyDeviceToHost, h->stream));
   return KURA_OK;
 }
@@ -651,19 +655,19 @@ extern "C" int kura_run(kura_handle* h, const kura_callbacks* cb) {
     if (rc) return fail(rc, kura::TensorEngine::last_error());
     long long acc = 0, rej = 0;
     int errc = 0;
-    std::vector<float> rbuf;
-    std::vector<int> ibuf;
+    std::vector<float> rall;
+    std::vector<int> iall;
+    int most = 0;
+    for (const auto& T : h->htraj) most = std::max(most, T.out_count);
+    rc = h->te->read_orders(most, rall, iall);
+    if (rc) return fail(rc, kura::TensorEngine::last_error());
     for (int b = 0; b < h->B; ++b) {
       TrajG& T = h->htraj[b];
       acc += T.accepted;
       rej += T.rejected;
       if (T.status < 0 && !errc) errc = T.status;
-      rbuf.resize(std::max(T.out_count, 1));
-      ibuf.resize(std::max(T.out_count, 1));
-      if (T.out_count > 0) {
-        rc = h->te->read_order(b, T.out_count, rbuf.data(), ibuf.data());
-        if (rc) return fail(rc, kura::TensorEngine::last_error());
-      }
+      const float* rbuf = rall.data() + (size_t)b * most;
+      const int* ibuf = iall.data() + (size_t)b * most;
       for (int q = 0; q < T.out_count; ++q) {
         h->order[b].push_back(rbuf[q]);
         if (cb && cb->on_output) {
@@ -840,7 +844,7 @@ extern "C" int kura_run(kura_handle* h, const kura_callbacks* cb) {
   }
   long long acc = 0, rej = 0, bars = 0;
   for (auto& T : h->htraj) { acc += T.accepted; rej += T.rejected; }
-  CU(cudaMemcpy(&bars, h->counters, sizeof(long long), cudaMemcpyDeviceToHost));
+  std::memcpy(&bars, (const char*)h->err_h + 8, sizeof bars);  // came back with the last launch
   h->stats.accepted = acc;
   h->stats.rejected = rej;
   h->stats.barriers = bars;

@@ -351,6 +351,7 @@ struct kura_mlp {
   bf16 *dZ[NL] = {}, *dZT[NL] = {};  // gradient at the output of layer l
   float *Tb = nullptr, *loss = nullptr, *Xin = nullptr, *Tin = nullptr;
   int *counter = nullptr, *err = nullptr;
+  float* y_pin = nullptr;  // pinned: one chunk's outputs, then the error flag
   CUtensorMap fA[NL], fX[NL], wA[NL], wX[NL], hA[NL], hX[NL];
   cudaStream_t st = nullptr, st2 = nullptr;  // st2: the weight gradients, beside the input gradients
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -535,6 +536,7 @@ extern "C" int kura_mlp_create(int32_t in_dim, int32_t hidden, int32_t out_dim, 
   if (e == cudaSuccess) e = dalloc(m, &m->loss, 1);
   if (e == cudaSuccess) e = dalloc(m, &m->counter, 1);
   if (e == cudaSuccess) e = dalloc(m, &m->err, 1);
+  if (e == cudaSuccess) e = cudaMallocHost((void**)&m->y_pin, sizeof(float) * ((size_t)Bt * out_dim + 1));
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&m->ev[0]);
   if (e == cudaSuccess) e = cudaEventCreate(&m->ev[1]);
@@ -581,6 +583,7 @@ extern "C" void kura_mlp_destroy(kura_mlp* m) {
   for (cudaStream_t st : {m->st, m->st2})
     if (st) cudaStreamSynchronize(st);
   for (void* p : m->allocs) cudaFree(p);
+  if (m->y_pin) cudaFreeHost(m->y_pin);
   for (cudaEvent_t v : m->ev)
     if (v) cudaEventDestroy(v);
   for (cudaEvent_t v : m->evz)
@@ -636,10 +639,18 @@ extern "C" int kura_mlp_forward(kura_mlp* m, const float* x, int64_t n, float* y
                                               m->H[0], m->HT[0], m->Tb);
     MLPCU(cudaGetLastError());
     MLPCU(forward(m, rows));
-    MLPCU(cudaMemcpyAsync(y + r0 * m->out_dim, m->Y, sizeof(float) * m->out_dim * rows, cudaMemcpyDeviceToHost, m->st));
+    // outputs and error flag through pinned memory, one wait for both
+    const size_t ny = (size_t)rows * m->out_dim;
+    MLPCU(cudaMemcpyAsync(m->y_pin, m->Y, sizeof(float) * ny, cudaMemcpyDeviceToHost, m->st));
+    MLPCU(cudaMemcpyAsync(m->y_pin + ny, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->st));
     MLPCU(cudaStreamSynchronize(m->st));
-    int rc = check_err(m);
-    if (rc != KURA_OK) return rc;
+    int flag;
+    std::memcpy(&flag, m->y_pin + ny, sizeof flag);
+    if (flag) {
+      int rc = check_err(m);
+      if (rc != KURA_OK) return rc;
+    }
+    std::memcpy(y + r0 * m->out_dim, m->y_pin, sizeof(float) * ny);
   }
   return KURA_OK;
 }

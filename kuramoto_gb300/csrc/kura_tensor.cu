@@ -665,10 +665,28 @@ struct TensorEngine::Impl {
   float* t_eval = nullptr;
   float* out_r = nullptr;
   int* out_idx = nullptr;
+  int* ctl = nullptr;       // flags, err and cnt in one piece, cleared and read at once
   int* err = nullptr;
   int* flags = nullptr;     // [0]: a trajectory needs its first slope, [1]: one steps in the next attempt; the GEMMs skip on 0
   unsigned* cnt = nullptr;  // [bp] arrivals of a trajectory's blocks
-  int* h_run = nullptr;     // pinned: flags[1] and the error code
+  int* h_run = nullptr;     // pinned: the flags and the error code
+  // pinned copies of a small ensemble's uploads, and whether one is still on its way
+  float* h_theta = nullptr;
+  TrajG* h_traj = nullptr;
+  std::vector<char> on_its_way;
+  size_t t_eval_cap = 0, ring_cap = 0;
+  int graph_ring = 0, graph_n_eval = 0;  // what the attempt graph was captured with
+  void drop_graph() {
+    if (graph) cudaGraphExecDestroy(graph);
+    graph = nullptr;
+  }
+  // the product's form (parts of A, their map, the split) goes into the attempt graph
+  void new_adjacency(bool lo) {
+    has_lo = lo;
+    adj_set = true;
+    shaped = false;
+    drop_graph();
+  }
   int ring = 0, n_eval = 0, nblk = 1;
   CUtensorMap tmA, tmAlo, tmX, tmXhi;
   bool has_lo = false, adj_set = false;
@@ -706,10 +724,12 @@ template <typename T> static cudaError_t zalloc(T** p, size_t count) {
 TensorEngine::TensorEngine() : d(new Impl) {}
 TensorEngine::~TensorEngine() {
   void* ptrs[] = {d->omega, d->ph_hi, d->ph_lo, d->ph_w, d->g, d->X, d->x32, d->Ahi, d->Alo, d->Flo, d->rinv, d->fin_theta,
-                  d->fin_coup, d->traj, d->src, d->part, d->t_eval, d->out_r, d->out_idx, d->err, d->flags, d->cnt};
+                  d->fin_coup, d->traj, d->src, d->part, d->t_eval, d->out_r, d->out_idx, d->ctl};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (d->h_run) cudaFreeHost(d->h_run);
+  if (d->h_theta) cudaFreeHost(d->h_theta);
+  if (d->h_traj) cudaFreeHost(d->h_traj);
   if (d->graph) cudaGraphExecDestroy(d->graph);
   if (d->ev0) cudaEventDestroy(d->ev0);
   if (d->ev1) cudaEventDestroy(d->ev1);
@@ -745,10 +765,17 @@ int TensorEngine::init(int64_t n, int k, int batch, int seed, double atol, doubl
   TCU(zalloc(&I.traj, bp));
   TCU(zalloc(&I.src, 8 * bp));
   TCU(zalloc(&I.part, (size_t)bp * T_MAXC * I.nblk * 2));
-  TCU(zalloc(&I.flags, 2));
-  TCU(zalloc(&I.cnt, bp));
-  TCU(zalloc(&I.err, 4));
-  TCU(cudaHostAlloc((void**)&I.h_run, 2 * sizeof(int), cudaHostAllocDefault));
+  TCU(zalloc(&I.ctl, 4 + bp));
+  I.flags = I.ctl;
+  I.err = I.ctl + 2;
+  I.cnt = reinterpret_cast<unsigned*>(I.ctl + 4);
+  TCU(cudaHostAlloc((void**)&I.h_run, 3 * sizeof(int), cudaHostAllocDefault));
+  // from 4 MB of phases on the copies themselves outweigh the waits
+  if ((size_t)I.B * I.n * sizeof(float) <= (4u << 20)) {
+    TCU(cudaHostAlloc((void**)&I.h_theta, (size_t)I.B * I.n * sizeof(float), cudaHostAllocDefault));
+    TCU(cudaHostAlloc((void**)&I.h_traj, sizeof(TrajG) * I.B, cudaHostAllocDefault));
+    I.on_its_way.assign(I.B, 0);
+  }
   TCU(cudaEventCreate(&I.ev0));
   TCU(cudaEventCreate(&I.ev1));
   const char* tg = getenv("KURA_TIME_COUPLING");
@@ -800,8 +827,7 @@ int TensorEngine::generate_adjacency() {
     g_terr = "cuTensorMapEncodeTiled failed";
     return KURA_ERR_CUDA;
   }
-  I.has_lo = need_lo;
-  I.adj_set = true;
+  I.new_adjacency(need_lo);
   return KURA_OK;
 }
 
@@ -820,8 +846,7 @@ int TensorEngine::set_adjacency(const float* adj_host) {
     g_terr = "cuTensorMapEncodeTiled failed";
     return KURA_ERR_CUDA;
   }
-  I.has_lo = true;
-  I.adj_set = true;
+  I.new_adjacency(true);
   return KURA_OK;
 }
 
@@ -846,27 +871,58 @@ int TensorEngine::set_state(int b, const float* theta_dev, const TrajG& T) {
   TCU(cudaStreamSynchronize(I.st));
   return KURA_OK;
 }
+int TensorEngine::upload_state(int b, const float* theta, const TrajG& T) {
+  Impl& I = *d;
+  float* dev = staging(b);
+  if (!I.h_theta) {
+    TCU(cudaMemcpyAsync(dev, theta, sizeof(float) * I.n, cudaMemcpyHostToDevice, I.st));
+    return set_state(b, dev, T);
+  }
+  if (I.on_its_way[b]) {  // its pinned copy may still be read
+    TCU(cudaStreamSynchronize(I.st));
+    I.on_its_way.assign(I.B, 0);
+  }
+  float* pin = I.h_theta + (size_t)b * I.n;
+  std::memcpy(pin, theta, sizeof(float) * I.n);
+  I.h_traj[b] = T;
+  I.on_its_way[b] = 1;
+  const size_t off = (size_t)b * I.np;  // phase buffer 0
+  TCU(cudaMemcpyAsync(dev, pin, sizeof(float) * I.n, cudaMemcpyHostToDevice, I.st));
+  TCU(launch_init_state(dev, I.n, I.np, I.ph_hi + off, I.ph_lo + off, I.ph_w + off, I.st));
+  TCU(cudaMemcpyAsync(I.traj + b, I.h_traj + b, sizeof(TrajG), cudaMemcpyHostToDevice, I.st));
+  return KURA_OK;
+}
 float* TensorEngine::staging(int b) { return d->fin_theta + (size_t)b * d->np; }
 
 int TensorEngine::set_horizon(const std::vector<float>& t_eval, int ring, std::vector<TrajG>& traj) {
   Impl& I = *d;
   I.n_eval = (int)t_eval.size();
-  if (I.t_eval) cudaFree(I.t_eval);
-  if (I.out_r) cudaFree(I.out_r);
-  if (I.out_idx) cudaFree(I.out_idx);
-  I.t_eval = nullptr; I.out_r = nullptr; I.out_idx = nullptr;
-  TCU(zalloc(&I.t_eval, t_eval.size()));
+  // the buffers of an earlier horizon serve as long as they are large enough, and the attempt graph
+  // as long as nothing that it was captured with has changed
+  const bool grow_t = !I.t_eval || t_eval.size() > I.t_eval_cap;
+  const bool grow_r = !I.out_r || (size_t)ring > I.ring_cap;
+  if (grow_t || grow_r || I.graph_ring != ring || I.graph_n_eval != I.n_eval) I.drop_graph();
+  if (grow_t) {
+    if (I.t_eval) cudaFree(I.t_eval);
+    I.t_eval = nullptr;
+    TCU(zalloc(&I.t_eval, t_eval.size()));
+    I.t_eval_cap = t_eval.size();
+  }
+  if (grow_r) {
+    I.ring_cap = 0;  // until both are there
+    if (I.out_r) cudaFree(I.out_r);
+    if (I.out_idx) cudaFree(I.out_idx);
+    I.out_r = nullptr; I.out_idx = nullptr;
+    TCU(zalloc(&I.out_r, (size_t)I.bp * ring));
+    TCU(zalloc(&I.out_idx, (size_t)I.bp * ring));
+    I.ring_cap = ring;
+  }
+  I.ring = ring;
   if (!t_eval.empty())
     TCU(cudaMemcpyAsync(I.t_eval, t_eval.data(), sizeof(float) * t_eval.size(), cudaMemcpyHostToDevice, I.st));
-  I.ring = ring;
-  TCU(zalloc(&I.out_r, (size_t)I.bp * ring));
-  TCU(zalloc(&I.out_idx, (size_t)I.bp * ring));
   TCU(cudaMemcpyAsync(I.traj, traj.data(), sizeof(TrajG) * I.B, cudaMemcpyHostToDevice, I.st));
   TCU(cudaStreamSynchronize(I.st));
-  if (I.graph) {
-    cudaGraphExecDestroy(I.graph);
-    I.graph = nullptr;
-  }
+  if (!I.on_its_way.empty()) I.on_its_way.assign(I.B, 0);
   return KURA_OK;
 }
 
@@ -1022,9 +1078,7 @@ static cudaError_t attempt(TensorEngine::Impl& I) {
 int TensorEngine::run(std::vector<TrajG>& traj, kura_stats& stats, long long max_replays) {
   Impl& I = *d;
   if (!I.adj_set) { g_terr = "adjacency not set"; return KURA_ERR_INVALID; }
-  TCU(cudaMemsetAsync(I.err, 0, sizeof(int), I.st));
-  TCU(cudaMemsetAsync(I.flags, 0, 2 * sizeof(int), I.st));
-  TCU(cudaMemsetAsync(I.cnt, 0, sizeof(unsigned) * I.bp, I.st));
+  TCU(cudaMemsetAsync(I.ctl, 0, sizeof(int) * (4 + I.bp), I.st));
   TCU(cudaEventRecord(I.ev0, I.st));
   // first slope of the run, the record at t0 and the coefficients of the first attempt
   k_t_first<<<I.B, 32, 0, I.st>>>(I.traj, I.src, I.flags);
@@ -1042,6 +1096,8 @@ int TensorEngine::run(std::vector<TrajG>& traj, kura_stats& stats, long long max
     }
     TCU(cudaGraphInstantiate(&I.graph, gr, 0));
     cudaGraphDestroy(gr);
+    I.graph_ring = I.ring;
+    I.graph_n_eval = I.n_eval;
   }
   long long launches = 0;
   while (true) {
@@ -1049,11 +1105,10 @@ int TensorEngine::run(std::vector<TrajG>& traj, kura_stats& stats, long long max
       TCU(cudaGraphLaunch(I.graph, I.st));
       launches++;
     }
-    TCU(cudaMemcpyAsync(I.h_run, I.flags + 1, sizeof(int), cudaMemcpyDeviceToHost, I.st));
-    TCU(cudaMemcpyAsync(I.h_run + 1, I.err, sizeof(int), cudaMemcpyDeviceToHost, I.st));
+    TCU(cudaMemcpyAsync(I.h_run, I.ctl, 3 * sizeof(int), cudaMemcpyDeviceToHost, I.st));
     TCU(cudaStreamSynchronize(I.st));
-    if (I.h_run[1]) { g_terr = "tensor GEMM aborted (wait time limit)"; return KURA_ERR_BARRIER_TIMEOUT; }
-    if (!I.h_run[0]) break;
+    if (I.h_run[2]) { g_terr = "tensor GEMM aborted (wait time limit)"; return KURA_ERR_BARRIER_TIMEOUT; }
+    if (!I.h_run[1]) break;
     if (I.time_gemm) {  // every replay of this batch stepped some trajectory: sample the last one
       for (int q = 0; q < 6; ++q) {
         float gm = 0.f;
@@ -1075,9 +1130,14 @@ int TensorEngine::run(std::vector<TrajG>& traj, kura_stats& stats, long long max
   return KURA_OK;
 }
 
-int TensorEngine::read_order(int b, int count, float* r, int* idx) {
-  TCU(cudaMemcpy(r, d->out_r + (size_t)b * d->ring, sizeof(float) * count, cudaMemcpyDeviceToHost));
-  if (idx) TCU(cudaMemcpy(idx, d->out_idx + (size_t)b * d->ring, sizeof(int) * count, cudaMemcpyDeviceToHost));
+int TensorEngine::read_orders(int count, std::vector<float>& r, std::vector<int>& idx) {
+  const size_t w = sizeof(float) * count, pitch = sizeof(float) * d->ring;
+  r.resize((size_t)d->B * count);
+  idx.resize((size_t)d->B * count);
+  if (count <= 0) return KURA_OK;
+  TCU(cudaMemcpy2DAsync(r.data(), w, d->out_r, pitch, w, d->B, cudaMemcpyDeviceToHost, d->st));
+  TCU(cudaMemcpy2DAsync(idx.data(), w, d->out_idx, pitch, w, d->B, cudaMemcpyDeviceToHost, d->st));
+  TCU(cudaStreamSynchronize(d->st));
   return KURA_OK;
 }
 

@@ -143,6 +143,62 @@ def test_tensor_batch_128_long_horizon(native, oracle_lib):
     net.close()
 
 
+def test_tensor_engine_reused_over_horizons(native):
+    """One engine over horizons that grow, shrink and grow again (kept buffers, kept graph), with a state
+    that is replaced before its upload is over, gives the records of a fresh engine each time."""
+    n, batch = 700, 5
+    rng = np.random.default_rng(3)
+    om = (1.8 * rng.standard_cauchy(n)).astype(np.float32)
+    cs = [1.0 + 0.5 * b for b in range(batch)]
+    net = None
+    for t1, dt in ((2.0, 0.5), (2.0, 0.5), (1.0, 0.25), (1.0, 0.5), (6.0, 0.1), (2.0, 0.5)):
+        thetas = [rng.uniform(-3, 3, n).astype(np.float32) for _ in range(batch)]
+        fresh = make(native, n, 3, thetas, om, cs, t1=t1, dt=dt)
+        fresh.run()
+        if net is None:
+            net = make(native, n, 3, thetas, om, cs, t1=t1, dt=dt)
+        else:
+            for b in range(batch):
+                scratch = rng.uniform(-3, 3, n).astype(np.float32)
+                net.set_state(b, scratch, 0.0, 0.3)
+                scratch[:] = thetas[b]
+                net.set_state(b, scratch, 0.0, dt / 100)
+                scratch[:] = np.nan  # the caller's buffer is its own again
+            net.set_horizon(t1, dt, True)
+        net.run()
+        for b in range(batch):
+            np.testing.assert_array_equal(net.order(b), fresh.order(b))
+            np.testing.assert_array_equal(net.state(b)[0], fresh.state(b)[0])
+
+
+def test_tensor_engine_reused_over_adjacencies(native):
+    """A new adjacency of another form (volcano: one part; general: two) on an engine that has run."""
+    n, batch, k = 300, 3, 3
+    rng = np.random.default_rng(5)
+    om = rng.standard_normal(n).astype(np.float32)
+    cs = [1.0, 2.0, 3.0]
+    adjs = [None, rng.standard_normal((n, n)).astype(np.float32) / n, None]
+    net = None
+    for adj in adjs:
+        thetas = [rng.uniform(-3, 3, n).astype(np.float32) for _ in range(batch)]
+        fresh = make(native, n, k, thetas, om, cs, t1=2.0, dt=0.5, adj=adj)
+        fresh.run()
+        if net is None:
+            net = make(native, n, k, thetas, om, cs, t1=2.0, dt=0.5, adj=adj)
+        else:
+            if adj is None:
+                net.generate_adjacency()
+            else:
+                net.set_adjacency(adj)
+            for b in range(batch):
+                net.set_state(b, thetas[b], 0.0, 0.005)
+            net.set_horizon(2.0, 0.5, True)
+        net.run()
+        for b in range(batch):
+            np.testing.assert_array_equal(net.order(b), fresh.order(b))
+            np.testing.assert_array_equal(net.state(b)[0], fresh.state(b)[0])
+
+
 def test_tensor_rejects_unsupported(native):
     with pytest.raises(native.KuraError):
         native.Network(100, k=5, coupling=1, batch=16, engine=TENSOR)  # volcano coupling
