@@ -42,8 +42,10 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // one CTA each.  What bounds these GEMMs (512 x 256 x 256) is the epilogue's chain of TMEM reads,
 // expf and stores, 16 columns at a time, not the 0.07 us of tensor work: with one block of 256
 // columns a hidden layer took 33 us on 4 of the 152 SMs, with 32-column blocks on 32 SMs 9 us.
-// The K loop of a column is the same in either form, and so are the results, bit for bit.
-constexpr int MLP_NC = 32;
+// 16 is the narrowest that the MMA takes: a training step went from 65 to 59 us, a forward pass of
+// 64 rows from 55 to 48.  The K loop of a column is the same in every form, and so are the results,
+// bit for bit.
+constexpr int MLP_NC = 16;
 
 // ---------------------------------------------------------------- GEMM epilogues
 // forward: z = acc + b; hidden layers store silu(z) (row-major and transposed, BF16) and
@@ -155,6 +157,7 @@ struct DhEpi {
 __global__ void k_mlp_gather(const float* __restrict__ X, const float* __restrict__ T, const int* __restrict__ idx,
                              const int* counter, int in_dim, int out_dim, int Bt, int nvalid, bf16* H0, bf16* HT0,
                              float* Tb) {
+  pdl_launch();
   const int step = counter ? *counter : 0;
   const int total = Bt * max(in_dim, out_dim);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
@@ -177,6 +180,8 @@ __global__ void k_mlp_gather(const float* __restrict__ X, const float* __restric
 __global__ void k_mlp_loss(const float* __restrict__ Y, const float* __restrict__ Tb, int nvalid, int out_dim,
                            int out_p, int Bt, bf16* dZ, bf16* dZT, float* loss, int* counter) {
   __shared__ float red[32];
+  pdl_launch();
+  pdl_wait();
   const float scale = 2.f / ((float)nvalid * (float)out_dim);
   float acc = 0.f;
   for (int t = threadIdx.x; t < Bt * out_dim; t += blockDim.x) {
@@ -389,11 +394,16 @@ constexpr unsigned long long GEMM_LIMIT_NS = 20000000000ull;
 
 template <class Epi>
 cudaError_t gemm(kura_mlp* m, cudaStream_t st, const CUtensorMap& a, const CUtensorMap& x, int mtiles, int width,
-                 int ktiles, const Epi& e) {
+                 int ktiles, const Epi& e, bool overlap) {
   constexpr int NC = kura::MLP_NC;
   const int nsplit = width / NC;
-  kura::k_tensor_gemm<NC, Epi><<<std::min(mtiles * nsplit, m->sms), kura::TG_THREADS, kura::TGCfg<NC>::SMEM, st>>>(
-      a, x, mtiles, mtiles, ktiles, nsplit, NC, e, m->err, GEMM_LIMIT_NS, nullptr);
+  const dim3 grid((unsigned)std::min(mtiles * nsplit, m->sms));
+  const auto k = kura::k_tensor_gemm<NC, Epi>;
+  if (overlap)
+    return kura::launch_pdl(k, grid, kura::TG_THREADS, kura::TGCfg<NC>::SMEM, st, 1, a, x, mtiles, mtiles, ktiles,
+                            nsplit, NC, e, m->err, GEMM_LIMIT_NS, nullptr);
+  k<<<grid, kura::TG_THREADS, kura::TGCfg<NC>::SMEM, st>>>(a, x, mtiles, mtiles, ktiles, nsplit, NC, e, m->err,
+                                                           GEMM_LIMIT_NS, nullptr);
   return cudaGetLastError();
 }
 template <class Epi>
@@ -412,7 +422,7 @@ cudaError_t forward(kura_mlp* m, int rows) {
     // of the last layer only the column blocks that hold real outputs
     const int width = last ? kura::round_up(L.out, kura::MLP_NC) : L.out_p;
     cudaError_t e = gemm(m, m->st, m->fA[l], m->fX[l], kura::round_up(rows, kura::TG_BM) / kura::TG_BM, width,
-                         L.in_p / kura::TG_BK, ep);
+                         L.in_p / kura::TG_BK, ep, true);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
@@ -428,10 +438,11 @@ cudaError_t backward(kura_mlp* m) {
     if (e == cudaSuccess) e = cudaStreamWaitEvent(m->st2, m->evz[l], 0);
     kura::DwEpi dw{m->G + L.w_off, L.out_p, L.in_p};
     if (e == cudaSuccess)
-      e = gemm(m, m->st2, m->wA[l], m->wX[l], L.out_m / kura::TG_BM, L.in_p, m->Bt / kura::TG_BK, dw);
+      e = gemm(m, m->st2, m->wA[l], m->wX[l], L.out_m / kura::TG_BM, L.in_p, m->Bt / kura::TG_BK, dw,
+               false);
     if (l == 0 || e != cudaSuccess) break;
     kura::DhEpi dh{m->S[l], m->dZ[l - 1], m->dZT[l - 1], m->Bt, L.in_p};
-    e = gemm(m, m->st, m->hA[l], m->hX[l], m->Bt / kura::TG_BM, L.in_p, L.out_p / kura::TG_BK, dh);
+    e = gemm(m, m->st, m->hA[l], m->hX[l], m->Bt / kura::TG_BM, L.in_p, L.out_p / kura::TG_BK, dh, true);
   }
   if (e == cudaSuccess) e = cudaEventRecord(m->evw, m->st2);
   if (e == cudaSuccess) e = cudaStreamWaitEvent(m->st, m->evw, 0);
@@ -667,9 +678,8 @@ extern "C" int kura_mlp_gradients(kura_mlp* m, const float* x, const float* targ
                                             m->H[0], m->HT[0], m->Tb);
   MLPCU(cudaGetLastError());
   MLPCU(forward(m, m->Bt));
-  kura::k_mlp_loss<<<1, 1024, 0, m->st>>>(m->Y, m->Tb, (int)n, m->out_dim, Lo.out_p, m->Bt, m->dZ[NL - 1],
-                                          m->dZT[NL - 1], m->loss, nullptr);
-  MLPCU(cudaGetLastError());
+  MLPCU(kura::launch_pdl(kura::k_mlp_loss, dim3(1), 1024, 0, m->st, 1, m->Y, m->Tb, (int)n, m->out_dim, Lo.out_p,
+                         m->Bt, m->dZ[NL - 1], m->dZT[NL - 1], m->loss, nullptr));
   MLPCU(backward(m));
   MLPCU(update(m, kura::AdamArgs{}, kura::UPD_BIAS_GRAD));
   std::vector<float> pad(m->nparam);
@@ -730,11 +740,9 @@ extern "C" int kura_mlp_train(kura_mlp* m, const float* x, const float* target, 
                                               m->HT[0], m->Tb);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = forward(m, m->Bt);
-    if (e == cudaSuccess) {
-      kura::k_mlp_loss<<<1, 1024, 0, m->st>>>(m->Y, m->Tb, m->Bt, m->out_dim, Lo.out_p, m->Bt, m->dZ[NL - 1],
-                                              m->dZT[NL - 1], dL, m->counter);
-      e = cudaGetLastError();
-    }
+    if (e == cudaSuccess)
+      e = kura::launch_pdl(kura::k_mlp_loss, dim3(1), 1024, 0, m->st, 1, m->Y, m->Tb, m->Bt, m->out_dim, Lo.out_p,
+                           m->Bt, m->dZ[NL - 1], m->dZT[NL - 1], dL, m->counter);
     if (e == cudaSuccess) e = backward(m);
     if (e == cudaSuccess)
       e = update(m, kura::AdamArgs{m->Mo, m->Vo, m->counter, lr, lr_final, total, 0.9f, 0.999f, 1e-8f},

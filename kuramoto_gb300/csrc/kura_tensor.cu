@@ -184,10 +184,6 @@ __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast
 __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
   *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
 }
-// A kernel that the previous one's launch may overlap: what it reads and writes of the previous
-// one's data comes after pdl_wait(), which returns when that one has completed.
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __global__ void __launch_bounds__(ST_THREADS) k_t_stage(TView v, const TCoef* src) {
   pdl_launch();
@@ -924,26 +920,6 @@ int TensorEngine::set_horizon(const std::vector<float>& t_eval, int ring, std::v
   TCU(cudaStreamSynchronize(I.st));
   if (!I.on_its_way.empty()) I.on_its_way.assign(I.B, 0);
   return KURA_OK;
-}
-
-// a launch that may overlap the end of the one before it (the kernel calls pdl_wait)
-template <class... P, class... A>
-static cudaError_t launch_pdl(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cudaLaunchAttribute attr[2];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = cluster;
-  attr[1].val.clusterDim.y = 1;
-  attr[1].val.clusterDim.z = 1;
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((unsigned)threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cfg.attrs = attr;
-  cfg.numAttrs = cluster > 1 ? 2 : 1;
-  return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
 
 template <int NCOL, int MT>

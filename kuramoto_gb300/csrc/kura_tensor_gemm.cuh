@@ -60,7 +60,6 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
                   int big_tiles, int ktiles, int nsplit, int xstride, Epi epi, int* err, unsigned long long limit_ns,
                   const int* run_flag) {
   using C = TGCfg<NCOL, MT, BK>;
-  if (run_flag && *run_flag == 0) return;  // nothing to compute (every column inactive)
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + C::STAGES * C::STAGE_BYTES);
@@ -71,7 +70,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
   uint32_t* tmem_slot = (uint32_t*)(accempty + 2);
   volatile int* sabort = (volatile int*)(tmem_slot + 1);
   const int nbig = big_tiles * nsplit;
-  const int units = nbig + (mtiles - big_tiles) * MT * nsplit;
+  int units = nbig + (mtiles - big_tiles) * MT * nsplit;
   // unit u -> first row tile, row tiles in the unit, column block
   auto decode = [&](int u, int& rt0, int& mtu, int& sp) {
     if (u < nbig) {
@@ -107,6 +106,11 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
   umma::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
   const uint32_t idesc = umma::idesc_f32(Epi::F16, TG_BM, C::NMMA);
+  // Setup overlaps the end of the kernel before, when the launch allows it.  The next one is let in
+  // only now that this CTA has its TMEM: a CTA that waits never holds what another needs to go on.
+  pdl_launch();
+  pdl_wait();
+  if (run_flag && *run_flag == 0) units = 0;  // nothing to compute (every column inactive)
 
   if (warp == 0) {
     // ---------------- TMA producer
@@ -221,6 +225,27 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
     umma::tc_fence_after();
     umma::tmem_dealloc(tmem, C::TMEM_COLS);
   }
+}
+
+// a launch that may overlap the end of the one before it (the kernel calls pdl_wait)
+template <class... P, class... A>
+static cudaError_t launch_pdl(void (*k)(P...), dim3 grid, int threads, size_t smem, cudaStream_t st, int cluster,
+                              A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((unsigned)threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
 }
 
 // host: 2-D tensor map of a K-major F16 or BF16 matrix [rows][k] (row stride k elements) with a

@@ -62,7 +62,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
                  const int* run_flag) {
   using C = TSCfg<NCOL, MT>;
   constexpr int BP = C::BP;
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_launch();
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* full = (uint64_t*)(smem + C::STAGES * C::STAGE_BYTES);
@@ -88,7 +88,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
     umma::prefetch_tmap(&tmX);
   }
   // all that ran while the launch before this one (the stage kernel) was still going
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_wait();
   if (run_flag && *run_flag == 0) return;  // nothing to compute: the same for every CTA of the cluster
   if (warp == 2) umma::tmem_alloc(tmem_slot, C::TMEM_COLS);  // warp 2 also frees it
   umma::tc_fence_before();

@@ -11,6 +11,11 @@
 #include <stdint.h>
 
 namespace kura {
+// A kernel that the previous one's launch may overlap: what it reads and writes of the previous
+// one's data comes after pdl_wait(), which returns when that one has completed.
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 namespace umma {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
