@@ -13,8 +13,11 @@
 //   inputs   dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1})   A = dZ_l [B][out], X = W_l^T [in][out]
 // Widths are padded to multiples of 64 (the K tile) with zero weights, which stay zero:
 // their gradients vanish.  Adam updates FP32 master weights and rewrites the BF16 copies;
-// one whole training step (gather, forward, loss, backward, Adam) is a CUDA graph replayed
-// once per step, with the step counter on the device.
+// one whole training step (forward, loss, backward, Adam, gathering the next rows) is a CUDA graph
+// replayed once per step, with the step counter on the device.  A step is a chain of nine kernels,
+// each of some microseconds of latency: what can leave the chain (loss, weight gradients, the next
+// rows) runs beside it, and a GEMM's setup overlaps the end of the kernel before it.  For 512 rows
+// and 256 hidden units a step takes 49 us (313 us with one kernel for each piece, one after another).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -49,7 +52,9 @@ constexpr int MLP_NC = 16;
 
 // ---------------------------------------------------------------- GEMM epilogues
 // forward: z = acc + b; hidden layers store silu(z) (row-major and transposed, BF16) and
-// silu'(z); the last layer stores the real outputs of z, packed [Bt][out_dim]
+// silu'(z); the last layer stores the real outputs of z, packed [Bt][out_dim], and for training the
+// gradient of the mean squared error, 2 (y - t) / (n out_dim), in both layouts (rows from nvalid on
+// are zero; the padding columns of dZ and dZT were zeroed with the buffers and stay zero)
 struct FwdEpi {
   static constexpr bool F16 = false;
   const float* bias;
@@ -58,6 +63,11 @@ struct FwdEpi {
   bf16* HT;  // [ld][Bt]
   float* S;  // [Bt][ld]
   float* Y;  // [Bt][out_dim]
+  const float* T;  // [Bt][out_dim], or null: no gradient
+  int nvalid;
+  float scale;  // 2 / (nvalid out_dim)
+  bf16* dZ;     // [Bt][ld]
+  bf16* dZT;    // [ld][Bt]
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int r = m0 + row;
 #pragma unroll
@@ -71,8 +81,16 @@ struct FwdEpi {
       for (int j = 0; j < 16; ++j) z[j] = a[j] + bias[c0 + j];
       if (last) {
 #pragma unroll
-        for (int j = 0; j < 16; ++j)
-          if (c0 + j < out_dim) Y[(size_t)r * out_dim + c0 + j] = z[j];
+        for (int j = 0; j < 16; ++j) {
+          if (c0 + j >= out_dim) break;
+          Y[(size_t)r * out_dim + c0 + j] = z[j];
+          if (T) {
+            const float e = z[j] - T[(size_t)r * out_dim + c0 + j];
+            const bf16 b = __float2bfloat16_rn(r < nvalid ? scale * e : 0.f);
+            dZ[(size_t)r * ld + c0 + j] = b;
+            dZT[(size_t)(c0 + j) * Bt + r] = b;
+          }
+        }
         continue;
       }
       float h[16], d[16];
@@ -154,47 +172,48 @@ struct DhEpi {
 // minibatch rows of the dataset (training) or of a caller's chunk (idx == null): BF16 input
 // rows and their transpose, FP32 targets; rows >= nvalid are zero.  The padding columns past
 // in_dim were zeroed with the buffers and are never written
-__global__ void k_mlp_gather(const float* __restrict__ X, const float* __restrict__ T, const int* __restrict__ idx,
-                             const int* counter, int in_dim, int out_dim, int Bt, int nvalid, bf16* H0, bf16* HT0,
-                             float* Tb) {
-  pdl_launch();
-  const int step = counter ? *counter : 0;
-  const int total = Bt * max(in_dim, out_dim);
-  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += gridDim.x * blockDim.x) {
-    const int c = t / Bt, r = t % Bt;  // c-major: the transposed store is coalesced
+struct GatherArgs {
+  const float *X, *T;
+  const int *idx, *counter;
+  long long steps;  // with a counter: steps of the run, past which there is nothing to gather
+  int in_dim, out_dim, Bt, nvalid;
+  bf16 *H0, *HT0;
+  float* Tb;
+};
+__device__ __forceinline__ void gather_rows(const GatherArgs& a, int block, int blocks) {
+  const int step = a.counter ? *a.counter : 0;
+  if (a.counter && step >= a.steps) return;
+  const int total = a.Bt * max(a.in_dim, a.out_dim);
+  for (int t = block * blockDim.x + threadIdx.x; t < total; t += blocks * blockDim.x) {
+    const int c = t / a.Bt, r = t % a.Bt;  // c-major: the transposed store is coalesced
     long long src = -1;
-    if (r < nvalid) src = idx ? (long long)idx[(long long)step * Bt + r] : (long long)r;
-    if (c < in_dim) {
-      const bf16 b = __float2bfloat16_rn(src >= 0 ? X[src * in_dim + c] : 0.f);
-      HT0[(size_t)c * Bt + r] = b;
-      H0[(size_t)r * PADW + c] = b;
+    if (r < a.nvalid) src = a.idx ? (long long)a.idx[(long long)step * a.Bt + r] : (long long)r;
+    if (c < a.in_dim) {
+      const bf16 b = __float2bfloat16_rn(src >= 0 ? a.X[src * a.in_dim + c] : 0.f);
+      a.HT0[(size_t)c * a.Bt + r] = b;
+      a.H0[(size_t)r * PADW + c] = b;
     }
-    if (T && c < out_dim) Tb[(size_t)r * out_dim + c] = src >= 0 ? T[src * out_dim + c] : 0.f;
+    if (a.T && c < a.out_dim) a.Tb[(size_t)r * a.out_dim + c] = src >= 0 ? a.T[src * a.out_dim + c] : 0.f;
   }
 }
-
-// mean squared error over the valid rows and the first out_dim outputs; its gradient
-// 2 (y - t) / (n out_dim) in both layouts (BF16).  Only the out_dim real columns are visited:
-// the padding columns of dZ and dZT were zeroed with the buffers and stay zero (over all 64
-// columns of 512 rows one block took 40 us, over the surrogate's two it takes 4.5 us)
-__global__ void k_mlp_loss(const float* __restrict__ Y, const float* __restrict__ Tb, int nvalid, int out_dim,
-                           int out_p, int Bt, bf16* dZ, bf16* dZT, float* loss, int* counter) {
-  __shared__ float red[32];
+constexpr int GATHER_BLOCKS = 64;
+__global__ void k_mlp_gather(const __grid_constant__ GatherArgs a) {
   pdl_launch();
-  pdl_wait();
-  const float scale = 2.f / ((float)nvalid * (float)out_dim);
+  gather_rows(a, blockIdx.x, gridDim.x);
+}
+
+// mean squared error over the valid rows and the first out_dim outputs (its gradient is the last
+// layer's epilogue's); beside the backward pass, on a stream of its own
+__global__ void k_mlp_loss(const float* __restrict__ Y, const float* __restrict__ Tb, int nvalid, int out_dim, int Bt,
+                           float* loss, int* counter) {
+  __shared__ float red[32];
   float acc = 0.f;
   for (int t = threadIdx.x; t < Bt * out_dim; t += blockDim.x) {
     const int j = t / Bt, r = t % Bt;
-    float g = 0.f;
     if (r < nvalid) {
       const float e = Y[(size_t)r * out_dim + j] - Tb[(size_t)r * out_dim + j];
       acc = fmaf(e, e, acc);
-      g = scale * e;
     }
-    const bf16 b = __float2bfloat16_rn(g);
-    dZ[(size_t)r * out_p + j] = b;
-    dZT[(size_t)j * Bt + r] = b;
   }
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
@@ -225,16 +244,25 @@ struct AdamArgs {
   long long total_steps;
   float b1, b2, eps;
 };
-__device__ __forceinline__ float adam_step(float* P, const AdamArgs& a, long long i, float g, float lr, float c1,
-                                           float c2) {
-  const float m = a.b1 * a.M[i] + (1.f - a.b1) * g;
-  const float v = a.b2 * a.V[i] + (1.f - a.b2) * g * g;
-  a.M[i] = m;
-  a.V[i] = v;
-  const float p = P[i] - lr * (m / c1) / (sqrtf(v / c2) + a.eps);
-  P[i] = p;
-  return p;
-}
+// the parameter after its step, from its gradient and its own state
+struct AdamVal {
+  float p, m, v;
+  __device__ __forceinline__ void load(const float* P, const AdamArgs& a, long long i) {
+    p = P[i];
+    m = a.M[i];
+    v = a.V[i];
+  }
+  __device__ __forceinline__ float step(float* P, const AdamArgs& a, long long i, float g, float lr, float c1, float c2) {
+    // which product is rounded by itself is written out: training amplifies the last bit
+    m = __fmaf_rn(1.f - a.b1, g, __fmul_rn(a.b1, m));
+    v = __fmaf_rn(__fmul_rn(1.f - a.b2, g), g, __fmul_rn(a.b2, v));
+    a.M[i] = m;
+    a.V[i] = v;
+    p = p - lr * (m / c1) / (sqrtf(v / c2) + a.eps);
+    P[i] = p;
+    return p;
+  }
+};
 constexpr int UPD_THREADS = 256;
 constexpr int UPD_BIAS = 32;    // output units per bias block
 constexpr int UPD_ROWS = 128;   // rows of dZ staged per round of a bias block (the batch is a multiple)
@@ -244,12 +272,15 @@ constexpr int UPD_ROWS = 128;   // rows of dZ staged per round of a bias block (
 // the weights, [out][in] and, through a shared-memory tile, [in][out].  UPD_BIAS_GRAD: the bias
 // gradients, summed in the order of the rows by one thread per unit, over a tile of rows that the
 // whole block has brought into shared memory (the additions of a tile take 0.3 us; a thread that
-// loads its own rows waits for memory between them).  These are 1.3 MB of reads and writes, bound by launch latency and the depth of each
-// chain: as an Adam launch, a pack launch and a sum by one thread per unit and layer they took
-// 9 + 6.5 + 4 x 30 us per training step, together 9.7 us.
-enum { UPD_ADAM = 1, UPD_PACK = 2, UPD_BIAS_GRAD = 4 };
+// loads its own rows waits for memory between them).  UPD_GATHER: further blocks bring the rows of
+// the next step, whose launch would be 4.5 us more of the step's chain.  These are 1.3 MB of reads
+// and writes, bound by launch latency and the depth of each chain: as an Adam launch, a pack launch
+// and a sum by one thread per unit and layer they took 9 + 6.5 + 4 x 30 us per training step,
+// together 9.7 us, and 7.8 us since a thread's loads all precede its stores.
+enum { UPD_ADAM = 1, UPD_PACK = 2, UPD_BIAS_GRAD = 4, UPD_GATHER = 8 };
 __global__ void __launch_bounds__(UPD_THREADS)
-    k_mlp_update(float* P, float* G, const __grid_constant__ UpdArgs u, AdamArgs a, int Bt, int what) {
+    k_mlp_update(float* P, float* G, const __grid_constant__ UpdArgs u, AdamArgs a,
+                 const __grid_constant__ GatherArgs ga, int Bt, int what) {
   __shared__ bf16 tile[32][33];
   __shared__ bf16 stage[UPD_ROWS][32];
   int blk = blockIdx.x;
@@ -267,11 +298,24 @@ __global__ void __launch_bounds__(UPD_THREADS)
     const UpdLayer& L = u.l[l];
     if (blk < L.tiles) {
       const int o0 = blk / L.tiles_i * 32, i0 = blk % L.tiles_i * 32;
+      // every load before the first store, which the compiler must take for one to the same place
+      AdamVal val[4];
+      float g[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const long long e = L.w_off + (long long)(o0 + warp + 8 * q) * L.in_p + i0 + lane;
+        if (what & UPD_ADAM) {
+          val[q].load(P, a, e);
+          g[q] = G[e];
+        } else {
+          val[q].p = P[e];
+        }
+      }
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int o = warp + 8 * q;
         const long long e = L.w_off + (long long)(o0 + o) * L.in_p + i0 + lane;
-        const float p = (what & UPD_ADAM) ? adam_step(P, a, e, G[e], lr, c1, c2) : P[e];
+        const float p = (what & UPD_ADAM) ? val[q].step(P, a, e, g[q], lr, c1, c2) : val[q].p;
         if (what & UPD_PACK) {
           const bf16 b = __float2bfloat16_rn(p);
           L.W[(size_t)(o0 + o) * L.in_p + i0 + lane] = b;
@@ -294,6 +338,8 @@ __global__ void __launch_bounds__(UPD_THREADS)
       if (!(what & UPD_BIAS_GRAD)) return;
       const int o = blk * UPD_BIAS + lane;
       float s = 0.f;
+      AdamVal val{};
+      if ((what & UPD_ADAM) && warp == 0) val.load(P, a, L.b_off + o);
       const bf16* src = L.dZ + (size_t)warp * L.out_p + o;
       bf16 v[UPD_ROWS / 8];
       auto load = [&](int r0) {
@@ -314,12 +360,13 @@ __global__ void __launch_bounds__(UPD_THREADS)
       }
       if (warp == 0) {
         G[L.b_off + o] = s;
-        if (what & UPD_ADAM) adam_step(P, a, L.b_off + o, s, lr, c1, c2);
+        if (what & UPD_ADAM) val.step(P, a, L.b_off + o, s, lr, c1, c2);
       }
       return;
     }
     blk -= nb;
   }
+  if (what & UPD_GATHER) gather_rows(ga, blk, GATHER_BLOCKS);
 }
 struct Layer {
   int in, out, in_p, out_p, out_m;  // out_m: rows of dZ^T (at least one 128-row M tile)
@@ -358,9 +405,10 @@ struct kura_mlp {
   int *counter = nullptr, *err = nullptr;
   float* y_pin = nullptr;  // pinned: one chunk's outputs, then the error flag
   CUtensorMap fA[NL], fX[NL], wA[NL], wX[NL], hA[NL], hX[NL];
-  cudaStream_t st = nullptr, st2 = nullptr;  // st2: the weight gradients, beside the input gradients
+  // side: the loss and the weight gradients, beside the input gradients
+  cudaStream_t st = nullptr, side[2] = {nullptr, nullptr};
   cudaEvent_t ev[2] = {nullptr, nullptr};
-  cudaEvent_t evz[NL] = {}, evw = nullptr;  // dZ of a layer is ready; the weight gradients are
+  cudaEvent_t evz[NL] = {}, evw[2] = {nullptr, nullptr};  // dZ of a layer is ready; a side stream is done
   std::vector<void*> allocs;
 };
 
@@ -412,52 +460,69 @@ cudaError_t set_attr() {
                               kura::TGCfg<kura::MLP_NC>::SMEM);
 }
 
-// the first `rows` rows of the batch (rounded up to row tiles)
-cudaError_t forward(kura_mlp* m, int rows) {
+// the first `rows` rows of the batch (rounded up to row tiles); `nvalid` > 0: with the gradient of
+// the error over so many rows.  `overlap`: the kernel before the first layer lets it start early
+cudaError_t forward(kura_mlp* m, int rows, int nvalid, bool overlap) {
   for (int l = 0; l < NL; ++l) {
     const Layer& L = m->L[l];
     const bool last = (l == NL - 1);
     kura::FwdEpi ep{m->P + L.b_off, last ? 1 : 0, m->Bt, L.out_p, L.out, last ? nullptr : m->H[l + 1],
-                    last ? nullptr : m->HT[l + 1], last ? nullptr : m->S[l + 1], last ? m->Y : nullptr};
+                    last ? nullptr : m->HT[l + 1], last ? nullptr : m->S[l + 1], last ? m->Y : nullptr,
+                    last && nvalid > 0 ? m->Tb : nullptr, nvalid, 2.f / ((float)nvalid * (float)L.out),
+                    last ? m->dZ[l] : nullptr, last ? m->dZT[l] : nullptr};
     // of the last layer only the column blocks that hold real outputs
     const int width = last ? kura::round_up(L.out, kura::MLP_NC) : L.out_p;
     cudaError_t e = gemm(m, m->st, m->fA[l], m->fX[l], kura::round_up(rows, kura::TG_BM) / kura::TG_BM, width,
-                         L.in_p / kura::TG_BK, ep, true);
+                         L.in_p / kura::TG_BK, ep, l > 0 || overlap);
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
 }
 
 // The input gradients follow one another; each layer's weight gradient needs only that layer's dZ
-// and runs beside them on the second stream.
-cudaError_t backward(kura_mlp* m) {
+// and runs beside them, on the side streams in turn.  The loss needs only the outputs.
+cudaError_t backward(kura_mlp* m, int nvalid, float* loss, int* counter) {
   cudaError_t e = cudaSuccess;
   for (int l = NL - 1; l >= 0 && e == cudaSuccess; --l) {
     const Layer& L = m->L[l];
     e = cudaEventRecord(m->evz[l], m->st);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(m->st2, m->evz[l], 0);
+    if (l == NL - 1) {
+      cudaStream_t so = m->side[(l + 1) & 1];  // not the one that the first weight gradient takes
+      if (e == cudaSuccess) e = cudaStreamWaitEvent(so, m->evz[l], 0);
+      if (e == cudaSuccess) {
+        kura::k_mlp_loss<<<1, 1024, 0, so>>>(m->Y, m->Tb, nvalid, m->out_dim, m->Bt, loss, counter);
+        e = cudaGetLastError();
+      }
+    }
+    cudaStream_t sw = m->side[l & 1];
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(sw, m->evz[l], 0);
     kura::DwEpi dw{m->G + L.w_off, L.out_p, L.in_p};
     if (e == cudaSuccess)
-      e = gemm(m, m->st2, m->wA[l], m->wX[l], L.out_m / kura::TG_BM, L.in_p, m->Bt / kura::TG_BK, dw,
-               false);
+      e = gemm(m, sw, m->wA[l], m->wX[l], L.out_m / kura::TG_BM, L.in_p, m->Bt / kura::TG_BK, dw, false);
     if (l == 0 || e != cudaSuccess) break;
     kura::DhEpi dh{m->S[l], m->dZ[l - 1], m->dZT[l - 1], m->Bt, L.in_p};
     e = gemm(m, m->st, m->hA[l], m->hX[l], m->Bt / kura::TG_BM, L.in_p, L.out_p / kura::TG_BK, dh, true);
   }
-  if (e == cudaSuccess) e = cudaEventRecord(m->evw, m->st2);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(m->st, m->evw, 0);
+  for (int q = 0; q < 2; ++q) {
+    if (e == cudaSuccess) e = cudaEventRecord(m->evw[q], m->side[q]);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(m->st, m->evw[q], 0);
+  }
   return e;
 }
 
-cudaError_t update(kura_mlp* m, const kura::AdamArgs& a, int what) {
+cudaError_t update(kura_mlp* m, const kura::AdamArgs& a, int what, const kura::GatherArgs& ga = kura::GatherArgs{}) {
   kura::UpdArgs u;
-  int blocks = 0;
+  int blocks = what & kura::UPD_GATHER ? kura::GATHER_BLOCKS : 0;
   for (int l = 0; l < NL; ++l) {
     const Layer& L = m->L[l];
     u.l[l] = {L.w_off, L.b_off, L.in_p, L.out_p, (L.in_p / 32) * (L.out_p / 32), L.in_p / 32, m->W[l], m->WT[l], m->dZ[l]};
     blocks += u.l[l].tiles + L.out_p / kura::UPD_BIAS;
   }
-  kura::k_mlp_update<<<blocks, kura::UPD_THREADS, 0, m->st>>>(m->P, m->G, u, a, m->Bt, what);
+  kura::k_mlp_update<<<blocks, kura::UPD_THREADS, 0, m->st>>>(m->P, m->G, u, a, ga, m->Bt, what);
+  return cudaGetLastError();
+}
+cudaError_t gather(kura_mlp* m, const kura::GatherArgs& a) {
+  kura::k_mlp_gather<<<kura::GATHER_BLOCKS, 256, 0, m->st>>>(a);
   return cudaGetLastError();
 }
 cudaError_t pack(kura_mlp* m) { return update(m, kura::AdamArgs{}, kura::UPD_PACK); }
@@ -551,8 +616,9 @@ extern "C" int kura_mlp_create(int32_t in_dim, int32_t hidden, int32_t out_dim, 
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->st, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreate(&m->ev[0]);
   if (e == cudaSuccess) e = cudaEventCreate(&m->ev[1]);
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&m->st2, cudaStreamNonBlocking);
-  for (cudaEvent_t* v : {&m->evz[0], &m->evz[1], &m->evz[2], &m->evz[3], &m->evw})
+  for (cudaStream_t& sd : m->side)
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&sd, cudaStreamNonBlocking);
+  for (cudaEvent_t* v : {&m->evz[0], &m->evz[1], &m->evz[2], &m->evz[3], &m->evw[0], &m->evw[1]})
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(v, cudaEventDisableTiming);
   if (e == cudaSuccess) e = set_attr<kura::FwdEpi>();
   if (e == cudaSuccess) e = set_attr<kura::DwEpi>();
@@ -591,7 +657,7 @@ extern "C" int kura_mlp_create(int32_t in_dim, int32_t hidden, int32_t out_dim, 
 extern "C" void kura_mlp_destroy(kura_mlp* m) {
   if (!m) return;
   cudaSetDevice(m->device);
-  for (cudaStream_t st : {m->st, m->st2})
+  for (cudaStream_t st : {m->st, m->side[0], m->side[1]})
     if (st) cudaStreamSynchronize(st);
   for (void* p : m->allocs) cudaFree(p);
   if (m->y_pin) cudaFreeHost(m->y_pin);
@@ -599,8 +665,9 @@ extern "C" void kura_mlp_destroy(kura_mlp* m) {
     if (v) cudaEventDestroy(v);
   for (cudaEvent_t v : m->evz)
     if (v) cudaEventDestroy(v);
-  if (m->evw) cudaEventDestroy(m->evw);
-  for (cudaStream_t st : {m->st, m->st2})
+  for (cudaEvent_t v : m->evw)
+    if (v) cudaEventDestroy(v);
+  for (cudaStream_t st : {m->st, m->side[0], m->side[1]})
     if (st) cudaStreamDestroy(st);
   delete m;
 }
@@ -646,10 +713,9 @@ extern "C" int kura_mlp_forward(kura_mlp* m, const float* x, int64_t n, float* y
   for (int64_t r0 = 0; r0 < n; r0 += m->Bt) {
     const int rows = (int)std::min<int64_t>(m->Bt, n - r0);
     MLPCU(cudaMemcpyAsync(m->Xin, x + r0 * m->in_dim, sizeof(float) * rows * m->in_dim, cudaMemcpyHostToDevice, m->st));
-    kura::k_mlp_gather<<<64, 256, 0, m->st>>>(m->Xin, nullptr, nullptr, nullptr, m->in_dim, m->out_dim, m->Bt, rows,
-                                              m->H[0], m->HT[0], m->Tb);
-    MLPCU(cudaGetLastError());
-    MLPCU(forward(m, rows));
+    MLPCU(gather(m, kura::GatherArgs{m->Xin, nullptr, nullptr, nullptr, 0, m->in_dim, m->out_dim, m->Bt, rows, m->H[0],
+                                     m->HT[0], m->Tb}));
+    MLPCU(forward(m, rows, 0, true));
     // outputs and error flag through pinned memory, one wait for both
     const size_t ny = (size_t)rows * m->out_dim;
     MLPCU(cudaMemcpyAsync(m->y_pin, m->Y, sizeof(float) * ny, cudaMemcpyDeviceToHost, m->st));
@@ -671,16 +737,12 @@ extern "C" int kura_mlp_gradients(kura_mlp* m, const float* x, const float* targ
   if (!m || !x || !target || !grads) return mlp_fail(KURA_ERR_INVALID, "NULL argument");
   if (n < 1 || n > m->Bt) return mlp_fail(KURA_ERR_INVALID, "n must be 1..batch");
   MLPCU(cudaSetDevice(m->device));
-  const Layer& Lo = m->L[NL - 1];
   MLPCU(cudaMemcpyAsync(m->Xin, x, sizeof(float) * n * m->in_dim, cudaMemcpyHostToDevice, m->st));
   MLPCU(cudaMemcpyAsync(m->Tin, target, sizeof(float) * n * m->out_dim, cudaMemcpyHostToDevice, m->st));
-  kura::k_mlp_gather<<<64, 256, 0, m->st>>>(m->Xin, m->Tin, nullptr, nullptr, m->in_dim, m->out_dim, m->Bt, (int)n,
-                                            m->H[0], m->HT[0], m->Tb);
-  MLPCU(cudaGetLastError());
-  MLPCU(forward(m, m->Bt));
-  MLPCU(kura::launch_pdl(kura::k_mlp_loss, dim3(1), 1024, 0, m->st, 1, m->Y, m->Tb, (int)n, m->out_dim, Lo.out_p,
-                         m->Bt, m->dZ[NL - 1], m->dZT[NL - 1], m->loss, nullptr));
-  MLPCU(backward(m));
+  MLPCU(gather(m, kura::GatherArgs{m->Xin, m->Tin, nullptr, nullptr, 0, m->in_dim, m->out_dim, m->Bt, (int)n, m->H[0],
+                                   m->HT[0], m->Tb}));
+  MLPCU(forward(m, m->Bt, (int)n, true));
+  MLPCU(backward(m, (int)n, m->loss, nullptr));
   MLPCU(update(m, kura::AdamArgs{}, kura::UPD_BIAS_GRAD));
   std::vector<float> pad(m->nparam);
   float l = 0.f;
@@ -700,7 +762,6 @@ extern "C" int kura_mlp_train(kura_mlp* m, const float* x, const float* target, 
   if (n_samples < m->Bt) return mlp_fail(KURA_ERR_INVALID, "need at least one full batch of samples");
   if (epochs < 1) return mlp_fail(KURA_ERR_INVALID, "epochs must be >= 1");
   MLPCU(cudaSetDevice(m->device));
-  const Layer& Lo = m->L[NL - 1];
   const long long per_epoch = n_samples / m->Bt;
   const long long total = per_epoch * epochs;
   // the minibatch rows of every step: one shuffle per epoch (Fisher-Yates on splitmix64)
@@ -733,20 +794,15 @@ extern "C" int kura_mlp_train(kura_mlp* m, const float* x, const float* target, 
     MLPCU(cudaMemsetAsync(m->Vo, 0, sizeof(float) * m->nparam, m->st));
     MLPCU(cudaMemsetAsync(m->counter, 0, sizeof(int), m->st));
     MLPCU(cudaStreamSynchronize(m->st));
-    // one training step, captured
+    const kura::GatherArgs ga{dX, dT, dI, m->counter, total, m->in_dim, m->out_dim, m->Bt, m->Bt, m->H[0], m->HT[0], m->Tb};
+    MLPCU(gather(m, ga));
+    // one training step, captured; its update gathers the rows of the next one
     MLPCU(cudaStreamBeginCapture(m->st, cudaStreamCaptureModeThreadLocal));
-    cudaError_t e = cudaSuccess;
-    kura::k_mlp_gather<<<64, 256, 0, m->st>>>(dX, dT, dI, m->counter, m->in_dim, m->out_dim, m->Bt, m->Bt, m->H[0],
-                                              m->HT[0], m->Tb);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = forward(m, m->Bt);
-    if (e == cudaSuccess)
-      e = kura::launch_pdl(kura::k_mlp_loss, dim3(1), 1024, 0, m->st, 1, m->Y, m->Tb, m->Bt, m->out_dim, Lo.out_p,
-                           m->Bt, m->dZ[NL - 1], m->dZT[NL - 1], dL, m->counter);
-    if (e == cudaSuccess) e = backward(m);
+    cudaError_t e = forward(m, m->Bt, m->Bt, false);
+    if (e == cudaSuccess) e = backward(m, m->Bt, dL, m->counter);
     if (e == cudaSuccess)
       e = update(m, kura::AdamArgs{m->Mo, m->Vo, m->counter, lr, lr_final, total, 0.9f, 0.999f, 1e-8f},
-                 kura::UPD_ADAM | kura::UPD_PACK | kura::UPD_BIAS_GRAD);
+                 kura::UPD_ADAM | kura::UPD_PACK | kura::UPD_BIAS_GRAD | kura::UPD_GATHER, ga);
     cudaError_t ce = cudaStreamEndCapture(m->st, &g);
     MLPCU(e);
     MLPCU(ce);
