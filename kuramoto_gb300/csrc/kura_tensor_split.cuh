@@ -87,33 +87,56 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
     umma::prefetch_tmap(&tmA);
     umma::prefetch_tmap(&tmX);
   }
-  // all that ran while the launch before this one (the stage kernel) was still going
-  pdl_wait();
-  if (run_flag && *run_flag == 0) return;  // nothing to compute: the same for every CTA of the cluster
+  // One stage's loads.  A does not depend on the launch before this one (the stage kernel), so the
+  // first stages' A tiles, like the setup, are on their way while that one still runs; X follows.
+  // (Setup and A after the wait: runs of 3000 x 24 take 2.5 % longer, of 6007 x 64 1.5 %.)
+  auto kcol = [&](int q) { return (k0 + (q >= nk ? q - nk : q)) * TS_BK; };
+  auto load_a = [&](int q, int s) {
+    const bool lo = q >= nk;
+    umma::mbar_arrive_expect_tx(&full[s], C::A_BYTES + (lo ? C::X_BYTES / 2 : C::X_BYTES));
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+      umma::tma_load_2d(smem + s * C::STAGE_BYTES + mt * C::A1_BYTES, lo ? &tmAlo : &tmA, &full[s], kcol(q),
+                        (rt0 + mt) * TG_BM);
+  };
+  auto load_x = [&](int q, int s) {
+    umma::tma_load_2d(smem + s * C::STAGE_BYTES + C::A_BYTES, q >= nk ? &tmXhi : &tmX, &full[s], kcol(q), sp * xstride);
+  };
+  const int early = total < C::STAGES ? total : C::STAGES;
+  if (tid == 0)  // the thread that initialised the barriers
+    for (int q = 0; q < early; ++q) load_a(q, q);
+  __syncwarp();
   if (warp == 2) umma::tmem_alloc(tmem_slot, C::TMEM_COLS);  // warp 2 also frees it
   umma::tc_fence_before();
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  pdl_wait();
+  const bool skip = run_flag && *run_flag == 0;  // nothing to compute: the same for every CTA of the cluster
+  if (skip) {
+    if (tid == 0) {  // complete the early stages: no copy may outlive the CTA
+      for (int q = 0; q < early; ++q) load_x(q, q);
+      for (int q = 0; q < early; ++q) umma::mbar_wait(&full[q], 0, limit_ns, nullptr);
+    }
+    __syncthreads();
+    if (warp == 2) umma::tmem_dealloc(tmem, C::TMEM_COLS);
+    return;
+  }
 
   if (warp == 0) {
     if (lane == 0) {
       int s = 0;
       uint32_t ph = 0;
       int issued = 0;
-      for (int q = 0; q < total && !*sabort; ++q) {
-        if (!umma::mbar_wait(&empty[s], ph ^ 1, limit_ns, sabort)) {
-          *sabort = 1;
-          break;
+      for (int q = 0; q < total && (q < early || !*sabort); ++q) {
+        if (q >= early) {
+          if (!umma::mbar_wait(&empty[s], ph ^ 1, limit_ns, sabort)) {
+            *sabort = 1;
+            break;
+          }
+          load_a(q, s);
         }
-        const bool lo = q >= nk;
-        const int kc = (k0 + (lo ? q - nk : q)) * TS_BK;
-        unsigned char* st = smem + s * C::STAGE_BYTES;
-        umma::mbar_arrive_expect_tx(&full[s], C::A_BYTES + (lo ? C::X_BYTES / 2 : C::X_BYTES));
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-          umma::tma_load_2d(st + mt * C::A1_BYTES, lo ? &tmAlo : &tmA, &full[s], kc, (rt0 + mt) * TG_BM);
-        umma::tma_load_2d(st + C::A_BYTES, lo ? &tmXhi : &tmX, &full[s], kc, sp * xstride);
+        load_x(q, s);
         ++issued;
         if (++s == C::STAGES) { s = 0; ph ^= 1; }
       }
