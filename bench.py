@@ -62,7 +62,7 @@ WORKLOADS = {
                           attempts=64, atol=1e-6, rtol=0.0, engine="tensor", plain="dense65536w"),
     "dense65536w": dict(kind="windows", n=65536, k=5, cs=[3.0], init=2 * np.pi, t1=20.0, dt=0.01, attempts=64,
                         atol=1e-6, rtol=0.0, engine="persistent"),
-    # the same ensemble at N=32768 (a 2.1 GB BF16 adjacency, larger than L2): profiling captures
+    # the same ensemble at N=32768 (a 2.1 GB 16-bit adjacency, larger than L2): profiling captures
     "ensemble32768": dict(kind="windows", n=32768, k=5, cs=[3.0] * 128, init=2 * np.pi, t1=20.0, dt=0.01,
                           attempts=192, atol=1e-6, rtol=0.0, engine="tensor"),
     # a batch of 8 on either engine (the choice KURA_ENGINE_AUTO makes for small dense batches)
@@ -70,7 +70,7 @@ WORKLOADS = {
                             attempts=128, atol=1e-6, rtol=0.0, engine="tensor", plain="dense65536w"),
     "dense65536x8w": dict(kind="windows", n=65536, k=5, cs=[3.0] * 8, init=2 * np.pi, t1=20.0, dt=0.01,
                           attempts=32, atol=1e-6, rtol=0.0, engine="persistent"),
-    # the same ensemble at N=16384 (a 512 MiB BF16 adjacency, still larger than L2): profiling captures
+    # the same ensemble at N=16384 (a 512 MiB 16-bit adjacency, still larger than L2): profiling captures
     "ensemble16384": dict(n=16384, k=5, coupling=0, cs=[3.0] * 128, normal=False, init=2 * np.pi, t1=0.004,
                           dt=0.001, atol=1e-6, rtol=0.0, shared_theta=False, engine="tensor"),
     # 512 independent regenerated-volcano networks of uneven size in one launch: N log-uniform
@@ -329,7 +329,7 @@ def roofline(w, res, args):
     n = w["n"]
     if w.get("engine") == "tensor":
         # tensor-bound: algorithmic flops 24 N per accepted oscillator-step (2 products, 2 flop
-        # per multiply-add, 6 RHS); the split-BF16 product issues 2x that (hi and lo columns).
+        # per multiply-add, 6 RHS); the split product issues 2x that (hi and lo columns).
         # The GEMMs run back to back for the whole step: the sustained bf16 figure applies.
         peak = peaks.get("bf16_tflops_sustained", 1700.0)
         run_s = res["kernel_ms"] / 1e3 / max(args.steps, 1)
@@ -827,7 +827,7 @@ def main_windows(args, w):
     threads = os.cpu_count() or 1
     metric = "accepted DP45 steps x N x batch / s"
     config = {"workload": args.workload, "n": n, "k": w["k"], "coupling": "dense volcano adjacency (seed 1)",
-              "engine": "tcgen05 split-BF16 ensemble" if w["engine"] == "tensor" else "plain FP32 persistent",
+              "engine": "tcgen05 split-F16 ensemble" if w["engine"] == "tensor" else "plain FP32 persistent",
               "batch": B, "c": w["cs"][0], "theta0": "uniform [0, 2pi), one numpy stream per seed",
               "frequencies": "cauchy scale 1 (glibc rand, seed 1), shared", "t1": w["t1"], "dt": w["dt"],
               "atol": w["atol"], "rtol": w["rtol"],
@@ -948,7 +948,7 @@ def main_windows(args, w):
         return
     line = {"metric": metric, "value": value, "unit": "osc-steps/s", "n_gpus": ws, "steps": steps,
             "warmup": args.warmup, "ms_per_step": ms_max / max(steps, 1), "higher_is_better": True,
-            "scaling": "weak", "vs_baseline": None, "dtype": "f32 state, bf16 split operands, f32 accumulation",
+            "scaling": "weak", "vs_baseline": None, "dtype": "f32 state, f16 split operands, f32 accumulation",
             "data": "synthetic", "config": config}
     line["e2e"] = {"value": e2e_value, "unit": "osc-steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h}
     if w["engine"] == "tensor":
@@ -1028,7 +1028,7 @@ def roofline_tensor(n, B, d, step_ms, workload=None):
     flops = 4.0 * n * n * B
     ach = flops / (per / 1e3) / 1e12 if per > 0 else 0.0
     step_tf = 24.0 * n * d["accepted"] * n / (step_ms / 1e3) / 1e12 if step_ms > 0 else 0.0
-    # the adjacency (N*A in BF16) is read once per launch: a small batch makes the launch HBM-bound
+    # the adjacency (N*A in F16) is read once per launch: a small batch makes the launch HBM-bound
     hbm = peaks.get("hbm_gbs", 6800.0)
     a_gbs = 2.0 * n * n / (per / 1e3) / 1e9 if per > 0 else 0.0
     out = {"bound": "tensor", "achieved": round(ach, 1), "peak": peak, "unit": "TFLOP/s",

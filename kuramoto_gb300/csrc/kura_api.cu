@@ -97,7 +97,7 @@ static int resolve_engine(const kura_config* c) {
   if (c->engine == KURA_ENGINE_TENSOR) return KURA_ENGINE_TENSOR;
   if (c->engine == KURA_ENGINE_PERSISTENT) return KURA_ENGINE_PERSISTENT;
   // a dense batch of two or more that keeps only the order parameter: the tensor engine reads the
-  // BF16 adjacency once per RHS for the whole batch (a batch of 8 at N=65536: 0.95 of HBM against
+  // 16-bit adjacency once per RHS for the whole batch (a batch of 8 at N=65536: 0.95 of HBM against
   // the CUDA-core kernel's 0.34, 4.1x the throughput); per-step records need the persistent kernel
   if (c->coupling == KURA_COUPLING_DENSE && c->adj_storage != KURA_ADJ_I8 &&
       (c->batch > 8 || (c->batch >= 2 && c->dense_level == 0)))
