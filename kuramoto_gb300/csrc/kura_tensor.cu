@@ -185,20 +185,15 @@ __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d
   *reinterpret_cast<float4*>(p) = make_float4(a, b, c, d);
 }
 
-__global__ void __launch_bounds__(ST_THREADS) k_t_stage(TView v, const TCoef* src) {
-  pdl_launch();
-  pdl_wait();
-  const int b = blockIdx.y;
-  const int i = (blockIdx.x * ST_THREADS + threadIdx.x) * 4;
-  const TCoef& s = src[b];
-  if (!s.active || i >= v.n) return;
+// `last`: the newest slope where the caller has it in registers, else null; X: the operand buffer
+__device__ __forceinline__ void stage4(const TView& v, const TCoef& s, int b, int i, __half* X, const float4* last) {
   const size_t boff = ((size_t)s.base * v.bp + b) * v.np + i;
   const float4 om4 = ld4(v.omega + i), hi4 = ld4(v.ph_hi + boff), lo4 = ld4(v.ph_lo + boff);
   float4 gk[6];
 #pragma unroll
   for (int j = 0; j < 6; ++j) {
     gk[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (j < s.nW) gk[j] = ld4(v.g + ((size_t)s.slot[j] * v.bp + b) * v.np + i);
+    if (j < s.nW) gk[j] = last && j == s.nW - 1 ? *last : ld4(v.g + ((size_t)s.slot[j] * v.bp + b) * v.np + i);
   }
   float gs[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
@@ -237,7 +232,7 @@ __global__ void __launch_bounds__(ST_THREADS) k_t_stage(TView v, const TCoef* sr
   st4(x + 4, cs[2], sn[2], cs[3], sn[3]);
   auto put = [&](int q, const __half (&h)[4]) {
     const __half2 a = __halves2half2(h[0], h[1]), c = __halves2half2(h[2], h[3]);
-    *reinterpret_cast<uint2*>(v.X + xrow(q, b, v.bp) * v.np + i) =
+    *reinterpret_cast<uint2*>(X + xrow(q, b, v.bp) * v.np + i) =
         make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&c));
   };
   put(0, ch);
@@ -262,6 +257,13 @@ __global__ void __launch_bounds__(ST_THREADS) k_t_stage(TView v, const TCoef* sr
       }
     }
   }
+}
+__global__ void __launch_bounds__(ST_THREADS) k_t_stage(TView v, const TCoef* src) {
+  pdl_launch();
+  pdl_wait();
+  const int b = blockIdx.y;
+  const int i = (blockIdx.x * ST_THREADS + threadIdx.x) * 4;
+  if (src[b].active && i < v.n) stage4(v, src[b], b, i, v.X, nullptr);
 }
 
 // ---------------------------------------------------------------- GEMM epilogues
@@ -309,11 +311,16 @@ template <int BP> struct KuraEpi {
     }
   }
 };
-// the same for the split GEMM: the couplings (times N) of rows i..i+3 of trajectory b
+// The same for the split GEMM: the couplings (times N) of rows i..i+3 of trajectory b.  Within an
+// attempt it goes on to the operands of the next stage (`next`), which need no other row, into the
+// operand buffer that this launch does not read, which saves the launch and the pass of a stage
+// kernel between two GEMMs (Impl::one_group() says when).
 struct SplitEpi {
   static constexpr bool F16 = true;
   TView v;
   const TCoef* src;
+  const TCoef* next;  // or null
+  __half* Xn;
   __device__ bool wants(int b) const { return b < v.B && src[b].active; }
   __device__ void rows4(int i, int b, const float4& c4, const float4& s4) const {
     if (i >= v.n) return;
@@ -336,6 +343,10 @@ struct SplitEpi {
         v.fin_coup[(o + q) * 2 + 1] = Fs[q];
         if (v.mode == 2) v.fin_theta[o + q] = v.omega[i + q] + gv[q];
       }
+    }
+    if (next) {
+      const float4 last = make_float4(gv[0], gv[1], gv[2], gv[3]);
+      stage4(v, next[b], b, i, Xn, &last);
     }
   }
 };
@@ -684,7 +695,14 @@ struct TensorEngine::Impl {
     drop_graph();
   }
   int ring = 0, n_eval = 0, nblk = 1;
-  CUtensorMap tmA, tmAlo, tmX, tmXhi;
+  CUtensorMap tmA, tmAlo, tmX, tmXhi, tmX2, tmX2hi;
+  // the second operand buffer: the split GEMM reads one and makes the next stage's operands in the other
+  __half* X2 = nullptr;
+  // The rule: a thread of the split GEMM then has one group of four rows, so that nothing in its
+  // epilogue waits for a second pass over the slopes.  Whole runs, with the stage kernel / in the
+  // epilogue: 3000 x 24 (one group) 8.41 / 8.07 ms; 6007 x 64 (3.2 groups a thread) 5.55 / 5.71 ms.
+  bool one_group() const { return shaped && shape.mt != 0 && shape.mt * x_bph(bp) * (TG_BM / 4) <= shape.s * TS_THREADS; }
+  bool fused() const { return X2 && one_group(); }
   bool has_lo = false, adj_set = false;
   SplitShape shape;  // how the coupling GEMM runs, chosen at its first launch
   bool shaped = false;
@@ -719,7 +737,7 @@ template <typename T> static cudaError_t zalloc(T** p, size_t count) {
 
 TensorEngine::TensorEngine() : d(new Impl) {}
 TensorEngine::~TensorEngine() {
-  void* ptrs[] = {d->omega, d->ph_hi, d->ph_lo, d->ph_w, d->g, d->X, d->x32, d->Ahi, d->Alo, d->Flo, d->rinv, d->fin_theta,
+  void* ptrs[] = {d->omega, d->ph_hi, d->ph_lo, d->ph_w, d->g, d->X, d->X2, d->x32, d->Ahi, d->Alo, d->Flo, d->rinv, d->fin_theta,
                   d->fin_coup, d->traj, d->src, d->part, d->t_eval, d->out_r, d->out_idx, d->ctl};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -947,19 +965,20 @@ static int clusters_at_once(int s) {
 
 template <int NCOL, int MT>
 static cudaError_t launch_split(TensorEngine::Impl& I, const TView& v, const TCoef* src, int s, int ktiles, int nsplit,
-                                int xstride, const int* run_flag) {
+                                int xstride, const int* run_flag, int xbuf, const TCoef* next) {
   using C = TSCfg<NCOL, MT>;
   auto k = k_split_gemm<NCOL, MT, SplitEpi>;
   cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
   if (e != cudaSuccess) return e;
   const int tiles = (I.n + TG_BM - 1) / TG_BM;
   return launch_pdl(k, dim3((unsigned)((tiles + MT - 1) / MT * nsplit * s)), TS_THREADS, C::SMEM, I.st, s, I.tmA,
-                    I.has_lo ? I.tmAlo : I.tmA, I.tmX, I.tmXhi, ktiles, s, nsplit, xstride, I.has_lo ? 1 : 0,
-                    SplitEpi{v, src}, I.err, 20000000000ull, run_flag);
+                    I.has_lo ? I.tmAlo : I.tmA, xbuf ? I.tmX2 : I.tmX, xbuf ? I.tmX2hi : I.tmXhi, ktiles, s, nsplit, xstride, I.has_lo ? 1 : 0,
+                    SplitEpi{v, src, next, xbuf ? I.X : I.X2}, I.err, 20000000000ull, run_flag);
 }
 
 template <int NCOL>
-static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode, const int* run_flag) {
+static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode, const int* run_flag, int xbuf,
+                               const TCoef* next) {
   TView v{I.n, I.np, I.bp, I.B, mode, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, I.fin_theta, I.fin_coup,
           I.Flo, I.rinv};
   constexpr int BP = NCOL / 4;  // trajectories per work unit
@@ -987,8 +1006,8 @@ static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode
     I.shaped = true;
   }
   const SplitShape sh = I.shape;
-  if (sh.mt == 1) return launch_split<NCOL, 1>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag);
-  if (sh.mt == 2) return launch_split<NCOL, 2>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag);
+  if (sh.mt == 1) return launch_split<NCOL, 1>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag, xbuf, next);
+  if (sh.mt == 2) return launch_split<NCOL, 2>(I, v, src, sh.s, ktiles, nsplit, xstride, run_flag, xbuf, next);
   const unsigned long long limit = 20000000000ull;
   if (I.has_lo) {
     auto kl = k_tensor_gemm<NCOL / 2, LoEpi<BP>, 2, TE_BK>;
@@ -1009,24 +1028,29 @@ static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode
 
 // one unit holds up to 64 trajectories (NCOL = 256: two accumulators fit in TMEM); a batch
 // of 128 is two column blocks per row tile
-static cudaError_t gemm(TensorEngine::Impl& I, const TCoef* src, int mode, const int* run_flag) {
+static cudaError_t gemm(TensorEngine::Impl& I, const TCoef* src, int mode, const int* run_flag, int xbuf,
+                        const TCoef* next) {
   switch (I.bp) {
-    case 16: return launch_gemm<64>(I, src, mode, run_flag);
-    case 32: return launch_gemm<128>(I, src, mode, run_flag);
-    default: return launch_gemm<256>(I, src, mode, run_flag);
+    case 16: return launch_gemm<64>(I, src, mode, run_flag, xbuf, next);
+    case 32: return launch_gemm<128>(I, src, mode, run_flag, xbuf, next);
+    default: return launch_gemm<256>(I, src, mode, run_flag, xbuf, next);
   }
 }
 
+// xbuf: the operand buffer; made: its operands are there already; next: the coefficients of the stage
+// whose operands the GEMM makes
 static cudaError_t coupling(TensorEngine::Impl& I, const TCoef* src, int mode, float* fin_theta, const int* run_flag,
-                            int timed = -1) {
+                            int timed = -1, int xbuf = 0, bool made = false, const TCoef* next = nullptr) {
   TView v{I.n, I.np, I.bp, I.B, mode, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, fin_theta, I.fin_coup,
           I.Flo, I.rinv};
-  cudaError_t e = launch_pdl(k_t_stage, dim3((unsigned)((I.n + 4 * ST_THREADS - 1) / (4 * ST_THREADS)), (unsigned)I.B),
-                             ST_THREADS, 0, I.st, 1, v, src);
+  cudaError_t e = cudaSuccess;
+  if (!made)
+    e = launch_pdl(k_t_stage, dim3((unsigned)((I.n + 4 * ST_THREADS - 1) / (4 * ST_THREADS)), (unsigned)I.B), ST_THREADS, 0,
+                   I.st, 1, v, src);
   if (e != cudaSuccess) return e;
   const bool tm = I.time_gemm && timed >= 0;
   if (tm && (e = cudaEventRecordWithFlags(I.gev[2 * timed], I.st, cudaEventRecordExternal)) != cudaSuccess) return e;
-  if ((e = gemm(I, src, mode, run_flag)) != cudaSuccess) return e;
+  if ((e = gemm(I, src, mode, run_flag, xbuf, next)) != cudaSuccess) return e;
   if (tm) e = cudaEventRecordWithFlags(I.gev[2 * timed + 1], I.st, cudaEventRecordExternal);
   return e;
 }
@@ -1042,7 +1066,11 @@ static cudaError_t attempt(TensorEngine::Impl& I) {
   TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo, I.rinv};
   cudaError_t e = cudaSuccess;
   for (int s = 2; s <= 7; ++s) {
-    e = coupling(I, I.src + (size_t)(s - 1) * I.bp, 0, nullptr, I.flags + 1, s - 2);
+    const TCoef* src = I.src + (size_t)(s - 1) * I.bp;
+    if (I.fused())
+      e = coupling(I, src, 0, nullptr, I.flags + 1, s - 2, s & 1, s > 2, s < 7 ? src + I.bp : nullptr);
+    else
+      e = coupling(I, src, 0, nullptr, I.flags + 1, s - 2);
     if (e != cudaSuccess) return e;
   }
   e = launch_pdl(k_t_error, dim3((unsigned)(I.fixed ? 1 : I.nblk), (unsigned)I.B), T_RBLK, 0, I.st, 1, v,
@@ -1062,6 +1090,16 @@ int TensorEngine::run(std::vector<TrajG>& traj, kura_stats& stats, long long max
   TCU(coupling(I, I.src, 0, nullptr, I.flags));
   TCU(output(I, 1));
   if (!I.graph) {
+    if (I.one_group() && !I.X2) {
+      // without room for it the stage kernel goes on making all operands
+      if (zalloc(&I.X2, 4 * (size_t)I.bp * I.np) != cudaSuccess ||
+          make_tmap_16(&I.tmX2, true, I.X2, I.np, 4 * I.bp, 4 * x_bph(I.bp), TE_BK) ||
+          make_tmap_16(&I.tmX2hi, true, I.X2, I.np, 4 * I.bp, 2 * x_bph(I.bp), TE_BK)) {
+        cudaGetLastError();
+        if (I.X2) cudaFree(I.X2);
+        I.X2 = nullptr;
+      }
+    }
     cudaGraph_t gr;
     TCU(cudaStreamBeginCapture(I.st, cudaStreamCaptureModeThreadLocal));
     cudaError_t e = attempt(I);

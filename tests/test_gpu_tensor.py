@@ -143,6 +143,25 @@ def test_tensor_batch_128_long_horizon(native, oracle_lib):
     net.close()
 
 
+@pytest.mark.parametrize("n,batch", [(130, 2), (257, 16), (1000, 7), (1021, 24), (2500, 3)])
+def test_tensor_operands_from_the_gemm_match_fp64(native, oracle_lib, n, batch):
+    """Sizes whose attempts make the stages' operands in the GEMM's epilogue: ragged last tiles and
+    groups of four rows, padded columns, one and several CTAs per tile.  The bound is the other
+    runs': 1e-4 plus four times what float32 arithmetic itself is off."""
+    _, om = normal_inputs(n, 21)
+    thetas = [normal_inputs(n, 300 + b, init=2 * np.pi)[0] for b in range(batch)]
+    cs = [1.0 + 0.5 * (b % 4) for b in range(batch)]
+    net = make(native, n, 5, thetas, om, cs, seed=2, t1=5.0, dt=0.5)
+    net.run()
+    for b in (0, batch - 1):
+        r = net.order(b)
+        ref = oracle_lib.run(thetas[b], om, k=5, c1=cs[b], seed=2, fp64=True, t1=5.0, dt=0.5)
+        r32 = oracle_lib.run(thetas[b], om, k=5, c1=cs[b], seed=2, fp64=False, t1=5.0, dt=0.5)
+        assert r.size == ref.order.size == 11
+        assert np.all(np.abs(r - ref.order) <= 1e-4 + 4 * np.abs(r32.order - ref.order)), b
+    net.close()
+
+
 def test_tensor_engine_reused_over_horizons(native):
     """One engine over horizons that grow, shrink and grow again (kept buffers, kept graph), with a state
     that is replaced before its upload is over, gives the records of a fresh engine each time."""
