@@ -627,7 +627,7 @@ def main_surrogate(args, w):
                        "epochs": w["epochs"], "batch": 512, "l2": "not flushed (one pass)"},
             "e2e": {"value": st["osc_steps"] / gen_wall, "unit": "osc-steps/s", "h2d_bytes_per_step": 8 * len(X) * w["n"],
                     "d2h_bytes_per_step": 4 * len(X) * (int(w["t1"]) + 1)},
-            "gpu_launches": 1 + steps_total * 19,
+            "gpu_launches": 2 + steps_total * 13,
             "training": {"samples": len(X) - nval, "steps": steps_total, "device_ms": round(train_ms, 1),
                          "first_epoch_loss": float(losses[0]), "last_epoch_loss": float(losses[-1]),
                          "achieved_tflops": round(mlp_flops / (train_ms / 1e3) / 1e12, 3)},
@@ -952,9 +952,9 @@ def main_windows(args, w):
             "data": "synthetic", "config": config}
     line["e2e"] = {"value": e2e_value, "unit": "osc-steps/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h}
     if w["engine"] == "tensor":
-        # per attempt: coefficients, 6 x (stage phases, GEMM), error, decision, 2 output kernels;
+        # per attempt: 6 x (stage phases, GEMM), error with the decision, output with the coefficients;
         # per step: the first-slope kernels (their GEMM is skipped once the slopes are on the device)
-        line["gpu_launches"] = 17 * d["launches"] + 6 * steps
+        line["gpu_launches"] = 14 * d["launches"] + 4 * steps
         line["roofline"] = roofline_tensor(n, B, d, ms, args.workload)
     else:
         # one persistent launch per step; A is read once per RHS for the whole batch
@@ -1120,7 +1120,7 @@ def main():
     line["e2e"] = {"value": res["e2e_value"], "unit": "osc-steps/s", "h2d_bytes_per_step": res["h2d"],
                    "d2h_bytes_per_step": res["d2h"]}
     # launches of our kernels per step: B state uploads + the integrator's own launches
-    line["gpu_launches"] = (B * args.steps + res["launches"] * (1 if w.get("engine") != "tensor" else 17))
+    line["gpu_launches"] = (B * args.steps + res["launches"] * (1 if w.get("engine") != "tensor" else 14))
     line["roofline"] = roofline(w, res, args)
     line["clocks"] = res["clocks"]
     line["accepted_steps_per_run"] = res["acc_per_step"]
