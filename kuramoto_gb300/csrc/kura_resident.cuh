@@ -90,6 +90,13 @@ __host__ __device__ inline int res_units(const ResSplit& s) {
   const int c = (s.vrows + 31) / 32, w = res_vwarps(s.B);
   return c < w ? c : w;
 }
+// Where CTA `cta` leaves its nv partial sums of the exchange of parity `par` (RES_GRIDX).  A CTA may
+// still read the half of one exchange while another writes for the next (a half is written again only
+// after a further barrier), and the number of sums differs from one exchange to the next: the halves
+// lie PW_MAX sums of every CTA apart, whatever nv is.
+__host__ __device__ inline size_t res_part(const ResSplit& s, int par, int cta, int nv) {
+  return (size_t)par * s.vblocks * s.B * PW_MAX + (size_t)cta * nv;
+}
 __host__ __device__ inline int res_align(int b) { return (b + 15) & ~15; }
 // shared memory of a CTA in bytes; off[] as used by the kernel
 __host__ __device__ inline size_t res_layout(const ResSplit& s, int hl, int mode, int nt, int* off) {
@@ -333,7 +340,7 @@ struct Resident {
       if (MODE == RES_ONE) {
         mine[vb * NV + q] = s;
       } else if (MODE == RES_GRIDX) {
-        part[((size_t)(nbar & 1) * VB + gi) * NV + q] = s;
+        part[res_part(N.split, nbar & 1, gi, NV) + q] = s;
       } else {
         const uint32_t a = (uint32_t)__cvta_generic_to_shared(mine + (vb0 + vb) * NV + q);
 #pragma unroll 4
@@ -356,7 +363,7 @@ struct Resident {
         if (DEN) cp_async_wait<0>();
         return false;
       }
-      mine = part + (size_t)((nbar - 1) & 1) * VB * NV;
+      mine = part + res_part(N.split, (nbar - 1) & 1, 0, NV);
     } else {
       __syncthreads();
     }
