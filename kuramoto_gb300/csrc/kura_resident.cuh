@@ -97,6 +97,37 @@ __host__ __device__ inline int res_units(const ResSplit& s) {
 __host__ __device__ inline size_t res_part(const ResSplit& s, int par, int cta, int nv) {
   return (size_t)par * s.vblocks * s.B * PW_MAX + (size_t)cta * nv;
 }
+// The sums that leave the pass of a kind (rows() below): values v0 .. v0 + nv - 1 of every trajectory,
+// projections among them or not, and `npw`, the values that the persistent kernel would gather at once.
+// rec_r: the pass over y (kind 0) records r; coup: records keep the couplings (dense level 2)
+struct ResSums {
+  int v0, nv, npw;
+  bool proj;
+};
+__host__ __device__ inline ResSums res_sums(int kind, int k, bool den, bool rec_r, bool coup) {
+  const bool stage = kind >= 2 && kind <= 7;
+  if (den) {
+    const bool sums = kind >= 8 || (kind == 0 && rec_r);
+    return {2 * RES_KMAX, !sums ? 0 : kind == 8 ? 1 : 2, kind == 8 ? 1 : 2, false};
+  }
+  const bool all = kind == 0 || (kind == 9 && coup), proj = stage || all;
+  const int np1 = 2 * k > 1 ? 2 * k : 1;
+  const int npw = kind == 8 ? 1 : 2 * k + (kind == 9 || (kind == 0 && rec_r) ? 2 : 0);
+  return {proj ? 0 : 2 * RES_KMAX, stage ? np1 : all ? RES_RED : kind == 8 ? 1 : 2, npw > 1 ? npw : 1, proj};
+}
+// Slices of blocks that the ordered sums are formed in, each at most 16 blocks where 128 threads
+// allow: as the persistent kernel's, whose bits depend on it
+__host__ __device__ inline int res_slices(int blocks, int npw) {
+  int S = 128 / npw;
+  if (S < 1) S = 1;
+  return S < (blocks + 15) / 16 ? S : (blocks + 15) / 16;
+}
+// floats of the buffer of slices: every value of every slice.  (The number of slices follows npw, the
+// number of values nv, which is larger in kind 0 and in a record with couplings.)
+__host__ __device__ inline int res_slice_floats(const ResSplit& s) {
+  const int most = res_slices(s.vblocks, 1) * s.B * RES_RED;
+  return most > 1024 ? most : 1024;  // RES_GRID cuts its own to 1024
+}
 __host__ __device__ inline int res_align(int b) { return (b + 15) & ~15; }
 // shared memory of a CTA in bytes; off[] as used by the kernel
 __host__ __device__ inline size_t res_layout(const ResSplit& s, int hl, int mode, int nt, int* off) {
@@ -113,7 +144,7 @@ __host__ __device__ inline size_t res_layout(const ResSplit& s, int hl, int mode
   take((mode == RES_GRID ? (nt / 32) * 2 : B * nu) * RES_RED * 4);  // 3 warps' or units' sums
   take(B * RES_RED * 4);                   // 4 totals
   take(mode >= RES_GRID ? 0 : (mode == RES_CLUSTER ? 2 : 1) * s.vblocks * B * RES_RED * 4);  // 5 totals of every block
-  take(mode == RES_ONE ? 0 : 1024 * 4);    // 6 sums of slices of blocks or CTAs
+  take(mode == RES_ONE ? 0 : res_slice_floats(s) * 4);  // 6 sums of slices of blocks or CTAs (RES_ONE: one slice)
   take((B << s.k) * 8);                    // 7 sign-pattern table
   take(64 + B * 28);                       // 8 flags, per-trajectory state of the run, its warps
   take(nu * 4);                            // 9 rows of the units
@@ -367,9 +398,7 @@ struct Resident {
     } else {
       __syncthreads();
     }
-    int S = 128 / npw;
-    if (S < 1) S = 1;
-    if (S > (VB + 15) / 16) S = (VB + 15) / 16;
+    const int S = res_slices(VB, npw);
     if (S > 1 && NV) {
       for (int sl = tid / vstep; sl < S; sl += NT / vstep) {
         if (q >= NV) break;
@@ -424,7 +453,7 @@ struct Resident {
 
   // fixed: the totals are sums of sines and cosines, at most 2^20 of them.
   __device__ __forceinline__ bool exchange(int v0, int nv, bool proj, int npw, bool fixed) {
-    if (EX) return exchange_blocks(v0, nv, proj, max(npw, 1));
+    if (EX) return exchange_blocks(v0, nv, proj, npw);
     __syncthreads();
     const int NV = B * nv;
     float tot = 0.f;
@@ -963,7 +992,6 @@ struct Resident {
     }
     rec0 = want_r;
     const bool coup = N.dense_level >= 2;
-    const int np1 = max(2 * k, 1);
     long long attempts = 0;
     int kind = 0;
     if (act) {
@@ -982,17 +1010,14 @@ struct Resident {
       pass(kind);
       if (kind == 1 || (kind == 8 && N.fixed)) {
         __syncthreads();
-      } else if (DEN) {
-        const bool sums = kind >= 8 || (kind == 0 && want_r);
-        if (!exchange_blocks(2 * RES_KMAX, !sums ? 0 : kind == 8 ? 1 : 2, false, kind == 8 ? 1 : 2,
-                             kind < 8 || (kind == 9 && coup)))
-          return false;
       } else {
-        const bool st = kind >= 2 && kind <= 7, all = kind == 0 || (kind == 9 && coup);
-        if (!exchange(st || all ? 0 : 2 * RES_KMAX, st ? np1 : all ? RES_RED : kind == 8 ? 1 : 2, st || all,
-                      kind == 8 ? 1 : 2 * k + (kind == 9 || (kind == 0 && want_r) ? 2 : 0), st))
-          return false;
-        if (st || all) fill_table();
+        const ResSums q = res_sums(kind, k, DEN, want_r, coup);
+        if (DEN) {
+          if (!exchange_blocks(q.v0, q.nv, q.proj, q.npw, kind < 8 || (kind == 9 && coup))) return false;
+        } else {
+          if (!exchange(q.v0, q.nv, q.proj, q.npw, kind >= 2 && kind <= 7)) return false;
+          if (q.proj) fill_table();
+        }
       }
       const bool mine = tid < B && ((act >> tid) & 1);
       if (kind >= 2 && kind <= 7) {

@@ -47,9 +47,32 @@ static void part() {
   });
 }
 
+// the slices of ordered sums fit their buffer in every kind of pass
+static void slices() {
+  all_shapes([](const ResSplit& s) {
+    int off[18];
+    for (int mode : {RES_ONE, RES_CLUSTER, RES_GRIDX}) {
+      if (mode != RES_GRIDX && (s.den || s.vrows * s.vblocks * s.B > 12288)) continue;
+      if (mode == RES_ONE && s.vblocks > 4) continue;
+      ResSplit t = s;
+      t.ctas = mode == RES_ONE ? 1 : mode == RES_CLUSTER ? (s.vblocks < 16 ? s.vblocks : 16) : s.vblocks;
+      t.rows = (s.vblocks + t.ctas - 1) / t.ctas * s.vrows;
+      res_layout(t, 1, mode, 512, off);
+      const int room = (off[7] - off[6]) / 4;
+      for (int kind : {0, 2, 8, 9})
+        for (int flags = 0; flags < 4; ++flags) {
+          const ResSums q = res_sums(kind, s.k, s.den != 0, flags & 1, flags & 2);
+          const int S = res_slices(s.vblocks, q.npw), need = S > 1 ? S * s.B * q.nv : 0;
+          if (need > room) fail("slices", s, need, room);
+        }
+    }
+  });
+}
+
 int main(int argc, char** argv) {
   const char* what = argc > 1 ? argv[1] : "";
   if (!strcmp(what, "part")) part();
+  else if (!strcmp(what, "slices")) slices();
   else return 2;
   printf("%d violations\n", bad);
   return bad != 0;

@@ -74,6 +74,43 @@ def test_same_bits_as_the_persistent_kernel(native, n, k, batch, family, rtol):
         assert np.array_equal(state[b].view(np.uint32), fin[b].view(np.uint32))
 
 
+# batches on many blocks, whose sums at the start take more slices times values than a stage's: the grid
+# in the same order from 113 blocks on, every rank that leaves the table small
+@pytest.mark.parametrize("n,k,batch", [(7200, 2, 8), (8000, 2, 8), (10000, 2, 8), (9300, 4, 8), (11999, 4, 8), (9000, 3, 7),
+                                       (11999, 2, 7), (10000, 1, 6), (11999, 0, 6), (11999, 8, 8)])
+def test_same_bits_of_large_batches(native, n, k, batch):
+    th, om = normal_inputs(n, 40 + n)
+    thetas = [(th * np.float32(1 + 0.1 * b)).astype(np.float32) for b in range(batch)]
+    cs = [1.0 + 0.4 * b for b in range(batch)]
+    order, state, st, _ = handle_run(native, n, k, thetas, om, cs, 2.0, 0.5, 0.0)
+    r, fin, acc = persistent_run(native, n, k, thetas, om, cs, 2.0, 0.5, 0.0)
+    assert st["accepted"] == acc
+    for b in range(batch):
+        assert np.array_equal(order[b].view(np.uint32), r[b].view(np.uint32))
+        assert np.array_equal(state[b].view(np.uint32), fin[b].view(np.uint32))
+
+
+@pytest.mark.parametrize("n,k,batch", [(10000, 2, 8), (9300, 4, 8)])
+def test_couplings_of_large_batches(native, oracle_lib, n, k, batch):
+    """Records with couplings (dense level 2) of the same batches, in one launch and cut into launches."""
+    th, om = normal_inputs(n, 12, init=2 * np.pi)
+    thetas = [(th + np.float32(0.1 * b)).astype(np.float32) for b in range(batch)]
+    cs = [1.5 + 0.3 * b for b in range(batch)]
+    a = handle_run(native, n, k, thetas, om, cs, 1.0, 0.25, 0.0, level=2)
+    c = handle_run(native, n, k, thetas, om, cs, 1.0, 0.25, 0.0, level=2, attempts=3)
+    assert len(a[3]) == len(c[3]) == 5 * batch
+    key = lambda q: (q[0], q[1])  # noqa: E731
+    for x, y in zip(sorted(a[3], key=key), sorted(c[3], key=key)):
+        assert x[:3] == y[:3] and np.array_equal(x[3], y[3]) and np.array_equal(x[4], y[4])
+    for b in (0, batch - 1):
+        ref = oracle_lib.run(thetas[b], om, k=k, c1=cs[b], onthefly=True, seed=7, fp64=True, t1=1.0, dt=0.25, h0=0.0025,
+                             dense=2)
+        for q, x in enumerate(sorted((v for v in a[3] if v[0] == b), key=key)):
+            assert abs(x[2] - ref.order[q]) < 1e-5
+            assert np.max(np.abs(x[3] - ref.thetas[q])) < 1e-4
+            assert np.max(np.abs(x[4] - np.asarray(ref.couplings[q]).reshape(-1))) < 1e-4
+
+
 # the fixed-point grid: phases in shared memory and, at the last size, in L2
 @pytest.mark.parametrize("n,k,batch", [(12000, 5, 1), (20011, 8, 3), (65000, 0, 1)])
 def test_fixed_point_sums_match_the_persistent_kernel(native, n, k, batch):

@@ -20,7 +20,7 @@ def layout_bin(tmp_path_factory):
     return out
 
 
-@pytest.mark.parametrize("rule", ["part"])
+@pytest.mark.parametrize("rule", ["part", "slices"])
 def test_rule_holds_for_every_shape(layout_bin, rule):
     r = subprocess.run([layout_bin, rule], capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout
