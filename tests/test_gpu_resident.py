@@ -75,9 +75,10 @@ def test_same_bits_as_the_persistent_kernel(native, n, k, batch, family, rtol):
 
 
 # batches on many blocks, whose sums at the start take more slices times values than a stage's: the grid
-# in the same order from 113 blocks on, every rank that leaves the table small
-@pytest.mark.parametrize("n,k,batch", [(7200, 2, 8), (8000, 2, 8), (10000, 2, 8), (9300, 4, 8), (11999, 4, 8), (9000, 3, 7),
-                                       (11999, 2, 7), (10000, 1, 6), (11999, 0, 6), (11999, 8, 8)])
+# in the same order from 113 blocks on, every rank that leaves the table small (the entry point that
+# runs the persistent kernel takes 65536 pairs; the test below has larger ones)
+@pytest.mark.parametrize("n,k,batch", [(7200, 2, 8), (8000, 2, 8), (8000, 0, 8), (8192, 8, 8), (9000, 3, 7), (9300, 4, 7),
+                                       (10000, 1, 6), (10900, 0, 6)])
 def test_same_bits_of_large_batches(native, n, k, batch):
     th, om = normal_inputs(n, 40 + n)
     thetas = [(th * np.float32(1 + 0.1 * b)).astype(np.float32) for b in range(batch)]
@@ -90,7 +91,7 @@ def test_same_bits_of_large_batches(native, n, k, batch):
         assert np.array_equal(state[b].view(np.uint32), fin[b].view(np.uint32))
 
 
-@pytest.mark.parametrize("n,k,batch", [(10000, 2, 8), (9300, 4, 8)])
+@pytest.mark.parametrize("n,k,batch", [(10000, 2, 8), (9300, 4, 8), (11999, 4, 8), (11999, 2, 7), (11999, 8, 8)])
 def test_couplings_of_large_batches(native, oracle_lib, n, k, batch):
     """Records with couplings (dense level 2) of the same batches, in one launch and cut into launches."""
     th, om = normal_inputs(n, 12, init=2 * np.pi)
