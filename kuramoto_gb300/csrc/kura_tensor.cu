@@ -7,8 +7,8 @@
 // computed as (N A) x [X_hi | X_lo] with X = [cos | sin] split into F16 hi + lo and FP32
 // accumulation in TMEM; the GEMM epilogue forms g = c_b (sin F_c - cos F_s) / N directly.
 // For the reference's volcano rule N*A_ij is an integer in [-K, K], exact in F16 up to 2048, so
-// the product carries the precision of the hi+lo split of X: 2^-21 absolute, where BF16 parts of
-// the same size and rate hold 2^-18.  A general adjacency is split as 2^p_i N A_ij = A_hi + A_lo
+// the product carries the precision of the hi+lo split of X: 2^-21 of 1 and 2^-18 or better of itself,
+// where BF16 parts of the same size and rate hold 2^-18 of x.  A general adjacency is split as 2^p_i N A_ij = A_hi + A_lo
 // with a power of two per row, which keeps a row's largest entry near 2^14: A_hi has 7 significant
 // bits, A_lo 11 more.  The term A_lo X_hi is added by further K steps.
 //
@@ -41,12 +41,17 @@ constexpr int T_MAXC = 32;  // output crossings handled per step
 #define KURA_GEMM_BK 64
 #endif
 constexpr int TE_BK = KURA_GEMM_BK;
-// X_hi is a multiple of 2^-8 and X_lo the rest to 11 bits (2^-21 absolute): the tensor core cuts each
-// product off at the accumulator's last bit, always toward zero, and the coarse steps leave it
-// nothing to cut from A_hi X_hi.  With X_hi and A_hi of 11 bits each the couplings of n = 6007
-// positive weights were 2.8e-6 off, 2.0e-6 of it bias; they are
-// 2.7e-7 off now (BF16 parts: 1.8e-6), and 3.7e-7 for the volcano rule at n = 20000 (2.3e-6).
-constexpr float X_STEPS = 256.f;
+// The parts of a component x of (cos, sin): X_hi is a multiple of a step, X_lo the rest to 11 bits.
+// From |x| = 2^-3 on the step is 2^-8: the tensor core cuts each product off at the accumulator's last
+// bit, always toward zero, and coarse steps leave it nothing to cut from A_hi X_hi.  Below, X_hi has
+// X_BITS significant bits: where all phases lie near 0 or pi, a step of 2^-8 leaves all of sin to X_lo.
+// n = 6007 positive weights, rms error of the sums of sin against 64 bits: phases over [0, pi) 3.0e-7
+// of the absolute row sum (2.4e-7 with steps of 2^-8 throughout, 1.1e-6 with BF16 parts), phases of
+// 1e-2 around 0 1.0e-6 of the sums themselves (3.1e-5 and 4.4e-6).  9 bits in X_hi: 3.2e-7 and 5e-7.
+// Both parts carry a factor 2^15, which keeps X_lo clear of F16's smallest steps down to x = 2^-22
+// and comes off again with the scale of the row (rinv).
+constexpr int X_BITS = 7;
+constexpr float X_SCALE = 32768.f;
 constexpr int T_RBLK = 256; // rows per block of the reduction kernels
 
 struct TCoef {
@@ -71,7 +76,7 @@ struct TView {
   float* fin_theta;
   float* fin_coup;
   float* Flo;  // [2][bp][np] partial couplings of the A_lo pass (general adjacency)
-  const float* rinv;  // [np] 1 / (N 2^p_i): the scale of a row's couplings
+  const float* rinv;  // [np] 1 / (N 2^p_i X_SCALE): the scale of a row's couplings
 };
 
 // row of X holding column q (0 hi cos, 1 hi sin, 2 lo cos, 3 lo sin) of trajectory b: the
@@ -179,6 +184,16 @@ __global__ void k_t_coef_final(TrajG* traj, TCoef* src, int B, const float* t_ev
 // flight: one at a time moved 336 MB at N = 65536, B = 128 in 99 us, four in about 62.  The last
 // group may reach into the padding (np is a multiple of 256), whose state stays finite and meets
 // zero columns of A.
+// F16 parts of x, hi in the lower half
+__device__ __forceinline__ uint32_t x_parts(float x) {
+  // adding and taking away 1.5 * 2^23 steps rounds to a multiple of the step
+  const uint32_t small = (__float_as_uint(x) & 0x7f800000u) + ((uint32_t)(24 - X_BITS) << 23);
+  const uint32_t large = __float_as_uint(32768.f);  // 2^23 * 2^-8
+  const float m = __uint_as_float(((__float_as_uint(x) & 0x7fffffffu) < __float_as_uint(0.125f) ? small : large) | 0x400000u);
+  const float hi = __fsub_rn(__fadd_rn(x, m), m);
+  const __half2 h = __floats2half2_rn(hi * X_SCALE, (x - hi) * X_SCALE);
+  return *reinterpret_cast<const uint32_t*>(&h);
+}
 constexpr int ST_THREADS = 128;
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
 __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) {
@@ -213,7 +228,7 @@ __device__ __forceinline__ void stage4(const TView& v, const TCoef& s, int b, in
   }
   const float om[4] = {om4.x, om4.y, om4.z, om4.w}, yh[4] = {hi4.x, hi4.y, hi4.z, hi4.w}, yl[4] = {lo4.x, lo4.y, lo4.z, lo4.w};
   float cs[4], sn[4], zh[4], zl[4];
-  __half ch[4], sh[4], cl[4], sl[4];
+  uint32_t cp[4], sp[4];
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const f2 pr = two_prod(om[q], s.m_hi);
@@ -222,23 +237,20 @@ __device__ __forceinline__ void stage4(const TView& v, const TCoef& s, int b, in
     zh[q] = s2.hi;
     zl[q] = yl[q] + ((s1.lo + s2.lo) + __fmaf_rn(om[q], s.m_lo, pr.lo));
     sincos_pair(zh[q], zl[q], &sn[q], &cs[q]);
-    ch[q] = __float2half_rn(rintf(cs[q] * X_STEPS) * (1.f / X_STEPS));
-    sh[q] = __float2half_rn(rintf(sn[q] * X_STEPS) * (1.f / X_STEPS));
-    cl[q] = __float2half_rn(cs[q] - __half2float(ch[q]));
-    sl[q] = __float2half_rn(sn[q] - __half2float(sh[q]));
+    cp[q] = x_parts(cs[q]);
+    sp[q] = x_parts(sn[q]);
   }
   float* x = reinterpret_cast<float*>(v.x32 + (size_t)b * v.np + i);
   st4(x, cs[0], sn[0], cs[1], sn[1]);
   st4(x + 4, cs[2], sn[2], cs[3], sn[3]);
-  auto put = [&](int q, const __half (&h)[4]) {
-    const __half2 a = __halves2half2(h[0], h[1]), c = __halves2half2(h[2], h[3]);
+  auto put = [&](int q, const uint32_t (&h)[4], uint32_t half) {  // half: 0x5410 the hi parts, 0x7632 the lo parts
     *reinterpret_cast<uint2*>(X + xrow(q, b, v.bp) * v.np + i) =
-        make_uint2(*reinterpret_cast<const uint32_t*>(&a), *reinterpret_cast<const uint32_t*>(&c));
+        make_uint2(__byte_perm(h[0], h[1], half), __byte_perm(h[2], h[3], half));
   };
-  put(0, ch);
-  put(1, sh);
-  put(2, cl);
-  put(3, sl);
+  put(0, cp, 0x5410u);
+  put(1, sp, 0x5410u);
+  put(2, cp, 0x7632u);
+  put(3, sp, 0x7632u);
   if (s.store_y7 || s.rec) {
     const size_t o = ((size_t)(s.base ^ 1) * v.bp + b) * v.np + i;
 #pragma unroll
@@ -621,9 +633,9 @@ __global__ void k_t_split(const float* __restrict__ adj, int n, int np, float sc
       for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, sh[w]);
       int e = 14;  // frexp's exponent: m in [2^(e-1), 2^e)
       if (m > 0.f && m <= 3.4028235e38f) frexpf(m, &e);
-      e = max(-110, min(e, 120));  // 2^(14-e) and its reciprocal stay normal floats
+      e = max(-70, min(e, 120));  // 2^(14-e) and the row's scale stay normal floats
       smax = ldexpf(1.f, 14 - e);
-      rinv[i] = (1.f / scale) * ldexpf(1.f, e - 14);
+      rinv[i] = (1.f / scale) * ldexpf(1.f, e - 14) * (1.f / X_SCALE);
     }
     __syncthreads();
     const float p = smax;
@@ -642,7 +654,7 @@ __global__ void k_t_adj_out(const __half* hi, const __half* lo, int n, int np, c
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
       float a = __half2float(hi[(size_t)i * np + j]);
       if (lo) a += __half2float(lo[(size_t)i * np + j]);
-      adj[(size_t)i * n + j] = __fmul_rn(a, rinv[i]);
+      adj[(size_t)i * n + j] = __fmul_rn(a, rinv[i] * X_SCALE);
     }
 }
 
@@ -833,7 +845,7 @@ int TensorEngine::generate_adjacency() {
   if (need_lo && !I.Flo) TCU(zalloc(&I.Flo, (size_t)2 * I.bp * I.np));
   dim3 grid((unsigned)std::min((I.np + 255) / 256, 64), (unsigned)std::min(I.np, 65535));
   k_t_volcano_f16<<<grid, 256, 0, I.st>>>(bits, I.n, I.K, words, I.np, I.Ahi, need_lo ? I.Alo : nullptr);
-  k_t_fill<<<(I.np + 255) / 256, 256, 0, I.st>>>(I.rinv, I.np, 1.0f / (float)I.n);
+  k_t_fill<<<(I.np + 255) / 256, 256, 0, I.st>>>(I.rinv, I.np, (1.0f / (float)I.n) * (1.f / X_SCALE));
   TCU(cudaGetLastError());
   TCU(cudaStreamSynchronize(I.st));
   if (bits) cudaFree(bits);

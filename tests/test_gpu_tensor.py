@@ -92,6 +92,24 @@ def test_tensor_split_gemm_general_adjacency(native, oracle_lib, n, batch):
     net.close()
 
 
+@pytest.mark.parametrize("amp", [0.1, 1e-2, 1e-4, 1e-6])
+@pytest.mark.parametrize("n,batch", [(130, 3), (1000, 24)])
+def test_tensor_small_phases_keep_their_digits(native, n, batch, amp):
+    """Phases around 0: the sums of sin are small, each term with its own relative error."""
+    rng = np.random.default_rng(n)
+    om = np.zeros(n, np.float32)
+    th = (amp * rng.standard_normal(n)).astype(np.float32)
+    net = make(native, n, 5, [th] * batch, om, [1.0] * batch, seed=3)
+    a = np.rint(net.adjacency().astype(np.float64) * n) / n
+    _, cp = net.rhs(batch - 1, th)
+    x = np.sin(th.astype(np.float64))
+    err = cp.reshape(n, 2)[:, 1] - a @ x
+    # per term 2^-18 of it, the error of the two parts of sin, independent of one another; the sums in
+    # float32 are 2^-24 of themselves off per step of 16 columns, always less than the terms' share
+    assert np.sqrt(np.mean(err**2)) <= 2.0**-18 * np.sqrt(np.mean((a * a) @ (x * x)))
+    net.close()
+
+
 def test_tensor_general_adjacency_split(native, oracle_lib):
     n, batch = 200, 16
     rng = np.random.default_rng(5)
