@@ -56,7 +56,7 @@ constexpr int MLP_NC = 16;
 // gradient of the mean squared error, 2 (y - t) / (n out_dim), in both layouts (rows from nvalid on
 // are zero; the padding columns of dZ and dZT were zeroed with the buffers and stay zero)
 struct FwdEpi {
-  static constexpr bool F16 = false;
+  static constexpr __device__ bool f16() { return false; }
   const float* bias;
   int last, Bt, ld, out_dim;
   bf16* H;   // [Bt][ld]
@@ -115,7 +115,7 @@ struct FwdEpi {
 
 // weight gradient: rows are output units; rows beyond the padded width are not stored
 struct DwEpi {
-  static constexpr bool F16 = false;
+  static constexpr __device__ bool f16() { return false; }
   float* G;  // [out_p][ld]
   int out_p, ld;
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
@@ -135,7 +135,7 @@ struct DwEpi {
 
 // input gradient of a hidden layer: dZ_{l-1} = (dZ_l W_l) * silu'(Z_{l-1}), BF16, both layouts
 struct DhEpi {
-  static constexpr bool F16 = false;
+  static constexpr __device__ bool f16() { return false; }
   const float* S;  // [Bt][ld]
   bf16* dZ;        // [Bt][ld]
   bf16* dZT;       // [ld][Bt]

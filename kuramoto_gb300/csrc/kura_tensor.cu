@@ -9,13 +9,16 @@
 // For the reference's volcano rule N*A_ij is an integer in [-K, K], exact in F16 up to 2048, so
 // the product carries the precision of the hi+lo split of X: 2^-21 of 1 and 2^-18 or better of itself,
 // where BF16 parts of the same size and rate hold 2^-18 of x.  A general adjacency is split as 2^p_i N A_ij = A_hi + A_lo
-// with a power of two per row, which keeps a row's largest entry near 2^14: A_hi has 7 significant
-// bits, A_lo 11 more.  The term A_lo X_hi is added by further K steps.
+// with a power of two per row, which puts a row's largest entry below 2^15: A_hi has 7 significant
+// bits, A_lo 11 more.  The term A_lo X_hi is added by further K steps.  F16 has five bits of exponent:
+// an adjacency with a row whose entries span more than 2^21 (or lie below 2^-70, or are not finite) is
+// held in BF16 parts instead, as are its X: each entry to 2^-18 of itself, at the same size and rate.
 //
 // The DP45 attempt (dp45_step, dp45.cu:87-141) is a fixed sequence of launches --
 // coefficients, 6 x (stage, GEMM), error norm, controller, outputs -- captured once in a
 // CUDA graph and replayed; every per-trajectory decision (accept/reject, step size, t,
 // output crossings) stays on the device.  The host only polls a completion flag.
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <algorithm>
@@ -77,6 +80,7 @@ struct TView {
   float* fin_coup;
   float* Flo;  // [2][bp][np] partial couplings of the A_lo pass (general adjacency)
   const float* rinv;  // [np] 1 / (N 2^p_i X_SCALE): the scale of a row's couplings
+  int bf16;           // the parts are BF16 (rinv is 1 / N)
 };
 
 // row of X holding column q (0 hi cos, 1 hi sin, 2 lo cos, 3 lo sin) of trajectory b: the
@@ -184,8 +188,13 @@ __global__ void k_t_coef_final(TrajG* traj, TCoef* src, int B, const float* t_ev
 // flight: one at a time moved 336 MB at N = 65536, B = 128 in 99 us, four in about 62.  The last
 // group may reach into the padding (np is a multiple of 256), whose state stays finite and meets
 // zero columns of A.
-// F16 parts of x, hi in the lower half
-__device__ __forceinline__ uint32_t x_parts(float x) {
+// the 16-bit parts of x, hi in the lower half
+__device__ __forceinline__ uint32_t x_parts(float x, bool bf16) {
+  if (bf16) {
+    const __nv_bfloat16 hi = __float2bfloat16_rn(x);
+    const __nv_bfloat162 h = __halves2bfloat162(hi, __float2bfloat16_rn(x - __bfloat162float(hi)));
+    return *reinterpret_cast<const uint32_t*>(&h);
+  }
   // adding and taking away 1.5 * 2^23 steps rounds to a multiple of the step
   const uint32_t small = (__float_as_uint(x) & 0x7f800000u) + ((uint32_t)(24 - X_BITS) << 23);
   const uint32_t large = __float_as_uint(32768.f);  // 2^23 * 2^-8
@@ -237,8 +246,8 @@ __device__ __forceinline__ void stage4(const TView& v, const TCoef& s, int b, in
     zh[q] = s2.hi;
     zl[q] = yl[q] + ((s1.lo + s2.lo) + __fmaf_rn(om[q], s.m_lo, pr.lo));
     sincos_pair(zh[q], zl[q], &sn[q], &cs[q]);
-    cp[q] = x_parts(cs[q]);
-    sp[q] = x_parts(sn[q]);
+    cp[q] = x_parts(cs[q], v.bf16);
+    sp[q] = x_parts(sn[q], v.bf16);
   }
   float* x = reinterpret_cast<float*>(v.x32 + (size_t)b * v.np + i);
   st4(x, cs[0], sn[0], cs[1], sn[1]);
@@ -282,10 +291,10 @@ __global__ void __launch_bounds__(ST_THREADS) k_t_stage(TView v, const TCoef* sr
 // accumulator columns of work unit sp: [hi cos | hi sin | lo cos | lo sin] of trajectories
 // sp*BP .. sp*BP + BP - 1, BP columns each
 template <int BP> struct KuraEpi {
-  static constexpr bool F16 = true;
   TView v;
   const TCoef* src;
   int has_lo;
+  __device__ bool f16() const { return !v.bf16; }
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int i = m0 + row;
     const float rinv = v.rinv[i];
@@ -328,11 +337,11 @@ template <int BP> struct KuraEpi {
 // operand buffer that this launch does not read, which saves the launch and the pass of a stage
 // kernel between two GEMMs (Impl::one_group() says when).
 struct SplitEpi {
-  static constexpr bool F16 = true;
   TView v;
   const TCoef* src;
   const TCoef* next;  // or null
   __half* Xn;
+  __device__ bool f16() const { return !v.bf16; }
   __device__ bool wants(int b) const { return b < v.B && src[b].active; }
   __device__ void rows4(int i, int b, const float4& c4, const float4& s4) const {
     if (i >= v.n) return;
@@ -364,9 +373,9 @@ struct SplitEpi {
 };
 // the A_lo pass: columns [hi cos | hi sin]; stores the partial couplings
 template <int BP> struct LoEpi {
-  static constexpr bool F16 = true;
   TView v;
   const TCoef* src;
+  __device__ bool f16() const { return !v.bf16; }
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int i = m0 + row;
 #pragma unroll 1
@@ -615,10 +624,12 @@ __global__ void k_t_fill(float* p, int n, float v) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
 }
-// general adjacency, one block per row: 2^p N A = hi (7 bits) + lo (11 bits) in F16, with 2^p so that the row's largest
-// entry lies in [2^13, 2^14) (1 for a row of zeros or one that holds an infinity)
+// general adjacency, one block per row: 2^p N A = hi (7 bits) + lo (11 bits) in F16, with 2^p so that the
+// row's largest entry lies in [2^14, 2^15) (1 for a row of zeros).  *wide is set where F16 holds an
+// entry less well than BF16 would: one below 2^-7, whose lo part meets F16's smallest step, one that is
+// not finite, or a row below what 2^-p / N / X_SCALE can undo.
 __global__ void k_t_split(const float* __restrict__ adj, int n, int np, float scale, __half* hi, __half* lo,
-                          float* rinv) {
+                          float* rinv, int* wide) {
   __shared__ float sh[32];
   __shared__ float smax;
   for (int i = blockIdx.x; i < np; i += gridDim.x) {
@@ -631,30 +642,52 @@ __global__ void k_t_split(const float* __restrict__ adj, int n, int np, float sc
     __syncthreads();
     if (threadIdx.x == 0) {
       for (int w = 1; w < (int)(blockDim.x >> 5); ++w) m = fmaxf(m, sh[w]);
-      int e = 14;  // frexp's exponent: m in [2^(e-1), 2^e)
-      if (m > 0.f && m <= 3.4028235e38f) frexpf(m, &e);
-      e = max(-70, min(e, 120));  // 2^(14-e) and the row's scale stay normal floats
-      smax = ldexpf(1.f, 14 - e);
-      rinv[i] = (1.f / scale) * ldexpf(1.f, e - 14) * (1.f / X_SCALE);
+      int e = 15;  // frexp's exponent: m in [2^(e-1), 2^e)
+      if (m > 0.f && isfinite(m)) frexpf(m, &e);
+      if (e < -70) {
+        e = 15;
+        *wide = 1;
+      }
+      smax = ldexpf(1.f, 15 - e);
+      rinv[i] = (1.f / scale) * ldexpf(1.f, e - 15) * (1.f / X_SCALE);
     }
     __syncthreads();
     const float p = smax;
+    bool out = false;
     for (int j = threadIdx.x; j < np; j += blockDim.x) {
-      const float a = (i < n && j < n) ? adj[(size_t)i * n + j] * scale * p : 0.f;
-      // Veltkamp's split: the upper 24 - 17 = 7 bits of a (an infinity or NaN stays itself)
-      const float t = 131073.f * a, up = t - (t - a);
-      const __half h = __float2half_rn(isfinite(a) ? up : a);
+      const float a0 = (i < n && j < n) ? adj[(size_t)i * n + j] * scale : 0.f, a = a0 * p;
+      out |= !isfinite(a) || (a0 != 0.f && fabsf(a) < 0.0078125f);
+      // Veltkamp's split: the upper 24 - 17 = 7 bits of a
+      const float t = 131073.f * a;
+      const __half h = __float2half_rn(t - (t - a));
       hi[(size_t)i * np + j] = h;
       lo[(size_t)i * np + j] = __float2half_rn(a - __half2float(h));
     }
+    if (out) *wide = 1;
   }
 }
-__global__ void k_t_adj_out(const __half* hi, const __half* lo, int n, int np, const float* rinv, float* adj) {
+// the same in BF16: N A = hi + lo, 8 bits each
+__global__ void k_t_split_bf16(const float* __restrict__ adj, int n, int np, float scale, __nv_bfloat16* hi,
+                               __nv_bfloat16* lo, float* rinv) {
+  for (int i = blockIdx.x; i < np; i += gridDim.x) {
+    if (threadIdx.x == 0) rinv[i] = 1.f / scale;
+    for (int j = threadIdx.x; j < np; j += blockDim.x) {
+      const float a = (i < n && j < n) ? adj[(size_t)i * n + j] * scale : 0.f;
+      const __nv_bfloat16 h = __float2bfloat16_rn(a);
+      hi[(size_t)i * np + j] = h;
+      lo[(size_t)i * np + j] = __float2bfloat16_rn(a - __bfloat162float(h));
+    }
+  }
+}
+__global__ void k_t_adj_out(const uint16_t* hi, const uint16_t* lo, int n, int np, const float* rinv, int bf16, float* adj) {
+  auto part = [&](uint16_t h) {
+    return bf16 ? __bfloat162float(__ushort_as_bfloat16(h)) : __half2float(__ushort_as_half(h));
+  };
   for (int i = blockIdx.y; i < n; i += gridDim.y)
     for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-      float a = __half2float(hi[(size_t)i * np + j]);
-      if (lo) a += __half2float(lo[(size_t)i * np + j]);
-      adj[(size_t)i * n + j] = __fmul_rn(a, rinv[i] * X_SCALE);
+      float a = part(hi[(size_t)i * np + j]);
+      if (lo) a += part(lo[(size_t)i * np + j]);
+      adj[(size_t)i * n + j] = __fmul_rn(a, bf16 ? rinv[i] : rinv[i] * X_SCALE);
     }
 }
 
@@ -672,7 +705,7 @@ struct TensorEngine::Impl {
   float* g = nullptr;
   __half* X = nullptr;
   float2* x32 = nullptr;
-  __half* Ahi = nullptr;
+  __half* Ahi = nullptr;  // (the 16-bit buffers hold BF16 where bf16 is set)
   __half* Alo = nullptr;
   float* Flo = nullptr;
   float* rinv = nullptr;  // [np] scale of each row's couplings
@@ -684,7 +717,7 @@ struct TensorEngine::Impl {
   float* t_eval = nullptr;
   float* out_r = nullptr;
   int* out_idx = nullptr;
-  int* ctl = nullptr;       // flags, err and cnt in one piece, cleared and read at once
+  int* ctl = nullptr;       // flags, err, a word for k_t_split and cnt in one piece, cleared and read at once
   int* err = nullptr;
   int* flags = nullptr;     // [0]: a trajectory needs its first slope, [1]: one steps in the next attempt; the GEMMs skip on 0
   unsigned* cnt = nullptr;  // [bp] arrivals of a trajectory's blocks
@@ -700,8 +733,9 @@ struct TensorEngine::Impl {
     graph = nullptr;
   }
   // the product's form (parts of A, their map, the split) goes into the attempt graph
-  void new_adjacency(bool lo) {
+  void new_adjacency(bool lo, bool bf) {
     has_lo = lo;
+    bf16 = bf;
     adj_set = true;
     shaped = false;
     drop_graph();
@@ -715,7 +749,7 @@ struct TensorEngine::Impl {
   // epilogue: 3000 x 24 (one group) 8.41 / 8.07 ms; 6007 x 64 (3.2 groups a thread) 5.55 / 5.71 ms.
   bool one_group() const { return shaped && shape.mt != 0 && shape.mt * x_bph(bp) * (TG_BM / 4) <= shape.s * TS_THREADS; }
   bool fused() const { return X2 && one_group(); }
-  bool has_lo = false, adj_set = false;
+  bool has_lo = false, adj_set = false, bf16 = false;
   SplitShape shape;  // how the coupling GEMM runs, chosen at its first launch
   bool shaped = false;
   cudaGraphExec_t graph = nullptr;
@@ -853,7 +887,7 @@ int TensorEngine::generate_adjacency() {
     g_terr = "cuTensorMapEncodeTiled failed";
     return KURA_ERR_CUDA;
   }
-  I.new_adjacency(need_lo);
+  I.new_adjacency(need_lo, false);
   return KURA_OK;
 }
 
@@ -864,15 +898,24 @@ int TensorEngine::set_adjacency(const float* adj_host) {
   TCU(cudaMemcpyAsync(dadj, adj_host, sizeof(float) * (size_t)I.n * I.n, cudaMemcpyHostToDevice, I.st));
   if (!I.Alo) TCU(zalloc(&I.Alo, (size_t)I.np * I.np));
   if (!I.Flo) TCU(zalloc(&I.Flo, (size_t)2 * I.bp * I.np));
-  k_t_split<<<(unsigned)std::min(I.np, 65535), 256, 0, I.st>>>(dadj, I.n, I.np, (float)I.n, I.Ahi, I.Alo, I.rinv);
+  int wide = 0;
+  TCU(cudaMemsetAsync(I.ctl + 3, 0, sizeof(int), I.st));
+  k_t_split<<<(unsigned)std::min(I.np, 65535), 256, 0, I.st>>>(dadj, I.n, I.np, (float)I.n, I.Ahi, I.Alo, I.rinv, I.ctl + 3);
   TCU(cudaGetLastError());
+  TCU(cudaMemcpyAsync(&wide, I.ctl + 3, sizeof(int), cudaMemcpyDeviceToHost, I.st));
   TCU(cudaStreamSynchronize(I.st));
+  if (wide) {
+    k_t_split_bf16<<<(unsigned)std::min(I.np, 65535), 256, 0, I.st>>>(dadj, I.n, I.np, (float)I.n, (__nv_bfloat16*)I.Ahi,
+                                                                      (__nv_bfloat16*)I.Alo, I.rinv);
+    TCU(cudaGetLastError());
+    TCU(cudaStreamSynchronize(I.st));
+  }
   cudaFree(dadj);
   if (make_tmap_16(&I.tmAlo, true, I.Alo, I.np, I.np, TG_BM, TE_BK)) {
     g_terr = "cuTensorMapEncodeTiled failed";
     return KURA_ERR_CUDA;
   }
-  I.new_adjacency(true);
+  I.new_adjacency(true, wide != 0);
   return KURA_OK;
 }
 
@@ -881,7 +924,8 @@ int TensorEngine::get_adjacency(float* adj_host) {
   float* dadj = nullptr;
   TCU(cudaMalloc((void**)&dadj, sizeof(float) * (size_t)I.n * I.n));
   dim3 grid((unsigned)std::min((I.n + 255) / 256, 64), (unsigned)std::min(I.n, 65535));
-  k_t_adj_out<<<grid, 256, 0, I.st>>>(I.Ahi, I.has_lo ? I.Alo : nullptr, I.n, I.np, I.rinv, dadj);
+  k_t_adj_out<<<grid, 256, 0, I.st>>>((const uint16_t*)I.Ahi, I.has_lo ? (const uint16_t*)I.Alo : nullptr, I.n, I.np, I.rinv,
+                                      I.bf16 ? 1 : 0, dadj);
   TCU(cudaGetLastError());
   TCU(cudaMemcpyAsync(adj_host, dadj, sizeof(float) * (size_t)I.n * I.n, cudaMemcpyDeviceToHost, I.st));
   TCU(cudaStreamSynchronize(I.st));
@@ -992,7 +1036,7 @@ template <int NCOL>
 static cudaError_t launch_gemm(TensorEngine::Impl& I, const TCoef* src, int mode, const int* run_flag, int xbuf,
                                const TCoef* next) {
   TView v{I.n, I.np, I.bp, I.B, mode, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, I.fin_theta, I.fin_coup,
-          I.Flo, I.rinv};
+          I.Flo, I.rinv, I.bf16};
   constexpr int BP = NCOL / 4;  // trajectories per work unit
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, I.device);
@@ -1054,7 +1098,7 @@ static cudaError_t gemm(TensorEngine::Impl& I, const TCoef* src, int mode, const
 static cudaError_t coupling(TensorEngine::Impl& I, const TCoef* src, int mode, float* fin_theta, const int* run_flag,
                             int timed = -1, int xbuf = 0, bool made = false, const TCoef* next = nullptr) {
   TView v{I.n, I.np, I.bp, I.B, mode, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, fin_theta, I.fin_coup,
-          I.Flo, I.rinv};
+          I.Flo, I.rinv, I.bf16};
   cudaError_t e = cudaSuccess;
   if (!made)
     e = launch_pdl(k_t_stage, dim3((unsigned)((I.n + 4 * ST_THREADS - 1) / (4 * ST_THREADS)), (unsigned)I.B), ST_THREADS, 0,
@@ -1068,14 +1112,14 @@ static cudaError_t coupling(TensorEngine::Impl& I, const TCoef* src, int mode, f
 }
 
 static cudaError_t output(TensorEngine::Impl& I, int first) {
-  TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo, I.rinv};
+  TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo, I.rinv, I.bf16};
   return launch_pdl(k_t_output, dim3((unsigned)I.nblk, (unsigned)I.B), T_RBLK, 0, I.st, 1, v, I.traj, I.t_eval, I.part,
                     I.nblk, I.out_r, I.out_idx, I.ring, I.src, I.cnt, I.flags, first);
 }
 
 // one attempt of every trajectory, its outputs, and the coefficients of the next
 static cudaError_t attempt(TensorEngine::Impl& I) {
-  TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo, I.rinv};
+  TView v{I.n, I.np, I.bp, I.B, 0, I.omega, I.ph_hi, I.ph_lo, I.ph_w, I.g, I.X, I.x32, nullptr, I.fin_coup, I.Flo, I.rinv, I.bf16};
   cudaError_t e = cudaSuccess;
   for (int s = 2; s <= 7; ++s) {
     const TCoef* src = I.src + (size_t)(s - 1) * I.bp;

@@ -48,7 +48,7 @@ template <int NCOL, int MT = 1, int BK = TG_BK> struct TGCfg {
 // sp * xstride .. + NCOL; mtiles counts groups of MT * 128 rows.  The first big_tiles groups
 // run as units of MT row tiles; the rest run one row tile per unit, so that the last wave of
 // a persistent grid holds units of half the work (a tail of one-tile units instead of a
-// partly filled wave of MT-tile units).  Epilogue interface: Epi::F16 says which 16-bit type the
+// partly filled wave of MT-tile units).  Epilogue interface: Epi::f16() says which 16-bit type the
 // operands have, and
 // Epi::row(taddr, row, m0, sp) is called by
 // every thread of warps 1-4 with taddr = TMEM address of this thread's accumulator row
@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(TG_THREADS, 1)
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t idesc = umma::idesc_f32(Epi::F16, TG_BM, C::NMMA);
+  const uint32_t idesc = umma::idesc_f32(epi.f16(), TG_BM, C::NMMA);
   // Setup overlaps the end of the kernel before, when the launch allows it.  The next one is let in
   // only now that this CTA has its TMEM: a CTA that waits never holds what another needs to go on.
   pdl_launch();

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(TS_THREADS, 1)
     __syncwarp();
   } else if (warp == 1) {
     if (lane == 0) {
-      const uint32_t id_hi = umma::idesc_f32(Epi::F16, TG_BM, NCOL), id_lo = umma::idesc_f32(Epi::F16, TG_BM, NCOL / 2);
+      const uint32_t id_hi = umma::idesc_f32(epi.f16(), TG_BM, NCOL), id_lo = umma::idesc_f32(epi.f16(), TG_BM, NCOL / 2);
       int s = 0;
       uint32_t ph = 0;
       for (int q = 0; q < total && !*sabort; ++q) {

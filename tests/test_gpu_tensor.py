@@ -110,6 +110,87 @@ def test_tensor_small_phases_keep_their_digits(native, n, batch, amp):
     net.close()
 
 
+@pytest.mark.parametrize("n,batch", [(130, 3), (1500, 24)])
+def test_tensor_rows_of_wide_range(native, n, batch):
+    """Rows whose entries span 2^40, rows of tiny entries and of zeros: every entry of N A is held in two
+    BF16 parts, in what is given back and in the couplings."""
+    def bf16(x):  # to nearest, ties to even
+        u = x.view(np.uint32)
+        return ((u + np.uint32(0x7FFF) + ((u >> np.uint32(16)) & np.uint32(1))) & np.uint32(0xFFFF0000)).view(np.float32)
+
+    def held(a):
+        na = a * np.float32(n)
+        hi = bf16(na)
+        return (hi + bf16(na - hi)) * (np.float32(1) / np.float32(n))
+
+    rng = np.random.default_rng(n)
+    adj = ((rng.random((n, n)) + 0.5) / n).astype(np.float32)
+    adj[::2] *= np.exp2(-rng.integers(0, 41, (len(adj[::2]), n))).astype(np.float32)
+    adj[5] *= np.float32(1e-25)
+    adj[:, 7] = 1.0  # the largest entry of its row, at a phase of 0
+    adj[3] = 0
+    adj[9] = adj[11] * np.float32(1e-30)
+    om = np.zeros(n, np.float32)
+    th = (rng.random(n) * np.pi).astype(np.float32)
+    th[7] = 0
+    net = make(native, n, 5, [th] * batch, om, [1.0] * batch, adj=adj)
+    assert np.array_equal(net.adjacency(), held(adj))
+    _, cp = net.rhs(batch - 1, th)
+    # the sums of sin, to which the largest entries give nothing: 2^-17 of an entry, 2^-17 of (cos, sin),
+    # 2^-16 of the dropped lo * lo part and the sums
+    x = np.sin(th.astype(np.float64))
+    bound = 3 * 2.0**-16 * np.abs(adj.astype(np.float64)) @ np.abs(x)
+    assert np.all(np.abs(cp.reshape(n, 2)[:, 1] - adj.astype(np.float64) @ x) <= bound)
+    # the engine goes back and forth between the two forms
+    for a in (((rng.random((n, n)) + 0.5) / n).astype(np.float32), adj):
+        net.set_adjacency(a)
+        back = net.adjacency()
+        if a is adj:
+            assert np.array_equal(back, held(adj))
+        else:
+            assert np.all(np.abs(back.astype(np.float64) - a) <= 2.0**-17 * np.abs(a.astype(np.float64)))
+        _, cp = net.rhs(0, th)
+        ref = a.astype(np.float64) @ np.stack([np.cos(th.astype(np.float64)), x], 1)
+        assert np.all(np.abs(cp.reshape(n, 2) - ref) <= 3 * 2.0**-16 * np.abs(a.astype(np.float64)).sum(1)[:, None])
+    net.close()
+
+
+def test_tensor_weights_that_are_not_finite(native):
+    """They reach their own row's couplings and no other row's."""
+    n, batch = 200, 2
+    rng = np.random.default_rng(2)
+    adj = ((rng.random((n, n)) + 0.5) / n).astype(np.float32)
+    adj[11, 20], adj[60, 3] = np.inf, np.nan
+    th = (rng.random(n)).astype(np.float32)
+    net = make(native, n, 5, [th] * batch, np.zeros(n, np.float32), [1.0] * batch, adj=adj)
+    _, cp = net.rhs(1, th)
+    cp = cp.reshape(n, 2)
+    rest = np.delete(np.arange(n), [11, 60])
+    assert not np.isfinite(cp[[11, 60]]).any() and np.isfinite(cp[rest]).all()
+    ref = adj[rest].astype(np.float64) @ np.stack([np.cos(th.astype(np.float64)), np.sin(th.astype(np.float64))], 1)
+    assert np.all(np.abs(cp[rest] - ref) <= 3 * 2.0**-16 * adj[rest].astype(np.float64).sum(1)[:, None])
+    net.close()
+
+
+@pytest.mark.parametrize("n,batch", [(300, 5), (3000, 24)])
+def test_tensor_phase_that_is_not_finite(native, n, batch):
+    """A NaN phase reaches every coupling of its own trajectory and none of the others'."""
+    rng = np.random.default_rng(2)
+    om = rng.standard_normal(n).astype(np.float32)
+    thetas = [rng.uniform(-3, 3, n).astype(np.float32) for _ in range(batch)]
+    net = make(native, n, 5, thetas, om, [1.0] * batch, seed=2)
+    good = [net.rhs(b, thetas[b])[0] for b in range(batch)]
+    bad = thetas[1].copy()
+    bad[n // 2] = np.nan
+    assert np.isnan(net.rhs(1, bad)[0]).all()
+    net.set_state(1, bad, 0.0, 0.01)
+    assert np.array_equal(net.rhs(0, thetas[0])[0], good[0])
+    net.set_state(1, thetas[1], 0.0, 0.01)
+    for b in range(batch):
+        assert np.array_equal(net.rhs(b, thetas[b])[0], good[b])
+    net.close()
+
+
 def test_tensor_general_adjacency_split(native, oracle_lib):
     n, batch = 200, 16
     rng = np.random.default_rng(5)
