@@ -290,7 +290,7 @@ extern "C" int kura_create(const kura_config* cfg, kura_handle** out) {
   CUH(dalloc(&h->xbuf, 2 * B * ld));
   if (h->res.split.den == kura::RES_IMMA) CUH(dalloc(&h->xdig, 16 * ld));
   CUH(dalloc(&h->part, 2 * (size_t)G * B * kura::PW_MAX));
-  if (h->res.mode == kura::RES_MODE_FIXED) CUH(dalloc(&h->fix, 3 * B * 16));
+  if (h->res.mode == kura::RES_MODE_FIXED || h->res.split.den == kura::RES_IMMA) CUH(dalloc(&h->fix, 3 * B * 16));
   CUH(dalloc(&h->ctl, 256));
   h->bar = (unsigned*)h->ctl;
   h->err = (int*)(h->ctl + 128);             // apart from the barrier's line, which every CTA polls

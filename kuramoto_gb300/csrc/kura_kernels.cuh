@@ -47,7 +47,7 @@ struct KParams {
   float* g;            // [7][B][ld] coupling part of the stage slopes k_j - omega
   float2* xbuf;        // [2][B][ld] (cos, sin) exchanged between CTAs
   float* part;         // [2][grid][B][PW_MAX] per-CTA partial sums
-  unsigned long long* fix;  // [3][B][16] fixed-point sums of the resident integrator (zeroed before each launch)
+  unsigned long long* fix;  // [3][B][16] fixed-point sums, or [3][2] 32-bit maxima (RES_IMMA), of the resident integrator (zeroed before each launch)
   unsigned* bar;       // grid barrier arrival counter (zeroed before each launch)
   int* err;            // launch-wide abort code
   TrajG* traj;         // [B]
@@ -100,7 +100,7 @@ struct ResSplit {
   int den, ld;  // stored adjacency: RES_F32 or RES_I8 with rows of ld values; 0: regenerated coupling
 };
 enum { RES_F32 = 1, RES_I8 = 2, RES_IMMA = 3 };  // RES_IMMA: int8 on the integer tensor pipe
-constexpr int RES_MODE_FIXED = 2;  // the form that needs KParams::fix
+constexpr int RES_MODE_FIXED = 2;  // this form and RES_IMMA need KParams::fix
 struct ResPlan {
   int mode = -1, hl = 0, grid = 0;
   ResSplit split{};

@@ -78,6 +78,8 @@ struct ResNet {
   float2* x;  // [2][ld] (cos, sin) of all rows, by parity of the exchange
   int8_t* xdig;  // [2][8][ld] their digits (RES_IMMA)
 };
+// RES_IMMA takes the float product's x tile and ring where digits do not hold the components
+static_assert(IM_SMEM_X + IM_SMEM_ACC >= CT_I8 / 16 * I8_CHUNK4 * 16 && 2 * IM_SLOTS >= I8_SLOTS, "shared memory of both products");
 constexpr int RES_CTF = 7168;  // columns per x tile of the float product: leaves room for the state at N = 65536
 
 // How the rows of a network are split and summed.  RES_GRID: CTA i owns rows i * rows ..; the
@@ -200,6 +202,7 @@ struct Resident {
   unsigned long long timeout_ns;
   int nbar, par, nfix, xpar;
   bool rec0;  // the pass over y (kind 0) records r
+  uint32_t mc, ms;  // RES_IMMA: the bits of the largest |cos| and |sin| of this thread's rows in the pass
 
   __device__ Resident(const ResNet& net, unsigned char* smem, int gi_, int G_) : N(net), gi(gi_), G(G_) {
     const ResSplit& sp = net.split;
@@ -234,6 +237,8 @@ struct Resident {
     B = net.B;
     k = net.k;
     target = 0;
+    mc = ms = 0;
+    if (DEN == RES_IMMA && tid < 2) flag[2 + tid] = 0;
     nbar = 0;
     par = 0;
     nfix = 0;
@@ -311,11 +316,25 @@ struct Resident {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
   }
+  // RES_IMMA: the largest |cos| and |sin| of all rows, by their bits, in the exchange of barrier `i`.
+  // Three pairs: the one read after the last barrier is cleared after this one and used after the next.
+  __device__ __forceinline__ uint32_t* largest(int i) const { return reinterpret_cast<uint32_t*>(fix) + 2 * (i % 3); }
+  // Whether digits of 2^-30 hold the components as well as floats do: the largest is 2^-7 or more, so
+  // that half a step is at most half an ulp of it, or all are zero; none is infinite or NaN
+  __device__ static __forceinline__ bool digits_hold(uint32_t bits) {
+    return bits == 0 || (bits >= __float_as_uint(0.0078125f) && bits < __float_as_uint(1.5f));
+  }
   // grid barrier with a time limit (as the persistent kernel's); every thread gets the verdict
   __device__ bool grid_sync() {
     __syncthreads();
     target += (unsigned)G;
     if (tid == 0) {
+      if (DEN == RES_IMMA) {
+        uint32_t* w = largest(nbar);
+        atomicMax(w, (uint32_t)flag[2]);
+        atomicMax(w + 1, (uint32_t)flag[3]);
+        flag[2] = flag[3] = 0;
+      }
       // the release covers what the other threads wrote before the block barrier above
       asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(bar), "r"(1u) : "memory");
       const unsigned long long t0 = now();
@@ -415,11 +434,19 @@ struct Resident {
       rsum[b * RES_RED + v] = finish(s, v, proj);
     }
     if (MODE != RES_GRIDX) nbar++;
+    bool digits = false;
+    if (DEN == RES_IMMA) {
+      if (want_F) {
+        const uint2 m = __ldcg(reinterpret_cast<const uint2*>(largest(nbar - 1)));
+        digits = digits_hold(m.x) && digits_hold(m.y);
+      }
+      if (gi == 0 && tid == 0) __stcg(reinterpret_cast<uint2*>(largest(nbar + 1)), make_uint2(0u, 0u));
+    }
     if (DEN && want_F) {
       const float2* x = N.x + (size_t)xpar * N.ld;
       if (DEN == RES_F32)
         mv_f32().run(x, [&](int, int row, float Fc, float Fs, float2) { Fr[row - r0] = make_float2(Fc, Fs); });
-      else if (DEN == RES_IMMA)
+      else if (DEN == RES_IMMA && digits)
         mv_imma().run(N.xdig + (size_t)xpar * 8 * N.ld,
                       [&](int row, float Fc, float Fs) { Fr[row - r0] = make_float2(Fc, Fs); });
       else
@@ -698,7 +725,10 @@ struct Resident {
               xd[j * N.ld] = (int8_t)(dc >> (8 * j));
               xd[(4 + j) * N.ld] = (int8_t)(ds >> (8 * j));
             }
-          } else if (DEN) {
+            mc = max(mc, __float_as_uint(fabsf(cs[u])));
+            ms = max(ms, __float_as_uint(fabsf(sn[u])));
+          }
+          if (DEN) {
             N.x[(size_t)xpar * N.ld + r0 + rr[u]] = make_float2(cs[u], sn[u]);
           }
           sx[a] += cs[u];
@@ -788,6 +818,14 @@ struct Resident {
         case 7: rows<7>(b, base, end, step, todo, acc, sx, sy); break;
         case 8: rows<8>(b, base, end, step, todo, acc, sx, sy); break;
         default: rows<9>(b, base, end, step, todo, acc, sx, sy); break;
+      }
+      if (DEN == RES_IMMA) {
+        const uint32_t c = __reduce_max_sync(0xffffffffu, mc), s = __reduce_max_sync(0xffffffffu, ms);
+        if (lane == 0) {
+          atomicMax((uint32_t*)flag + 2, c);
+          atomicMax((uint32_t*)flag + 3, s);
+        }
+        mc = ms = 0;
       }
       if (!flush) continue;
       float* dst = red + (EX ? b * nu + q0 : warp * 2 + e) * RES_RED;

@@ -237,3 +237,48 @@ def test_integer_product_matches_fp64(native, oracle_lib, n, k):
         assert abs(x[1] - ref.order[q]) < 1e-6
         # (cos, sin) in FP32 are 1e-7 off, at random; the sums of their digits are exact
         assert np.max(np.abs(x[3] - np.asarray(ref.couplings[q]).reshape(-1))) < 3e-6 * scale + 1e-6
+
+
+@pytest.mark.parametrize("amp", [0.3, 1e-2, 1e-5, 1e-6])
+@pytest.mark.parametrize("n", [12000, 18000])
+def test_integer_product_keeps_small_components(native, n, amp):
+    """Phases around 0: digits of 2^-30 would hold sin to few bits, so such a product is the float one."""
+    k = 5
+    th = (amp * np.random.default_rng(n).standard_normal(n)).astype(np.float32)
+    om = np.zeros(n, np.float32)
+    rec, _, _ = dense_run(native, n, k, th, om, 1.0, 1e-3, 1e-3, native.ADJ_I8)
+    u = native.volcano_factor(7, n, k).astype(np.float64)
+    sign = 1.0 - 2.0 * (np.arange(k) % 2)
+    ref = (sign * (u @ np.sin(th.astype(np.float64)))) @ u / n
+    err = rec[0][3].reshape(n, 2)[:, 1] - ref
+    # sin in float32 (2 ulp) and sums of n / 32 terms per lane whose roundings are independent:
+    # 2^-22 + sqrt(n / 32) 2^-24 < 2^-18 of the sums
+    assert np.sqrt(np.mean(err**2)) <= 2.0**-18 * np.sqrt(np.mean(ref**2))
+
+
+def fixed_step_run(native, th, om, coupling, **kw):
+    net = native.Network(len(th), k=5, coupling=coupling, seed=7, dense_level=1, fixed_step=True, **kw)
+    net.set_frequencies(om)
+    if coupling == 0:
+        net.generate_adjacency()
+    net.set_coupling(0, 1.0)
+    net.set_state(0, th, 0.0, 0.05)
+    net.set_horizon(0.5, 0.25, True)
+    rec = []
+    net.run(on_output=lambda b, i, t, r, theta, cp: rec.append((r, theta)) and False)
+    net.close()
+    return rec
+
+
+def test_integer_product_passes_on_what_is_not_finite(native):
+    """A fixed-step run with one frequency that is NaN: through the coupling every row is NaN after the
+    first step, as in the float32 product."""
+    n = 12000
+    th, om = normal_inputs(n, 5)
+    om[n // 3] = np.nan
+    f32 = fixed_step_run(native, th, om, 0)
+    i8 = fixed_step_run(native, th, om, 0, adj_storage=native.ADJ_I8)
+    assert len(f32) == len(i8) == 3
+    for (r, theta), (q, phi) in zip(f32, i8):
+        assert np.isnan(r) == np.isnan(q) and np.array_equal(np.isnan(theta), np.isnan(phi))
+    assert np.isnan(i8[1][1]).all()
