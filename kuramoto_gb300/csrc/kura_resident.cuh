@@ -320,7 +320,9 @@ struct Resident {
   // Three pairs: the one read after the last barrier is cleared after this one and used after the next.
   __device__ __forceinline__ uint32_t* largest(int i) const { return reinterpret_cast<uint32_t*>(fix) + 2 * (i % 3); }
   // Whether digits of 2^-30 hold the components as well as floats do: the largest is 2^-7 or more, so
-  // that half a step is at most half an ulp of it, or all are zero; none is infinite or NaN
+  // that half a step is at most half an ulp of it, or all are zero; none is infinite or NaN.  Otherwise
+  // the product is the float one.  Sums of sin, relative error at N = 40009: phases over pi 6e-8 (float
+  // product 9e-7), of 1e-2 around 0 5e-8 (4e-7), of 1e-4 in digits 3e-6 (5e-7), of 1e-6 3e-4 (7e-7)
   __device__ static __forceinline__ bool digits_hold(uint32_t bits) {
     return bits == 0 || (bits >= __float_as_uint(0.0078125f) && bits < __float_as_uint(1.5f));
   }
