@@ -290,7 +290,7 @@ extern "C" int kura_create(const kura_config* cfg, kura_handle** out) {
   CUH(dalloc(&h->xbuf, 2 * B * ld));
   if (h->res.split.den == kura::RES_IMMA) CUH(dalloc(&h->xdig, 16 * ld));
   CUH(dalloc(&h->part, 2 * (size_t)G * B * kura::PW_MAX));
-  if (h->res.mode == kura::RES_MODE_FIXED || h->res.split.den == kura::RES_IMMA) CUH(dalloc(&h->fix, 3 * B * 16));
+  if (h->res.mode == kura::RES_MODE_FIXED || h->res.split.den == kura::RES_IMMA) CUH(dalloc(&h->fix, kura::res_fix(h->B)));
   CUH(dalloc(&h->ctl, 256));
   h->bar = (unsigned*)h->ctl;
   h->err = (int*)(h->ctl + 128);             // apart from the barrier's line, which every CTA polls
@@ -616,7 +616,7 @@ static int launch_begin(kura_handle* h, int mode, bool log_steps) {
   // the test hook of the barrier's time limit needs a launch that has a grid barrier
   const bool resident = mode == kura::MODE_INTEGRATE && h->res.mode >= 0 && p.bar_extra == 0;
   if (resident && h->fix)
-    CU(cudaMemsetAsync(h->fix, 0, sizeof(unsigned long long) * 3 * h->B * 16, h->stream));
+    CU(cudaMemsetAsync(h->fix, 0, sizeof(unsigned long long) * kura::res_fix(h->B), h->stream));
   CU(cudaEventRecord(h->ev0, h->stream));
   if (resident)
     CU(kura::launch_resident(p, h->res, h->stream));

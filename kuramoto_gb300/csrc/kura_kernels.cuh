@@ -47,7 +47,8 @@ struct KParams {
   float* g;            // [7][B][ld] coupling part of the stage slopes k_j - omega
   float2* xbuf;        // [2][B][ld] (cos, sin) exchanged between CTAs
   float* part;         // [2][grid][B][PW_MAX] per-CTA partial sums
-  unsigned long long* fix;  // [3][B][16] fixed-point sums, or [3][2] 32-bit maxima (RES_IMMA), of the resident integrator (zeroed before each launch)
+  unsigned long long* fix;  // [res_fix(B)] words of the resident integrator: [3][B][16] fixed-point sums and [3] of flags,
+                            // or [3][2] 32-bit maxima (RES_IMMA); zeroed before each launch
   unsigned* bar;       // grid barrier arrival counter (zeroed before each launch)
   int* err;            // launch-wide abort code
   TrajG* traj;         // [B]
@@ -101,6 +102,7 @@ struct ResSplit {
 };
 enum { RES_F32 = 1, RES_I8 = 2, RES_IMMA = 3 };  // RES_IMMA: int8 on the integer tensor pipe
 constexpr int RES_MODE_FIXED = 2;  // this form and RES_IMMA need KParams::fix
+constexpr size_t res_fix(int batch) { return (size_t)3 * batch * 16 + 3; }  // their number
 struct ResPlan {
   int mode = -1, hl = 0, grid = 0;
   ResSplit split{};

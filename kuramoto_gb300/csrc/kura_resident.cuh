@@ -196,7 +196,7 @@ struct Resident {
   uint32_t touched;  // trajectories whose phases or slopes this launch has changed
   // grid barrier
   unsigned *bar, target, bar_extra;
-  unsigned long long* fix;  // [3][B * 2 k] projections in fixed point
+  unsigned long long* fix;  // [3][B * 2 k] projections in fixed point, and from 3 B 16 on [3] trajectories without
   int* err;
   float* part;
   unsigned long long timeout_ns;
@@ -502,16 +502,22 @@ struct Resident {
       // (2^-41 of rounding each) instead of leaving them for every CTA to gather: one load after the
       // barrier in the place of a round of 16 per thread and two more block barriers.  Three
       // buffers: the one read after the last barrier is cleared after this one and used after the next.
+      // A total that is not finite has no integer: the trajectory's bit in a word beside them says so.
       unsigned long long* f = fix + (size_t)(nfix % 3) * NV;
+      unsigned long long* nan = fix + 3 * B * 16;
       if (tid < NV) {
+        if (!isfinite(tot)) atomicOr(nan + nfix % 3, 1ull << b);
         const long long q = __float2ll_rn(tot * 1099511627776.f);
         asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(f + tid), "l"(q) : "memory");
       }
       if (!grid_sync()) return false;
       if (tid < NV) {
         const long long q = (long long)__ldcg(f + tid);
-        rsum[b * RES_RED + v] = finish(__ll2float_rn(q) * (1.f / 1099511627776.f), v, proj);
+        const uint32_t lost = (uint32_t)__ldcg(nan + nfix % 3) >> b & 1u;
+        // (added, so that both loads are under way together: 0.4 us an exchange as a branch)
+        rsum[b * RES_RED + v] = finish(__ll2float_rn(q) * (1.f / 1099511627776.f) + __uint_as_float(lost * 0x7fc00000u), v, proj);
         if (gi == 0) __stcg(fix + (size_t)((nfix + 2) % 3) * NV + tid, 0ull);
+        if (gi == 0 && tid == 0) __stcg(nan + (nfix + 2) % 3, 0ull);
       }
       nfix++;
       __syncthreads();

@@ -256,14 +256,14 @@ def test_integer_product_keeps_small_components(native, n, amp):
     assert np.sqrt(np.mean(err**2)) <= 2.0**-18 * np.sqrt(np.mean(ref**2))
 
 
-def fixed_step_run(native, th, om, coupling, **kw):
+def fixed_step_run(native, th, om, coupling, step=0.05, t1=0.5, dt=0.25, **kw):
     net = native.Network(len(th), k=5, coupling=coupling, seed=7, dense_level=1, fixed_step=True, **kw)
     net.set_frequencies(om)
     if coupling == 0:
         net.generate_adjacency()
     net.set_coupling(0, 1.0)
-    net.set_state(0, th, 0.0, 0.05)
-    net.set_horizon(0.5, 0.25, True)
+    net.set_state(0, th, 0.0, step)
+    net.set_horizon(t1, dt, True)
     rec = []
     net.run(on_output=lambda b, i, t, r, theta, cp: rec.append((r, theta)) and False)
     net.close()
@@ -282,3 +282,39 @@ def test_integer_product_passes_on_what_is_not_finite(native):
     for (r, theta), (q, phi) in zip(f32, i8):
         assert np.isnan(r) == np.isnan(q) and np.array_equal(np.isnan(theta), np.isnan(phi))
     assert np.isnan(i8[1][1]).all()
+
+
+@pytest.mark.parametrize("n", [11999, 12000, 30011])
+def test_regenerated_coupling_passes_on_what_is_not_finite(native, n):
+    """The same with nothing stored: sums in floating point below 12000 oscillators, in integers, which
+    have no NaN, from there on."""
+    th, om = normal_inputs(n, 5)
+    om[n // 3] = 3e38  # finite at the start, not so in the stages of the first step
+    rec = fixed_step_run(native, th, om, VOLCANO, step=4.0, t1=16.0, dt=8.0)
+    assert len(rec) == 3 and np.isfinite(rec[0][1]).all()
+    assert not np.isfinite(rec[1][1][n // 3])
+    for r, theta in rec[1:]:
+        assert np.isnan(r) and not np.isfinite(theta).any()
+
+
+@pytest.mark.parametrize("n", [12000, 200003])
+def test_a_trajectory_that_is_not_finite_stays_by_itself(native, n):
+    """One trajectory of five starts with a NaN phase: the others are the same bits as without it."""
+    th, om = normal_inputs(n, 5)
+    out = []
+    for bad in (False, True):
+        net = native.Network(n, k=5, coupling=VOLCANO, batch=5, seed=7, fixed_step=True)
+        net.set_frequencies(om)
+        for b in range(5):
+            t = (th * np.float32(1 + 0.1 * b)).astype(np.float32)
+            if bad and b == 3:
+                t[n // 2] = np.nan
+            net.set_coupling(b, 1.0 + 0.2 * b)
+            net.set_state(b, t, 0.0, 0.05)
+        net.set_horizon(0.5, 0.25, True)
+        net.run()
+        out.append([net.order(b) for b in range(5)])
+        net.close()
+    assert np.isnan(out[1][3]).all() and np.isfinite(out[0]).all()
+    for b in (0, 1, 2, 4):
+        assert np.array_equal(out[0][b], out[1][b])
