@@ -64,7 +64,9 @@ const void* pick(int mode, int hl, int den) {
 
 cudaError_t configure(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, const ResPlan& r, cudaStream_t st) {
   const void* f = pick(r.mode, r.hl, r.split.den);
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)r.smem);
+  // the limit is the kernel's, for every launch of it: always the same one, so that a thread that launches
+  // a small network does not lower it under another thread's large one
+  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_CAP);
   if (e == cudaSuccess && r.mode == RES_CLUSTER && r.grid > 8)
     e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   cfg->gridDim = dim3((unsigned)r.grid);

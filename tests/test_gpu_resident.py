@@ -318,3 +318,44 @@ def test_a_trajectory_that_is_not_finite_stays_by_itself(native, n):
     assert np.isnan(out[1][3]).all() and np.isfinite(out[0]).all()
     for b in (0, 1, 2, 4):
         assert np.array_equal(out[0][b], out[1][b])
+
+
+@pytest.mark.parametrize("coupling,sizes", [(VOLCANO, (300, 9000)), (VOLCANO, (2000, 11000)), (0, (300, 5000))])
+def test_networks_of_different_size_run_in_two_threads(native, coupling, sizes):
+    """Two networks that take the same kernel with different amounts of shared memory."""
+    import threading
+
+    nets, want, errors = [], [], []
+    for n in sizes:
+        th, om = normal_inputs(n, 5)
+        net = native.Network(n, k=5, coupling=coupling, seed=7)
+        net.set_frequencies(om)
+        if coupling == 0:
+            net.generate_adjacency()
+        net.set_coupling(0, 1.5)
+        nets.append((net, th))
+
+    def once(net, th):
+        net.set_state(0, th, 0.0, 0.01)
+        net.set_horizon(0.05, 0.05, True)
+        net.run()
+        return net.order(0)
+
+    for net, th in nets:
+        want.append(once(net, th))
+
+    def loop(i):
+        try:
+            for _ in range(300):
+                assert np.array_equal(once(*nets[i]), want[i])
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+
+    ts = [threading.Thread(target=loop, args=(i,)) for i in (0, 1)]
+    for t in ts:
+        t.start()
+    for t in ts:
+        t.join()
+    assert not errors, errors
+    for net, _ in nets:
+        net.close()
