@@ -1226,7 +1226,12 @@ cudaError_t persistent_config(int coupling, int bmax, int kmax, size_t* smem_byt
     smem_layout(coupling, bmax, kk, rows_per_cta, 0, off, &total);
   }
   *smem_bytes = (size_t)total;
-  cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, total);
+  // the limit belongs to the kernel, not to this network: all that an SM gives a block, so that a network
+  // made later does not lower it under this one
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, f);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024 - (int)fa.sharedSizeBytes);
   if (e != cudaSuccess) return e;
   return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks_per_sm, f, KT, (size_t)total);
 }

@@ -274,6 +274,19 @@ def test_barrier_timeout_reports_error_and_context_survives(native, monkeypatch)
     net.close()
 
 
+@pytest.mark.parametrize("large,small,batch", [(300000, 1000, 1), (20000, 500, 4)])
+def test_a_small_network_made_later_leaves_a_large_one_runnable(native, large, small, batch):
+    """Both take the same kernel (rank above 8), with different amounts of shared memory."""
+    nets = []
+    for n in (large, small):
+        th, om = normal_inputs(n, 2)
+        nets.append(make(native, n, 12, VOLCANO, th, om, dense_level=0, t1=0.1, dt=0.1, batch=batch))
+    for net in nets:
+        net.run()
+        assert net.order(0).size == 2
+        net.close()
+
+
 @pytest.mark.parametrize("coupling", [DENSE, VOLCANO])
 def test_checkpointed_launches_are_bitwise_identical(native, coupling):
     """A run cut into many launches (a checkpoint every 7 attempts, records drained while
