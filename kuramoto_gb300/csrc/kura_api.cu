@@ -613,8 +613,9 @@ static int launch_begin(kura_handle* h, int mode, bool log_steps) {
   std::memcpy(h->traj_pin, h->htraj.data(), sizeof(TrajG) * h->B);
   CU(cudaMemcpyAsync(h->traj, h->traj_pin, sizeof(TrajG) * h->B, cudaMemcpyHostToDevice, h->stream));
   CU(cudaMemsetAsync(h->ctl, 0, 132, h->stream));  // barrier and error flag
-  // the test hook of the barrier's time limit needs a launch that has a grid barrier
-  const bool resident = mode == kura::MODE_INTEGRATE && h->res.mode >= 0 && p.bar_extra == 0;
+  // the test hook of the barrier's time limit needs a launch that has a grid barrier: not one CTA or cluster
+  const bool resident = mode == kura::MODE_INTEGRATE && h->res.mode >= 0 &&
+                        (p.bar_extra == 0 || h->res.mode >= kura::RES_MODE_FIXED);
   if (resident && h->fix)
     CU(cudaMemsetAsync(h->fix, 0, sizeof(unsigned long long) * kura::res_fix(h->B), h->stream));
   CU(cudaEventRecord(h->ev0, h->stream));

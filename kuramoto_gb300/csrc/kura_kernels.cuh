@@ -101,7 +101,7 @@ struct ResSplit {
   int den, ld;  // stored adjacency: RES_F32 or RES_I8 with rows of ld values; 0: regenerated coupling
 };
 enum { RES_F32 = 1, RES_I8 = 2, RES_IMMA = 3 };  // RES_IMMA: int8 on the integer tensor pipe
-constexpr int RES_MODE_FIXED = 2;  // this form and RES_IMMA need KParams::fix
+constexpr int RES_MODE_FIXED = 2;  // this form and RES_IMMA need KParams::fix; the forms from it on have a grid barrier
 constexpr size_t res_fix(int batch) { return (size_t)3 * batch * 16 + 3; }  // their number
 struct ResPlan {
   int mode = -1, hl = 0, grid = 0;

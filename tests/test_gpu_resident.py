@@ -359,3 +359,40 @@ def test_networks_of_different_size_run_in_two_threads(native, coupling, sizes):
     assert not errors, errors
     for net, _ in nets:
         net.close()
+
+
+# regenerated coupling over the grid, in the same order and in fixed point; stored float32, int8 in
+# floats and on the integer pipe
+@pytest.mark.parametrize("n,batch,kw", [(11000, 2, dict(coupling=VOLCANO)), (13000, 1, dict(coupling=VOLCANO)),
+                                        (300, 1, dict(coupling=0)), (5000, 1, dict(coupling=0)),
+                                        (300, 1, dict(coupling=0, adj_storage=1)), (12000, 1, dict(coupling=0, adj_storage=1))])
+def test_barrier_time_limit_of_the_resident_forms(native, monkeypatch, n, batch, kw):
+    """Each barrier waits for one arrival that never comes: the launch ends with the error, and the
+    context runs the same network afterwards."""
+    th, om = normal_inputs(n, 2)
+
+    def run():
+        net = native.Network(n, k=5, batch=batch, seed=7, **kw)
+        net.set_frequencies(om)
+        if kw["coupling"] == 0:
+            net.generate_adjacency()
+        for b in range(batch):
+            net.set_coupling(b, 1.0)
+            net.set_state(b, th, 0.0, 0.01)
+        net.set_horizon(0.5, 0.25, True)
+        try:
+            net.run()
+            return net.order(0)
+        finally:
+            net.close()
+
+    assert native.ADJ_I8 == 1
+    want = run()
+    monkeypatch.setenv("KURA_BARRIER_TIMEOUT_MS", "300")
+    monkeypatch.setenv("KURA_TEST_BARRIER_EXTRA", "1")
+    with pytest.raises(native.KuraError) as e:
+        run()
+    assert e.value.code == -4
+    monkeypatch.delenv("KURA_TEST_BARRIER_EXTRA")
+    monkeypatch.delenv("KURA_BARRIER_TIMEOUT_MS")
+    assert np.array_equal(run(), want) and want.size == 3
