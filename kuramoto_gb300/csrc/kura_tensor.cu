@@ -37,13 +37,11 @@ namespace kura {
 namespace {
 
 constexpr int T_MAXC = 32;  // output crossings handled per step
-// K per pipeline stage of the coupling GEMM (32: 64-byte swizzle rows; 64: 128-byte rows).
-// 64 (three 64 KB stages, eight MMAs per stage handshake) measured 7 % faster per launch at
-// N=65536, B=128 than 32 (seven 32 KB stages, four MMAs per handshake)
-#ifndef KURA_GEMM_BK
-#define KURA_GEMM_BK 64
-#endif
-constexpr int TE_BK = KURA_GEMM_BK;
+// K per pipeline stage of the coupling GEMM, in 128-byte swizzle rows: 64 (three 64 KB stages, eight MMAs
+// per stage handshake) measured 7 % faster per launch at N=65536, B=128 than 32 in 64-byte rows (seven
+// 32 KB stages, four MMAs per handshake).  The split GEMM reads through the same tensor maps.
+constexpr int TE_BK = 64;
+static_assert(TE_BK == TS_BK, "one tensor map for both GEMMs");
 // The parts of a component x of (cos, sin): X_hi is a multiple of a step, X_lo the rest to 11 bits.
 // From |x| = 2^-3 on the step is 2^-8: the tensor core cuts each product off at the accumulator's last
 // bit, always toward zero, and coarse steps leave it nothing to cut from A_hi X_hi.  Below, X_hi has
