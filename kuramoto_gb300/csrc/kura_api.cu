@@ -315,7 +315,7 @@ extern "C" int kura_create(const kura_config* cfg, kura_handle** out) {
   h->finished.assign(B, 0);
   h->order.assign(B, {});
   h->stats.grid = h->res.mode >= 0 ? h->res.grid : G;
-  h->stats.block = h->res.split.den == kura::RES_F32 ? 576 : kura::KT;
+  h->stats.block = h->res.mode >= 0 ? kura::resident_threads(h->res) : kura::KT;
   *out = h;
   return KURA_OK;
 #undef CUH

@@ -111,6 +111,7 @@ struct ResPlan {
 // blocks, rows: the persistent kernel's grid for this network and its rows per CTA
 ResPlan resident_plan(int64_t n, int batch, int k, int blocks, int rows);
 ResPlan resident_plan_dense(int den, int64_t n, int ld, int blocks, int rows);
+int resident_threads(const ResPlan& r);  // per CTA
 cudaError_t launch_resident(const KParams& p, const ResPlan& r, cudaStream_t st);
 
 // sets the message returned by kura_last_error() for the calling thread

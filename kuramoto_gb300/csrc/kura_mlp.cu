@@ -48,7 +48,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // 16 is the narrowest that the MMA takes: a training step went from 65 to 59 us, a forward pass of
 // 64 rows from 55 to 48.  The K loop of a column is the same in every form, and so are the results,
 // bit for bit.
-constexpr int MLP_NC = 16;
+constexpr int MLP_NC = 16;  // the epilogues below read that many columns at once
 
 // ---------------------------------------------------------------- GEMM epilogues
 // forward: z = acc + b; hidden layers store silu(z) (row-major and transposed, BF16) and
@@ -70,46 +70,43 @@ struct FwdEpi {
   bf16* dZT;    // [ld][Bt]
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int r = m0 + row;
+    const int c0 = sp * MLP_NC;
+    float a[16];
+    umma::tmem_ld16(taddr, a);
+    umma::tmem_ld_wait();
+    float z[16];
 #pragma unroll
-    for (int q0 = 0; q0 < MLP_NC; q0 += 16) {
-      const int c0 = sp * MLP_NC + q0;
-      float a[16];
-      umma::tmem_ld16(taddr + q0, a);
-      umma::tmem_ld_wait();
-      float z[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) z[j] = a[j] + bias[c0 + j];
-      if (last) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          if (c0 + j >= out_dim) break;
-          Y[(size_t)r * out_dim + c0 + j] = z[j];
-          if (T) {
-            const float e = z[j] - T[(size_t)r * out_dim + c0 + j];
-            const bf16 b = __float2bfloat16_rn(r < nvalid ? scale * e : 0.f);
-            dZ[(size_t)r * ld + c0 + j] = b;
-            dZT[(size_t)(c0 + j) * Bt + r] = b;
-          }
-        }
-        continue;
-      }
-      float h[16], d[16];
+    for (int j = 0; j < 16; ++j) z[j] = a[j] + bias[c0 + j];
+    if (last) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
-        const float s = 1.f / (1.f + expf(-z[j]));
-        h[j] = z[j] * s;
-        d[j] = s * (1.f + z[j] * (1.f - s));
+        if (c0 + j >= out_dim) break;
+        Y[(size_t)r * out_dim + c0 + j] = z[j];
+        if (T) {
+          const float e = z[j] - T[(size_t)r * out_dim + c0 + j];
+          const bf16 b = __float2bfloat16_rn(r < nvalid ? scale * e : 0.f);
+          dZ[(size_t)r * ld + c0 + j] = b;
+          dZT[(size_t)(c0 + j) * Bt + r] = b;
+        }
       }
-      uint4* hp = reinterpret_cast<uint4*>(H + (size_t)r * ld + c0);
-      hp[0] = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
-      hp[1] = make_uint4(pack_bf16(h[8], h[9]), pack_bf16(h[10], h[11]), pack_bf16(h[12], h[13]),
-                         pack_bf16(h[14], h[15]));
-#pragma unroll
-      for (int j = 0; j < 16; ++j) HT[(size_t)(c0 + j) * Bt + r] = __float2bfloat16_rn(h[j]);
-      float4* dp = reinterpret_cast<float4*>(S + (size_t)r * ld + c0);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) dp[q] = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
+      return;
     }
+    float h[16], d[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const float s = 1.f / (1.f + expf(-z[j]));
+      h[j] = z[j] * s;
+      d[j] = s * (1.f + z[j] * (1.f - s));
+    }
+    uint4* hp = reinterpret_cast<uint4*>(H + (size_t)r * ld + c0);
+    hp[0] = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
+    hp[1] = make_uint4(pack_bf16(h[8], h[9]), pack_bf16(h[10], h[11]), pack_bf16(h[12], h[13]),
+                       pack_bf16(h[14], h[15]));
+#pragma unroll
+    for (int j = 0; j < 16; ++j) HT[(size_t)(c0 + j) * Bt + r] = __float2bfloat16_rn(h[j]);
+    float4* dp = reinterpret_cast<float4*>(S + (size_t)r * ld + c0);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) dp[q] = make_float4(d[4 * q], d[4 * q + 1], d[4 * q + 2], d[4 * q + 3]);
   }
 };
 
@@ -120,16 +117,13 @@ struct DwEpi {
   int out_p, ld;
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int r = m0 + row;
+    float a[16];
+    umma::tmem_ld16(taddr, a);
+    umma::tmem_ld_wait();
+    if (r >= out_p) return;
+    float4* g = reinterpret_cast<float4*>(G + (size_t)r * ld + sp * MLP_NC);
 #pragma unroll
-    for (int q0 = 0; q0 < MLP_NC; q0 += 16) {
-      float a[16];
-      umma::tmem_ld16(taddr + q0, a);
-      umma::tmem_ld_wait();
-      if (r >= out_p) continue;
-      float4* g = reinterpret_cast<float4*>(G + (size_t)r * ld + sp * MLP_NC + q0);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) g[q] = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
-    }
+    for (int q = 0; q < 4; ++q) g[q] = make_float4(a[4 * q], a[4 * q + 1], a[4 * q + 2], a[4 * q + 3]);
   }
 };
 
@@ -142,29 +136,26 @@ struct DhEpi {
   int Bt, ld;
   __device__ void row(uint32_t taddr, int row, int m0, int sp) {
     const int r = m0 + row;
+    const int c0 = sp * MLP_NC;
+    float a[16];
+    umma::tmem_ld16(taddr, a);
+    umma::tmem_ld_wait();
+    const float4* sp4 = reinterpret_cast<const float4*>(S + (size_t)r * ld + c0);
+    float d[16];
 #pragma unroll
-    for (int q0 = 0; q0 < MLP_NC; q0 += 16) {
-      const int c0 = sp * MLP_NC + q0;
-      float a[16];
-      umma::tmem_ld16(taddr + q0, a);
-      umma::tmem_ld_wait();
-      const float4* sp4 = reinterpret_cast<const float4*>(S + (size_t)r * ld + c0);
-      float d[16];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const float4 s = sp4[q];
-        d[4 * q] = a[4 * q] * s.x;
-        d[4 * q + 1] = a[4 * q + 1] * s.y;
-        d[4 * q + 2] = a[4 * q + 2] * s.z;
-        d[4 * q + 3] = a[4 * q + 3] * s.w;
-      }
-      uint4* dp = reinterpret_cast<uint4*>(dZ + (size_t)r * ld + c0);
-      dp[0] = make_uint4(pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]), pack_bf16(d[4], d[5]), pack_bf16(d[6], d[7]));
-      dp[1] = make_uint4(pack_bf16(d[8], d[9]), pack_bf16(d[10], d[11]), pack_bf16(d[12], d[13]),
-                         pack_bf16(d[14], d[15]));
-#pragma unroll
-      for (int j = 0; j < 16; ++j) dZT[(size_t)(c0 + j) * Bt + r] = __float2bfloat16_rn(d[j]);
+    for (int q = 0; q < 4; ++q) {
+      const float4 s = sp4[q];
+      d[4 * q] = a[4 * q] * s.x;
+      d[4 * q + 1] = a[4 * q + 1] * s.y;
+      d[4 * q + 2] = a[4 * q + 2] * s.z;
+      d[4 * q + 3] = a[4 * q + 3] * s.w;
     }
+    uint4* dp = reinterpret_cast<uint4*>(dZ + (size_t)r * ld + c0);
+    dp[0] = make_uint4(pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]), pack_bf16(d[4], d[5]), pack_bf16(d[6], d[7]));
+    dp[1] = make_uint4(pack_bf16(d[8], d[9]), pack_bf16(d[10], d[11]), pack_bf16(d[12], d[13]),
+                       pack_bf16(d[14], d[15]));
+#pragma unroll
+    for (int j = 0; j < 16; ++j) dZT[(size_t)(c0 + j) * Bt + r] = __float2bfloat16_rn(d[j]);
   }
 };
 

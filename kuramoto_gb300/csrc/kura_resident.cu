@@ -12,7 +12,8 @@ constexpr int NT = 512;
 // would wait for the one that has three
 constexpr int NT_F32 = 576;
 __host__ __device__ constexpr int threads_of(int den) { return den == RES_F32 ? NT_F32 : NT; }
-constexpr size_t SMEM_CAP = 227 * 1024 - 256;
+constexpr size_t SMEM_CAP = 227 * 1024 - 256;  // dynamic, beside the ResNet
+static_assert(sizeof(ResNet) <= 256, "SMEM_CAP");
 
 template <int MODE, bool HL, int DEN = 0>
 __global__ void __launch_bounds__(threads_of(DEN), 1) k_resident(const KParams p, const ResSplit split) {
@@ -24,7 +25,7 @@ __global__ void __launch_bounds__(threads_of(DEN), 1) k_resident(const KParams p
     net.hi = p.ph_hi; net.lo = p.ph_lo; net.w = p.ph_w; net.g = p.g;
     net.ld = p.ld;
     net.atol = p.atol; net.rtol = p.rtol; net.fixed = p.fixed; net.dense_level = p.dense_level;
-    net.t_eval = p.t_eval; net.dtf = 0.f; net.n_eval = p.n_eval;
+    net.t_eval = p.t_eval; net.n_eval = p.n_eval;
     net.out_r = p.out_r; net.out_idx = p.out_idx; net.out_theta = p.out_theta; net.out_coup = p.out_coup;
     net.out_ld = p.ld; net.ring = p.ring;
     net.log_t = p.log_t; net.log_h = p.log_h; net.log_cap = p.log_cap;
@@ -45,7 +46,7 @@ __global__ void __launch_bounds__(threads_of(DEN), 1) k_resident(const KParams p
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
-  if (!e.run(false, nullptr)) return;
+  if (!e.run()) return;
   if (blockIdx.x == 0) {
     if (threadIdx.x < p.batch) p.traj[threadIdx.x] = e.tr[threadIdx.x];
     if (threadIdx.x == 0) atomicAdd((unsigned long long*)p.counters, (unsigned long long)e.nbar);
@@ -117,6 +118,8 @@ bool shape(ResPlan* r, int B, int k, int blocks, int rows, int mode, int ctas, i
 // A cluster pays for its rows, a grid for its barrier.  Fixed point serves from 12000 oscillators
 // on, where it no longer matters in which order the sums are formed (kura_resident.cuh).
 constexpr int64_t ONE_PAIRS = 256, CLUSTER_PAIRS = 12288, FIXED_N = 12000;
+
+int resident_threads(const ResPlan& r) { return threads_of(r.split.den); }
 
 ResPlan resident_plan(int64_t n, int B, int k, int blocks, int rows) {
   ResPlan r;

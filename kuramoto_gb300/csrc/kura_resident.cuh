@@ -59,11 +59,10 @@ struct ResNet {
   long long ld;
   double atol, rtol;
   int fixed, dense_level;
-  const float* t_eval;  // output grid, or null: dtf * (i + 1)
-  float dtf;
+  const float* t_eval;  // output grid
   int n_eval;
   float* out_r;  // [B][ring]
-  int* out_idx;  // [B][ring] or null
+  int* out_idx;  // [B][ring]
   float* out_theta;
   float* out_coup;
   long long out_ld;
@@ -903,7 +902,7 @@ struct Resident {
   }
   // (read from L2: an acquire at every barrier empties L1, so the controller compares with te first)
   __device__ __forceinline__ double eval_time(int i) const {
-    return N.t_eval ? (double)N.t_eval[i] : (double)(N.dtf * (float)(i + 1));
+    return (double)N.t_eval[i];
   }
   // dense output at te from the last accepted step (interpolate, dp45.cu:70-76)
   __device__ void fill_record(int b, int j) {
@@ -965,7 +964,7 @@ struct Resident {
     const float* s = rsum + tid * RES_RED;
     const float xn = s[2 * RES_KMAX] / (float)N.n, yn = s[2 * RES_KMAX + 1] / (float)N.n;
     N.out_r[(size_t)tid * N.ring + ps[tid * 4 + 2]] = sqrtf(xn * xn + yn * yn);
-    if (N.out_idx) N.out_idx[(size_t)tid * N.ring + ps[tid * 4 + 2]] = ps[tid * 4 + 3];
+    N.out_idx[(size_t)tid * N.ring + ps[tid * 4 + 2]] = ps[tid * 4 + 3];
   }
   // couplings of the recorded rows (dense level 2), from the table
   __device__ void record_couplings() {
@@ -982,7 +981,7 @@ struct Resident {
   // is current, 1: the accepted step is still to be taken, 2: see load_phases), ps[4 b + 2] and
   // ps[4 b + 3] the record slot (-1: none) and index of the current pass.  Returns false when a
   // barrier gave up.
-  __device__ bool run(bool fresh_theta, const float* theta0) {
+  __device__ bool run() {
     for (int r = tid; r < nr; r += NT) {
       const int i = r0 + r;
       if (!DEN) {
@@ -1007,21 +1006,13 @@ struct Resident {
       const int sa = slot_a(b), k1 = tr[b].rot_g ? 6 : 0, k7 = 6 - k1;
       for (int r = tid; r < nr; r += NT) {
         const int P = b * N.split.rows + r;
-        if (fresh_theta) {
-          const double th = (double)theta0[r0 + r];
-          const double kk = rint(th / TWO_PI_D);
-          const double rr = th - kk * TWO_PI_D;
-          const float hi = (float)rr;
-          N.w[gaddr(0, b, r)] = (long long)kk;
-          store_y(b, r, P, make_float2(hi, (float)(rr - (double)hi)));
-        }
         // a launch that resumes the records of a step reads all its slopes
-        g[sa * np + P] = fresh_theta ? 0.f : N.g[gaddr(k1, b, r)];
-        g[(sa ^ 1) * np + P] = fresh_theta ? 0.f : N.g[gaddr(k7, b, r)];
+        g[sa * np + P] = N.g[gaddr(k1, b, r)];
+        g[(sa ^ 1) * np + P] = N.g[gaddr(k7, b, r)];
 #pragma unroll
-        for (int j = 2; j < 6; ++j) g[j * np + P] = fresh_theta ? 0.f : N.g[gaddr(j, b, r)];
+        for (int j = 2; j < 6; ++j) g[j * np + P] = N.g[gaddr(j, b, r)];
       }
-      if (!fresh_theta) load_phases(b, ps[b * 4]);
+      load_phases(b, ps[b * 4]);
     }
     __syncthreads();
 
