@@ -9,8 +9,8 @@
 // For the reference's volcano rule N*A_ij is an integer in [-K, K], exact in F16 up to 2048, so
 // the product carries the precision of the hi+lo split of X: 2^-21 of 1 and 2^-18 or better of itself,
 // where BF16 parts of the same size and rate hold 2^-18 of x.  A general adjacency is split as 2^p_i N A_ij = A_hi + A_lo
-// with a power of two per row, which puts a row's largest entry below 2^15: A_hi has 7 significant
-// bits, A_lo 11 more.  The term A_lo X_hi is added by further K steps.  F16 has five bits of exponent:
+// with a power of two per row, which puts a row's largest entry below 2^15: 11 significant bits in A_hi
+// and 11 more in A_lo.  The term A_lo X_hi is added by further K steps.  F16 has five bits of exponent:
 // an adjacency with a row whose entries span more than 2^21 (or lie below 2^-70, or are not finite) is
 // held in BF16 parts instead, as are its X: each entry to 2^-18 of itself, at the same size and rate.
 //
@@ -622,7 +622,7 @@ __global__ void k_t_fill(float* p, int n, float v) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) p[i] = v;
 }
-// general adjacency, one block per row: 2^p N A = hi (7 bits) + lo (11 bits) in F16, with 2^p so that the
+// general adjacency, one block per row: 2^p N A = hi + lo in F16, 11 bits each, with 2^p so that the
 // row's largest entry lies in [2^14, 2^15) (1 for a row of zeros).  *wide is set where F16 holds an
 // entry less well than BF16 would: one below 2^-7, whose lo part meets F16's smallest step, one that is
 // not finite, or a row below what 2^-p / N / X_SCALE can undo.
@@ -655,9 +655,7 @@ __global__ void k_t_split(const float* __restrict__ adj, int n, int np, float sc
     for (int j = threadIdx.x; j < np; j += blockDim.x) {
       const float a0 = (i < n && j < n) ? adj[(size_t)i * n + j] * scale : 0.f, a = a0 * p;
       out |= !isfinite(a) || (a0 != 0.f && fabsf(a) < 0.0078125f);
-      // Veltkamp's split: the upper 24 - 17 = 7 bits of a
-      const float t = 131073.f * a;
-      const __half h = __float2half_rn(t - (t - a));
+      const __half h = __float2half_rn(a);
       hi[(size_t)i * np + j] = h;
       lo[(size_t)i * np + j] = __float2half_rn(a - __half2float(h));
     }
