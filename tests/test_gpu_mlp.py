@@ -89,6 +89,13 @@ def test_column_blocks_match_oracle(native, in_dim, hidden, out_dim, batch, n):
                 k += size
 
 
+@pytest.mark.parametrize("in_dim,hidden,out_dim,batch,n", [(15, 64, 15, 128, 127), (16, 128, 16, 128, 128),
+                                                           (17, 64, 17, 256, 200), (47, 256, 47, 128, 5), (48, 64, 48, 128, 64)])
+def test_sixteen_column_blocks_match_oracle(native, in_dim, hidden, out_dim, batch, n):
+    """The same at the edges of 16-column blocks."""
+    test_column_blocks_match_oracle(native, in_dim, hidden, out_dim, batch, n)
+
+
 def test_one_training_step_is_oracle_adam(native):
     with native.MLP(IN, OUT, hidden=256, batch=256, seed=9) as m:
         p0 = m.params().astype(np.float64)

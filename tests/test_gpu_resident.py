@@ -239,6 +239,15 @@ def test_integer_product_matches_fp64(native, oracle_lib, n, k):
         assert np.max(np.abs(x[3] - np.asarray(ref.couplings[q]).reshape(-1))) < 3e-6 * scale + 1e-6
 
 
+@pytest.mark.parametrize("n,tiles", [(12010, 1), (12030, 2), (12045, 3), (18000, 8)])
+def test_integer_product_of_few_and_of_eight_row_tiles(native, oracle_lib, n, tiles):
+    """Row tiles of the last CTA's pass (1 to 3) and of a full CTA's (8), which the sizes above leave out."""
+    rows = -(-n // 152)
+    last = n - (-(-n // rows) - 1) * rows
+    assert tiles in (-(-last // 16), -(-rows // 16))
+    test_integer_product_matches_fp64(native, oracle_lib, n, 5)
+
+
 @pytest.mark.parametrize("amp", [0.3, 1e-2, 1e-5, 1e-6])
 @pytest.mark.parametrize("n", [12000, 18000])
 def test_integer_product_keeps_small_components(native, n, amp):

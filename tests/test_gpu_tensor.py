@@ -110,6 +110,29 @@ def test_tensor_small_phases_keep_their_digits(native, n, batch, amp):
     net.close()
 
 
+@pytest.mark.parametrize("general", [False, True])
+def test_tensor_couplings_to_two_f16_parts(native, general):
+    """One K step of 64: per term 2^-21 of (cos, sin) and, of a general weight, 2^-22 of it and 2^-20 of
+    what is left out (half a step of X_lo times 2^-11), independent of one another and evenly spread
+    (1 / sqrt 3); four additions per column and part, 2^-23 each: 2^-20 of the terms' root sum square.  BF16
+    parts are 2^-18.5 off here."""
+    n, batch = 64, 16
+    rng = np.random.default_rng(8)
+    thetas = [rng.uniform(0, 2 * np.pi, n).astype(np.float32) for _ in range(batch)]
+    adj = (rng.standard_normal((n, n)) / n).astype(np.float32) if general else None
+    net = make(native, n, 5, thetas, np.zeros(n, np.float32), [1.0] * batch, adj=adj)
+    a = adj.astype(np.float64) if general else np.rint(net.adjacency().astype(np.float64) * n) / n
+    err = []
+    for b in range(batch):
+        x = np.stack([np.cos(thetas[b].astype(np.float64)), np.sin(thetas[b].astype(np.float64))], 1)
+        err.append(net.rhs(b, thetas[b])[1].reshape(n, 2) - a @ x)
+    assert np.sqrt(np.mean(np.square(err))) <= 2.0**-20 * np.sqrt(np.mean((a * a).sum(1)))
+    if general:
+        # 11 + 11 bits of an entry, and the roundings of N A, 1/N and the product
+        assert np.all(np.abs(net.adjacency().astype(np.float64) - a) <= (2.0**-22 + 3 * 2.0**-24) * np.abs(a) + 2.0**-38 * np.abs(a).max())
+    net.close()
+
+
 @pytest.mark.parametrize("n,batch", [(130, 3), (1500, 24)])
 def test_tensor_rows_of_wide_range(native, n, batch):
     """Rows whose entries span 2^40, rows of tiny entries and of zeros: every entry of N A is held in two
