@@ -107,7 +107,10 @@ bool shape(ResPlan* r, int B, int k, int blocks, int rows, int mode, int ctas, i
 // Which form, by measured time per attempt (K = 5, Cauchy frequencies; the persistent kernel in
 // brackets):
 //   n x batch      one CTA   cluster (CTAs)   grid, same order   grid, fixed point
-//   300             16.5     17.1 (4)          26.2              21.4   [44]
+//   128             15.2     17.1 (2)
+//   256             15.7     17.1 (4)
+//   300             16.5     17.0 (4)          26.2              21.4   [44]
+//   400             17.4     17.0 (4)
 //   1000            23.4     17.5 (8)          26.4              25.1   [48]
 //   4000             -       21.4 (16)         29.3              25.6   [48]
 //   8000             -       23.9 (16)         31.1              25.7   [48]
@@ -115,7 +118,8 @@ bool shape(ResPlan* r, int B, int k, int blocks, int rows, int mode, int ctas, i
 //   1000 x 8         -       25.4 (16)         33.4              30.2   [56]
 //   4000 x 8         -       51.6 (16)         36.7              30.0   [56]
 //   200000 x 5       -        -                 -                61.6   [139]
-// A cluster pays for its rows, a grid for its barrier.  Fixed point serves from 12000 oscillators
+// One CTA and a cluster of four cross between 350 and 400 pairs and differ by 3 % from 300 to 400; the
+// line is drawn below that, at 256.  A cluster pays for its rows, a grid for its barrier.  Fixed point serves from 12000 oscillators
 // on, where it no longer matters in which order the sums are formed (kura_resident.cuh).
 constexpr int64_t ONE_PAIRS = 256, CLUSTER_PAIRS = 12288, FIXED_N = 12000;
 
