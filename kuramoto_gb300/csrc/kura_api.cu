@@ -683,7 +683,7 @@ extern "C" int kura_run(kura_handle* h, const kura_callbacks* cb) {
     h->stats.rejected = rej;
     if (errc) {
       std::string m = errc == KURA_ERR_STEP_UNDERFLOW ? "step size underflow"
-                      : errc == KURA_ERR_UNSUPPORTED ? "more than 32 output times crossed in one step"
+                      : errc == KURA_ERR_UNSUPPORTED ? "more output times crossed than the records hold"
                                                       : "non-finite error norm";
       for (int b = 0; b < h->B; ++b) {
         const TrajG& T = h->htraj[b];

@@ -36,7 +36,7 @@ namespace kura {
 
 namespace {
 
-constexpr int T_MAXC = 32;  // output crossings handled per step
+constexpr int T_MAXC = 32;  // output times recorded per launch; a step that crosses more waits for the next one
 // K per pipeline stage of the coupling GEMM, in 128-byte swizzle rows: 64 (three 64 KB stages, eight MMAs
 // per stage handshake) measured 7 % faster per launch at N=65536, B=128 than 32 in 64-byte rows (seven
 // 32 KB stages, four MMAs per handshake).  The split GEMM reads through the same tensor maps.
@@ -116,10 +116,11 @@ __global__ void k_t_first(const TrajG* traj, TCoef* src, int* flags) {
   }
 }
 // the six stages of trajectory b's next attempt, by 16 threads per stage; flags[1]: some
-// trajectory steps in it
+// trajectory steps in it, or sits it out because it still owes records of its last step (how many
+// output times a step crosses depends on the step control, and that on rounding: no limit on it)
 __device__ __forceinline__ void fill_attempt(const TrajG& T, TCoef* src, int bp, int b, int t, int* flags) {
   const bool act = (T.status == 0 && T.eval_i >= T.eval_end && T.t < T.t1);
-  if (t == 0 && act) flags[1] = 1;
+  if (t == 0 && (act || (T.status == 0 && T.eval_i < T.eval_end))) flags[1] = 1;
   if (t >= 6 * 16) return;
   const int j = t & 15, s = 2 + (t >> 4);
   TCoef& S = src[(s - 1) * bp + b];
@@ -587,7 +588,7 @@ __global__ void k_t_output(TView v, TrajG* traj, const float* t_eval, float* par
     }
     if (threadIdx.x == 0) {
       if (initial) T.need_init = 0;
-      else if (T.eval_i < T.eval_end) T.status = KURA_ERR_UNSUPPORTED;  // more than T_MAXC crossings in a step
+      else if (T.eval_i < T.eval_end && T.out_count >= ring) T.status = KURA_ERR_UNSUPPORTED;  // no room for the rest
     }
   }
   if (threadIdx.x == 0) {

@@ -284,6 +284,44 @@ def test_tensor_operands_from_the_gemm_match_fp64(native, oracle_lib, n, batch):
     net.close()
 
 
+@pytest.mark.parametrize("c,fixed,t1,dt,h0", [(0.0, False, 50.0, 0.1, 0.001), (1.0, True, 8.0, 0.01, 1.0),
+                                              (1.0, True, 5.0, 1.0 / 33, 1.0)])
+@pytest.mark.parametrize("n,batch", [(64, 3), (700, 7)])
+def test_tensor_step_over_many_output_times(native, n, batch, c, fixed, t1, dt, h0):
+    """Steps that cross up to hundreds of output times, 33 among them: every record is there, also when
+    budgets of attempts end between them.  Without coupling the phases are exact in both engines and r is a
+    float32 sum (5e-6); with it the bound is the other runs'."""
+    _, om = normal_inputs(n, 21)
+    thetas = [normal_inputs(n, 300 + b, init=2 * np.pi)[0] for b in range(batch)]
+
+    def net_of(engine):
+        net = native.Network(n, k=5, coupling=DENSE, batch=batch, seed=2, engine=engine, fixed_step=fixed)
+        net.set_frequencies(om)
+        net.generate_adjacency()
+        for b in range(batch):
+            net.set_coupling(b, c)
+            net.set_state(b, thetas[b], 0.0, h0 * (1 + 0.5 * b) if not fixed else h0)
+        net.set_horizon(t1, dt, True)
+        return net
+
+    out = []
+    for engine in (native.ENGINE_PERSISTENT, TENSOR):
+        net = net_of(engine)
+        net.run()
+        out.append([net.order(b) for b in range(batch)])
+        net.close()
+    net = net_of(TENSOR)
+    rec = [[] for _ in range(batch)]
+    while net.advance(4, on_output=lambda b, i, t, r, theta, cp: rec[b].append((i, r)) and False):
+        pass
+    net.close()
+    for b in range(batch):
+        assert out[0][b].size == out[1][b].size == int(np.float32(t1) / np.float32(dt)) + 1
+        assert np.max(np.abs(out[0][b] - out[1][b])) < (5e-6 if c == 0 else 1e-4)
+        assert [q[0] for q in rec[b]] == list(range(-1, out[1][b].size - 1))
+        assert np.array_equal(np.array([q[1] for q in rec[b]], np.float32), out[1][b])
+
+
 def test_tensor_engine_reused_over_horizons(native):
     """One engine over horizons that grow, shrink and grow again (kept buffers, kept graph), with a state
     that is replaced before its upload is over, gives the records of a fresh engine each time."""
